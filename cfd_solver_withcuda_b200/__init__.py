@@ -105,6 +105,13 @@ class MlpWgrad(ctypes.Structure):
                 ("db", ctypes.c_void_p), ("accumulate", ctypes.c_int)]
 
 
+class MpnnNet(ctypes.Structure):
+    """cfd_mpnn_net."""
+    _fields_ = [(n, ctypes.c_int) for n in ("layers", "node_in", "edge_in", "out", "n_nodes", "n_edges")] + \
+               [(n, ctypes.c_void_p) for n in ("params", "grads", "xn", "xe", "src", "dst", "dst_ptr", "src_ptr",
+                                                "src_order", "act", "pred", "dpred", "workspace")]
+
+
 class StepInfo(ctypes.Structure):
     _fields_ = [("iterations", ctypes.c_int), ("min_dt", ctypes.c_double), ("total_time", ctypes.c_double),
                 ("error", ctypes.c_double * 4), ("res_l2", ctypes.c_double * 4), ("bad_cell", ctypes.c_int),
@@ -179,6 +186,9 @@ SIGNATURES = {
     "cfd_mpnn_mlp_backward": (_I, [ctypes.POINTER(MlpBwd), _P]),
     "cfd_mpnn_weight_grad": (_I, [ctypes.POINTER(MlpWgrad), _P]),
     "cfd_mpnn_wgrad_blocks": (_I, []),
+    "cfd_mpnn_net_floats": (ctypes.c_size_t, [_I, _I, _I, _I, _I, _I]),
+    "cfd_mpnn_net_forward": (_I, [ctypes.POINTER(MpnnNet), _P]),
+    "cfd_mpnn_net_backward": (_I, [ctypes.POINTER(MpnnNet), _P]),
     "cfd_mpnn_status": (_I, [ctypes.POINTER(ctypes.c_int), _I]),
     "cfd_mpnn_add": (_I, [_P, _I, _P, _I, _P, _I, _I, _I, _P]),
     "cfd_mpnn_gather_add": (_I, [_P, _I, _P, _I, _P, _I, _I, _P]),

@@ -288,6 +288,8 @@ class Net:
         self.engine = engine
         self.bwd_engine = engine if bwd_engine is None else bwd_engine
         self.L, self.out, self.device = layers, out, torch.device(device)
+        # The mma.sync passes of a network with at most 16 outputs are issued by one library call each.
+        self.whole = self.engine == 0 and self.bwd_engine == 0 and out <= 16
         self.dims = {"enc_n": (node_in, W), "enc_e": (edge_in, W), "dec": (W, out)}
         for l in range(layers):
             self.dims["edge%d" % l] = (3 * W, W)
@@ -345,6 +347,12 @@ class Net:
         torch = _torch()
         W, L = self.HIDDEN, self.L
         f = lambda r, c: torch.empty((r, c), dtype=torch.float32, device=self.device)
+        if self.whole:
+            n = cb.lib().cfd_mpnn_net_floats(L, self.dims["enc_n"][0], self.dims["enc_e"][0], self.out, N, E)
+            self._bufs = {"key": (N, E), "act": torch.empty(n, dtype=torch.float32, device=self.device),
+                          "pred": f(N, self.out), "dpred": f(N, self.out),
+                          "loss": torch.zeros(1, dtype=torch.float32, device=self.device)}
+            return self._bufs
         b = {"key": (N, E), "h": [f(N, W) for _ in range(L + 1)], "e": [f(E, W) for _ in range(L + 1)],
              "agg": [f(N, W) for _ in range(L)], "z_enc_n": f(N, W), "z_enc_e": f(E, W),
              "z_edge": [f(E, W) for _ in range(L)], "z_node": [f(N, W) for _ in range(L)], "z_dec": f(N, W),
@@ -401,11 +409,30 @@ class Net:
         self._wgrad(dy, rows, [_seg(z1, silu=1)], gw2, gb2)
         self._wgrad(self._bufs["dz"], rows, x_segs, gw1, gb1)
 
+    def _net(self, xn, xe, gb, dpred=None):
+        """The library's description of one whole pass (cfd_mpnn_net)."""
+        b = self._bufs
+        a = cb.MpnnNet()
+        a.layers, a.node_in, a.edge_in, a.out = self.L, xn.shape[1], xe.shape[1], self.out
+        a.n_nodes, a.n_edges = xn.shape[0], xe.shape[0]
+        a.params, a.grads, a.workspace = self.flat.data_ptr(), self.grad.data_ptr(), self.workspace.data_ptr()
+        a.xn, a.xe = xn.data_ptr(), xe.data_ptr()
+        a.src, a.dst, a.dst_ptr = gb.src.data_ptr(), gb.dst.data_ptr(), gb.dst_ptr.data_ptr()
+        a.src_ptr, a.src_order = gb.src_ptr.data_ptr(), gb.src_order.data_ptr()
+        a.act, a.pred = b["act"].data_ptr(), b["pred"].data_ptr()
+        a.dpred = dpred.data_ptr() if dpred is not None else None
+        return a
+
     def forward(self, xn, xe, gb):
         """Prediction [nodes][out] for node features xn and edge features xe (float32 device
         tensors) on the stacked graph gb; keeps the activations for backward()."""
         N, E = xn.shape[0], xe.shape[0]
         b = self._buffers(N, E)
+        if self.whole:
+            cb._check(cb.lib().cfd_mpnn_net_forward(ctypes.byref(self._net(xn, xe, gb)), _stream(xn)))
+            self._graph = gb
+            self._x = (xn, xe)
+            return b["pred"]
         h, e, agg = b["h"], b["e"], b["agg"]
         self._mlp("enc_n", [_seg(xn)], N, h[0], b["z_enc_n"])
         self._mlp("enc_e", [_seg(xe)], E, e[0], b["z_enc_e"])
@@ -425,6 +452,9 @@ class Net:
         """Gradients of every parameter (into self.grad) from the prediction gradient dpred."""
         b, gb, W, L = self._bufs, self._graph, self.HIDDEN, self.L
         xn, xe = self._x
+        if self.whole:
+            cb._check(cb.lib().cfd_mpnn_net_backward(ctypes.byref(self._net(xn, xe, gb, dpred)), _stream(dpred)))
+            return
         N, E = xn.shape[0], xe.shape[0]
         lib, st = cb.lib(), _stream(dpred)
         dh, de, dx = b["dh"], b["de"], b["dx"]

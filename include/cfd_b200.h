@@ -493,6 +493,32 @@ typedef struct {
 cfd_status cfd_mpnn_weight_grad(const cfd_mlp_wgrad *a, void *stream);
 int cfd_mpnn_wgrad_blocks(void);
 
+/* Whole passes of the message-passing network (mma.sync blocks; the launches of cfd_mpnn_mlp_*,
+ * cfd_mpnn_weight_grad and the segment sums issued by one call, with the same sums in the same order,
+ * so the results are those of the single calls).  Blocks, hidden width 64, residual updates:
+ *   h = enc_n(xn), e = enc_e(xe);  per layer e += edge_l(h[src], h[dst], e),
+ *   agg[n] = sum of e over rows dst_ptr[n] .. dst_ptr[n+1], h += node_l(h, agg);  pred = dec(h).
+ * params / grads: per block W1 [64][in], b1, W2 [out][64], b2 in the order enc_n, enc_e, edge_0..,
+ * node_0.., dec; 16-byte aligned.  act: cfd_mpnn_net_floats(...) floats, 16-byte aligned, holds the
+ * activations from forward to backward.  The edges are sorted by dst; src_order lists them by src
+ * (CSR src_ptr).  backward overwrites grads; workspace as in cfd_mlp_wgrad for in_width 192. */
+typedef struct {
+  int layers, node_in, edge_in, out; /* out <= 16 */
+  int n_nodes, n_edges;
+  const float *params;
+  float *grads;                /* backward only */
+  const float *xn, *xe;        /* [n_nodes][node_in], [n_edges][edge_in] */
+  const int *src, *dst, *dst_ptr;
+  const int *src_ptr, *src_order; /* backward only */
+  float *act;
+  float *pred;                 /* out [n_nodes][out] */
+  const float *dpred;          /* backward only */
+  float *workspace;            /* backward only */
+} cfd_mpnn_net;
+size_t cfd_mpnn_net_floats(int layers, int node_in, int edge_in, int out, int n_nodes, int n_edges);
+cfd_status cfd_mpnn_net_forward(const cfd_mpnn_net *n, void *stream);
+cfd_status cfd_mpnn_net_backward(const cfd_mpnn_net *n, void *stream);
+
 /* Helpers of the training step (float32, device pointers, leading dimensions in elements):
  * out = a + b on a [rows][width] window; out[r] += src[idx[r]]; out[r] (+)= sum over the CSR list
  * of row r of x[idx[j]] in list order; the mean-squared error of n values with its gradient
