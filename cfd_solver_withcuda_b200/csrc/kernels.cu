@@ -263,7 +263,7 @@ __device__ __forceinline__ bool last_block(unsigned int *counter) {
 // partial[9 nb + q * ngroups + group], and the last group to finish reduces those in group order
 // into out[9] (shared memory).  Both rounds are a single set of independent loads, and the group
 // rounds run while other blocks are still working.  Returns true in the block that wrote out.
-__device__ __forceinline__ bool grid_reduce9(DevState &st, double *out) {
+__device__ __forceinline__ bool grid_reduce9(const DevState &st, double *out) {
   __shared__ bool flag;
   const int nb = gridDim.x;
   const int G = max(32, (nb + kMaxGroups - 1) / kMaxGroups);
@@ -313,7 +313,7 @@ __global__ void k_prim_all(DevMesh m, DevState st) {
 //   fixed-p exit     src/Exit_Boundary_Conditions.cpp:8-66 (exit kind 3)
 // src_is_S: the supersonic-exit copy reads the stage state (stage-consistent forms) instead of
 // U^n; cur_is_S: the state the primitives were last computed from is the stage state.
-__device__ __forceinline__ void bc_entry(const DevMesh &m, DevState &st, const BcParams &bp, int e, int src_is_S,
+__device__ __forceinline__ void bc_entry(const DevMesh &m, const DevState &st, const BcParams &bp, int e, int src_is_S,
                                          int cur_is_S) {
   const int4 b = m.bnd[e];
   const int kind = b.x, c = b.y, f = b.z, g = b.w;
@@ -474,8 +474,8 @@ __device__ __forceinline__ void load_cell(const DevMesh &m, const DevState &st, 
 
 // Contribution of face f of cell c: X = avg - diss (Calculate_Flux_For_All_Faces,
 // src/Net_Flux.cpp:18-43) and the del_t term (|V.n| + a) dl (src/Time_Step.cpp:326-336).
-template <int DISS, int ORDER>
-__device__ __forceinline__ void face_contrib(const DevMesh &m, const DevState &st, const FluxParams &fp,
+template <int DISS, int ORDER, typename O>
+__device__ __forceinline__ void face_contrib(O &o, const DevMesh &m, const DevState &st, const FluxParams &fp,
                                              const USrc &us, const CellState &q, int c, int f, double X[4],
                                              double &t) {
   const int NP = m.NP, NT = m.NT;
@@ -489,20 +489,25 @@ __device__ __forceinline__ void face_contrib(const DevMesh &m, const DevState &s
   if (DISS != 6 && DISS != 7) average_flux<double>(rc, uc, vc, pc, rn, un, vn, pn, nx, ny, dl, A);
   if (DISS == 3 && ORDER == 1) {
     if (N >= NP)
-      roe_1o<double>(rc, uc, vc, pc, ac, rc, uc, vc, pc, ac, nx, ny, dl, (q.degen >> f) & 1, D);
+      roe_1o<double>(o, rc, uc, vc, pc, ac, rc, uc, vc, pc, ac, nx, ny, dl, (q.degen >> f) & 1, D);
     else
-      roe_1o<double>(rc, uc, vc, pc, ac, rn, un, vn, pn, an, nx, ny, dl, (q.degen >> f) & 1, D);
+      roe_1o<double>(o, rc, uc, vc, pc, ac, rn, un, vn, pn, an, nx, ny, dl, (q.degen >> f) & 1, D);
   } else if (DISS == 3 && ORDER == 2) {
     const int n2 = m.n2[idx];
     const double d1 = m.d1l[idx], d2 = m.d2l[idx];
-    double dU[4];
+    double dU[4], phi[4];
     if (!fp.recon_prim) {
+      double q1[4], q2[4];
 #pragma unroll
       for (int k = 0; k < 4; k++) {
-        const double q1 = us.get(k, N), q2 = us.get(k, n2);
-        const double phi = limited_slope<double>(fp.limiter, q.Uc[k], q1, q2, d1, d2, fp.zeta, fp.zeta1);
-        const double VR = q1 + 0.5 * phi * d1;
-        const double VL = q.Uc[k] - 0.5 * phi * d1;
+        q1[k] = us.get(k, N);
+        q2[k] = us.get(k, n2);
+      }
+      limited_slopes<double>(o, fp.limiter, q.Uc, q1, q2, d1, d2, fp.zeta, fp.zeta1, phi);
+#pragma unroll
+      for (int k = 0; k < 4; k++) {
+        const double VR = q1[k] + 0.5 * phi[k] * d1;
+        const double VL = q.Uc[k] - 0.5 * phi[k] * d1;
         dU[k] = VR - VL;
       }
     } else {
@@ -512,19 +517,19 @@ __device__ __forceinline__ void face_contrib(const DevMesh &m, const DevState &s
       const double q1v[4] = {rn, un, vn, pn};
       const double q2v[4] = {prim[n2], prim[NT + n2], prim[2 * NT + n2], prim[3 * NT + n2]};
       double qR[4], qL[4];
+      limited_slopes<double>(o, fp.limiter, qc, q1v, q2v, d1, d2, fp.zeta, fp.zeta1, phi);
 #pragma unroll
       for (int k = 0; k < 4; k++) {
-        const double phi = limited_slope<double>(fp.limiter, qc[k], q1v[k], q2v[k], d1, d2, fp.zeta, fp.zeta1);
-        qR[k] = q1v[k] + 0.5 * phi * d1;
-        qL[k] = qc[k] - 0.5 * phi * d1;
+        qR[k] = q1v[k] + 0.5 * phi[k] * d1;
+        qL[k] = qc[k] - 0.5 * phi[k] * d1;
       }
       dU[0] = qR[0] - qL[0];
       dU[1] = qR[0] * qR[1] - qL[0] * qL[1];
       dU[2] = qR[0] * qR[2] - qL[0] * qL[2];
-      dU[3] = (qR[3] / kGM1 + 0.5 * qR[0] * (qR[1] * qR[1] + qR[2] * qR[2])) -
-              (qL[3] / kGM1 + 0.5 * qL[0] * (qL[1] * qL[1] + qL[2] * qL[2]));
+      dU[3] = (o.div_gm1(qR[3]) + 0.5 * qR[0] * (qR[1] * qR[1] + qR[2] * qR[2])) -
+              (o.div_gm1(qL[3]) + 0.5 * qL[0] * (qL[1] * qL[1] + qL[2] * qL[2]));
     }
-    roe_2o<double>(rc, uc, vc, pc, ac, rn, un, vn, pn, an, nx, ny, dl, dU, D);
+    roe_2o<double>(o, rc, uc, vc, pc, ac, rn, un, vn, pn, an, nx, ny, dl, dU, D);
   } else if (DISS == 2 || DISS == 4 || DISS == 5) {
     // MOVERS, RICCA, MOVERS_NWSC and their second-order forms (src/MOVERS.cpp, src/RICCA.cpp,
     // src/MOVERS_NWSC.cpp); RICCA_2O and MOVERS_NWSC_2O take the limited conserved jump of
@@ -537,22 +542,24 @@ __device__ __forceinline__ void face_contrib(const DevMesh &m, const DevState &s
     if (ORDER == 2 && DISS != 2) {
       const int n2 = m.n2[idx];
       const double d1 = m.d1l[idx], d2 = m.d2l[idx];
+      double q2[4], phi[4];
+#pragma unroll
+      for (int k = 0; k < 4; k++) q2[k] = us.get(k, n2);
+      limited_slopes<double>(o, fp.limiter, q.Uc, UR, q2, d1, d2, fp.zeta, fp.zeta1, phi);
 #pragma unroll
       for (int k = 0; k < 4; k++) {
-        const double q2 = us.get(k, n2);
-        const double phi = limited_slope<double>(fp.limiter, q.Uc[k], UR[k], q2, d1, d2, fp.zeta, fp.zeta1);
-        const double VR = UR[k] + 0.5 * phi * d1;
-        const double VL = q.Uc[k] - 0.5 * phi * d1;
+        const double VR = UR[k] + 0.5 * phi[k] * d1;
+        const double VL = q.Uc[k] - 0.5 * phi[k] * d1;
         dU2[k] = VR - VL;
       }
     }
     if (DISS == 2)
-      movers_diss<double, ORDER>(rc, uc, vc, pc, ac, rn, un, vn, pn, an, q.Uc, UR, nx, ny, dl, fp.movers_single,
+      movers_diss<double, ORDER>(o, rc, uc, vc, pc, ac, rn, un, vn, pn, an, q.Uc, UR, nx, ny, dl, fp.movers_single,
                                  fp.movers_efix, D);
     else if (DISS == 4)
-      ricca_diss<double, ORDER>(rc, uc, vc, pc, rn, un, vn, pn, nx, ny, dl, dU2, D);
+      ricca_diss<double, ORDER>(o, rc, uc, vc, pc, rn, un, vn, pn, nx, ny, dl, dU2, D);
     else
-      nwsc_diss<double, ORDER>(rc, uc, vc, pc, rn, un, vn, pn, q.Uc, UR, nx, ny, dl, dU2, D);
+      nwsc_diss<double, ORDER>(o, rc, uc, vc, pc, rn, un, vn, pn, q.Uc, UR, nx, ny, dl, dU2, D);
   } else if (DISS == 6 || DISS == 7) {
     // Reference forms of AUSM (src/Ausm_Flux.cpp:26-34, from U_Cells) and HLLC
     // (CUDA_KERNELS/HLLC_LLF_Flux_Cuda_Kernels.cu:98-100): faces whose neighbour is a ghost are
@@ -564,10 +571,10 @@ __device__ __forceinline__ void face_contrib(const DevMesh &m, const DevState &s
 #pragma unroll
       for (int k = 0; k < 4; k++) UR[k] = us.get(k, N);
       if (DISS == 6) {
-        ausm_face<double>(q.Uc, UR, nx, ny, dl, A);
+        ausm_face<double>(o, q.Uc, UR, nx, ny, dl, A);
       } else {
         const double qL[5] = {rc, uc, vc, pc, ac}, qR[5] = {rn, un, vn, pn, an};
-        hllc_face<double>(qL, q.Uc, qR, UR, nx, ny, dl, A);
+        hllc_face<double>(o, qL, q.Uc, qR, UR, nx, ny, dl, A);
       }
     }
   } else {  // LLF 1O
@@ -594,7 +601,7 @@ __device__ __forceinline__ double cell_dt(const DevMesh &m, const FluxParams &fp
 
 // Block min of del_t to `partial`; the last block writes Min_dt (get_Min_dt,
 // src/Numerical_Method.cpp:322-330).
-__device__ __forceinline__ void min_dt_epilogue(DevState &st, double dt, double *sh) {
+__device__ __forceinline__ void min_dt_epilogue(const DevState &st, double dt, double *sh) {
   double bm = block_min(dt, sh);
   if (threadIdx.x == 0) st.partial[blockIdx.x] = bm;
   if (last_block(st.counter)) {
@@ -611,37 +618,66 @@ __device__ __forceinline__ void min_dt_epilogue(DevState &st, double dt, double 
   }
 }
 
+// Contribution of one face with the plain operators: for faces whose branch-free evaluation met an
+// operand outside its range.
+template <int DISS, int ORDER>
+__device__ __noinline__ double4 face_contrib_again(const DevMesh &m, const DevState &st, const FluxParams &fp,
+                                                   int use_S, int c, int f) {
+  const USrc us{st.U, st.S, m.NT, m.NP, use_S};
+  Ieee<double> o;
+  CellState q;
+  load_cell<DISS, ORDER>(m, st, us, c, q);
+  double X[4], t;
+  face_contrib<DISS, ORDER>(o, m, st, fp, us, q, c, f, X, t);
+  return make_double4(X[0], X[1], X[2], X[3]);
+}
+
 // Evaluate_Cell_Net_Flux_1O/2O (src/Net_Flux.cpp:46-129) + Evaluate_Time_Step (src/Time_Step.cpp:293-359)
 // fused, one thread per cell: faces in order, Net += avg - diss; then del_t; block min + Min_dt.
 // MINB: minimum resident blocks per SM the register allocation is made for (1: unconstrained;
-// the second-order forms with the directional limiter are also built for 6 and 8, which cap
-// their 114 - 124 registers at 80 and 64 for more resident warps; the autotuner picks, the
-// results are the same bits).  SRC_S false: the conserved states come from U only (the caller
-// knows no stage state is read), which saves the per-load choice between U and the stage state.
+// the second-order forms with the directional limiter are also built for 6 and 8 for more resident
+// warps; the autotuner picks, the results are the same bits).  SRC_S false: the conserved states
+// come from U only (the caller knows no stage state is read), which saves the per-load choice
+// between U and the stage state.  The divisions and square roots are the branch-free ones (Fast64),
+// so the four faces' chains interleave; a cell with an operand outside their range is evaluated again.
 template <int DISS, int ORDER, int MINB = 1, bool SRC_S = true>
-__global__ void __launch_bounds__(kFluxBlock, MINB) k_flux(DevMesh m, DevState st, FluxParams fp, int src_is_S) {
+__global__ void __launch_bounds__(kFluxBlock, MINB) k_flux(const __grid_constant__ DevMesh m,
+                                                           const __grid_constant__ DevState st,
+                                                           const __grid_constant__ FluxParams fp, int src_is_S) {
   __shared__ double sh[32];
   const int NP = m.NP, NT = m.NT;
   const int c = blockIdx.x * blockDim.x + threadIdx.x;
   const bool done = step_done(st.ctl);
   double dt = 1e308 * 10.0;
   if (c < NP && !done) {
-    const USrc us{st.U, st.S, NT, NP, SRC_S && fp.consistent && src_is_S};
+    const int use_S = SRC_S && fp.consistent && src_is_S;
+    const USrc us{st.U, st.S, NT, NP, use_S};
     CellState q;
     load_cell<DISS, ORDER>(m, st, us, c, q);
     const int nf = m.nf[c];
     double N0 = 0.0, N1s = 0.0, N2s = 0.0, N3s = 0.0;
     double den = 0.0;
+    Fast64 o;
 #pragma unroll
     for (int f = 0; f < 4; f++) {
       if (f < nf) {
         double X[4], t;
-        face_contrib<DISS, ORDER>(m, st, fp, us, q, c, f, X, t);
+        face_contrib<DISS, ORDER>(o, m, st, fp, us, q, c, f, X, t);
         N0 += X[0];
         N1s += X[1];
         N2s += X[2];
         N3s += X[3];
         den += t;
+      }
+    }
+    if (o.bad()) {
+      N0 = N1s = N2s = N3s = 0.0;
+      for (int f = 0; f < nf; f++) {
+        const double4 X = face_contrib_again<DISS, ORDER>(m, st, fp, use_S, c, f);
+        N0 += X.x;
+        N1s += X.y;
+        N2s += X.z;
+        N3s += X.w;
       }
     }
     dt = cell_dt(m, fp, c, den);
@@ -660,7 +696,9 @@ __global__ void __launch_bounds__(kFluxBlock, MINB) k_flux(DevMesh m, DevState s
 // reference's order and value; fewer live registers per thread give the SM more warps to hide
 // the gather and FP64 latencies.
 template <int DISS, int ORDER>
-__global__ void __launch_bounds__(kFlux4Block) k_flux4(DevMesh m, DevState st, FluxParams fp, int src_is_S) {
+__global__ void __launch_bounds__(kFlux4Block) k_flux4(const __grid_constant__ DevMesh m,
+                                                       const __grid_constant__ DevState st,
+                                                       const __grid_constant__ FluxParams fp, int src_is_S) {
   __shared__ double sh[32];
   const int NP = m.NP, NT = m.NT;
   const int gid = blockIdx.x * blockDim.x + threadIdx.x;
@@ -671,10 +709,19 @@ __global__ void __launch_bounds__(kFlux4Block) k_flux4(DevMesh m, DevState st, F
   const int nf = cell_ok ? m.nf[c] : 0;
   double X[4] = {0.0, 0.0, 0.0, 0.0}, t = 0.0;
   if (f < nf) {
-    const USrc us{st.U, st.S, NT, NP, fp.consistent && src_is_S};
+    const int use_S = fp.consistent && src_is_S;
+    const USrc us{st.U, st.S, NT, NP, use_S};
     CellState q;
     load_cell<DISS, ORDER>(m, st, us, c, q);
-    face_contrib<DISS, ORDER>(m, st, fp, us, q, c, f, X, t);
+    Fast64 o;
+    face_contrib<DISS, ORDER>(o, m, st, fp, us, q, c, f, X, t);
+    if (o.bad()) {
+      const double4 Y = face_contrib_again<DISS, ORDER>(m, st, fp, use_S, c, f);
+      X[0] = Y.x;
+      X[1] = Y.y;
+      X[2] = Y.z;
+      X[3] = Y.w;
+    }
   }
   double Y[3][4], T[3];
 #pragma unroll
@@ -851,8 +898,8 @@ __global__ void __launch_bounds__(kFluxBlock) k_weno(DevMesh m, DevState st, Flu
 // fp.eflin > 0).
 // Flux of one unique face from the owner's record (c0: rho, u, v, p; c1, c2: gradients) and the
 // neighbour's (n0, n1, n2), face normal (nx, ny), length dl and centre-to-centre vector (dx, dy).
-template <typename T, int DISS>
-__device__ __forceinline__ double4 face_flux_rec(int glim, const double4 c0, const double4 c1, const double4 c2,
+template <typename T, int DISS, typename O>
+__device__ __forceinline__ double4 face_flux_rec(O &o, int glim, const double4 c0, const double4 c1, const double4 c2,
                                                  const double4 n0, const double4 n1, const double4 n2, const T nx,
                                                  const T ny, const T dl, const T dx, const T dy, const T eflin,
                                                  const T shock_fix = T(0.0)) {
@@ -860,14 +907,45 @@ __device__ __forceinline__ double4 face_flux_rec(int glim, const double4 c0, con
   const T qn[4] = {T(n0.x), T(n0.y), T(n0.z), T(n0.w)};
   const T gc[8] = {T(c1.x), T(c1.y), T(c1.z), T(c1.w), T(c2.x), T(c2.y), T(c2.z), T(c2.w)};
   const T gn[8] = {T(n1.x), T(n1.y), T(n1.z), T(n1.w), T(n2.x), T(n2.y), T(n2.z), T(n2.w)};
-  T qL[4], qR[4];
+  T qL[4], qR[4], dp[4], dmc[4], dmn[4];
 #pragma unroll
   for (int k = 0; k < 4; k++) {
-    const T dp = qn[k] - qc[k];
-    const T dmc = T(2.0) * (gc[2 * k] * dx + gc[2 * k + 1] * dy) - dp;
-    const T dmn = T(2.0) * (gn[2 * k] * dx + gn[2 * k + 1] * dy) - dp;
-    qL[k] = qc[k] + T(0.5) * muscl_slope<T>(glim, dmc, dp);
-    qR[k] = qn[k] - T(0.5) * muscl_slope<T>(glim, dmn, dp);
+    dp[k] = qn[k] - qc[k];
+    dmc[k] = T(2.0) * (gc[2 * k] * dx + gc[2 * k + 1] * dy) - dp[k];
+    dmn[k] = T(2.0) * (gn[2 * k] * dx + gn[2 * k + 1] * dy) - dp[k];
+  }
+  // The slopes.  Fast64: one branch on the limiter for all eight, so that their divisions interleave.
+  bool limited = false;
+  if constexpr (O::fast) {
+    if (glim == LIM_VANLEER) {
+      limited = true;
+#pragma unroll
+      for (int k = 0; k < 4; k++) {
+        qL[k] = qc[k] + 0.5 * muscl_slope_fast<LIM_VANLEER>(o, dmc[k], dp[k]);
+        qR[k] = qn[k] - 0.5 * muscl_slope_fast<LIM_VANLEER>(o, dmn[k], dp[k]);
+      }
+    } else if (glim == LIM_VANALBADA) {
+      limited = true;
+#pragma unroll
+      for (int k = 0; k < 4; k++) {
+        qL[k] = qc[k] + 0.5 * muscl_slope_fast<LIM_VANALBADA>(o, dmc[k], dp[k]);
+        qR[k] = qn[k] - 0.5 * muscl_slope_fast<LIM_VANALBADA>(o, dmn[k], dp[k]);
+      }
+    } else if (glim == LIM_MINMOD) {
+      limited = true;
+#pragma unroll
+      for (int k = 0; k < 4; k++) {
+        qL[k] = qc[k] + 0.5 * muscl_slope<T>(LIM_MINMOD, dmc[k], dp[k]);
+        qR[k] = qn[k] - 0.5 * muscl_slope<T>(LIM_MINMOD, dmn[k], dp[k]);
+      }
+    }
+  }
+  if (!limited) {
+#pragma unroll
+    for (int k = 0; k < 4; k++) {
+      qL[k] = qc[k] + T(0.5) * muscl_slope<T>(glim, dmc[k], dp[k]);
+      qR[k] = qn[k] - T(0.5) * muscl_slope<T>(glim, dmn[k], dp[k]);
+    }
   }
   if (!(qL[0] > T(0.0)) || !(qL[3] > T(0.0))) {
 #pragma unroll
@@ -877,7 +955,7 @@ __device__ __forceinline__ double4 face_flux_rec(int glim, const double4 c0, con
 #pragma unroll
     for (int k = 0; k < 4; k++) qR[k] = qn[k];
   }
-  const T aL = sqrt(T(kGamma) * qL[3] / qL[0]), aR = sqrt(T(kGamma) * qR[3] / qR[0]);
+  const T aL = o.root(o.div(T(kGamma) * qL[3], qL[0])), aR = o.root(o.div(T(kGamma) * qR[3], qR[0]));
   T A[4], D[4] = {T(0.0), T(0.0), T(0.0), T(0.0)};
   // DISS 3: Roe; DISS 103: Roe with the options of the form (linear-wave entropy fix, shock-stable
   // hybrid), a separate instance so that the plain form keeps its register footprint.
@@ -896,35 +974,62 @@ __device__ __forceinline__ double4 face_flux_rec(int glim, const double4 c0, con
       const T sL = fabs(vnL) + aL, sR = fabs(vnR) + aR;
       const T sm = sL > sR ? sL : sR;
       const T UL[4] = {qL[0], qL[0] * qL[1], qL[0] * qL[2],
-                       qL[3] / T(kGM1) + T(0.5) * qL[0] * (qL[1] * qL[1] + qL[2] * qL[2])};
+                       o.div_gm1(qL[3]) + T(0.5) * qL[0] * (qL[1] * qL[1] + qL[2] * qL[2])};
       const T UR[4] = {qR[0], qR[0] * qR[1], qR[0] * qR[2],
-                       qR[3] / T(kGM1) + T(0.5) * qR[0] * (qR[1] * qR[1] + qR[2] * qR[2])};
+                       o.div_gm1(qR[3]) + T(0.5) * qR[0] * (qR[1] * qR[1] + qR[2] * qR[2])};
 #pragma unroll
       for (int k = 0; k < 4; k++) D[k] = T(0.5) * sm * (UR[k] - UL[k]) * dl;
     } else {
-      roe_1o<T>(qL[0], qL[1], qL[2], qL[3], aL, qR[0], qR[1], qR[2], qR[3], aR, nx, ny, dl, false, D,
+      roe_1o<T>(o, qL[0], qL[1], qL[2], qL[3], aL, qR[0], qR[1], qR[2], qR[3], aR, nx, ny, dl, false, D,
                 DISS == 103 ? eflin : T(0.0));
     }
   } else {
     // Conserved face states for AUSM / HLLC: E = p/(g-1) + rho |V|^2 / 2.
     const T UL[4] = {qL[0], qL[0] * qL[1], qL[0] * qL[2],
-                     qL[3] / T(kGM1) + T(0.5) * qL[0] * (qL[1] * qL[1] + qL[2] * qL[2])};
+                     o.div_gm1(qL[3]) + T(0.5) * qL[0] * (qL[1] * qL[1] + qL[2] * qL[2])};
     const T UR[4] = {qR[0], qR[0] * qR[1], qR[0] * qR[2],
-                     qR[3] / T(kGM1) + T(0.5) * qR[0] * (qR[1] * qR[1] + qR[2] * qR[2])};
+                     o.div_gm1(qR[3]) + T(0.5) * qR[0] * (qR[1] * qR[1] + qR[2] * qR[2])};
     if (DISS == 6) {
-      ausm_face<T>(UL, UR, nx, ny, dl, A);
+      ausm_face<T>(o, UL, UR, nx, ny, dl, A);
     } else if (DISS == 8) {
       ausm_gpu_face<T>(UL, UR, nx, ny, dl, A);
     } else {
       const T q5L[5] = {qL[0], qL[1], qL[2], qL[3], aL}, q5R[5] = {qR[0], qR[1], qR[2], qR[3], aR};
-      hllc_face<T>(q5L, UL, q5R, UR, nx, ny, dl, A);
+      hllc_face<T>(o, q5L, UL, q5R, UR, nx, ny, dl, A);
     }
   }
   return make_double4(double(A[0] - D[0]), double(A[1] - D[1]), double(A[2] - D[2]), double(A[3] - D[3]));
 }
 
+// Division policy of the face kernels: the branch-free double operations, or plain float ones.
+template <typename T>
+using FaceOps = typename std::conditional<std::is_same<T, double>::value, Fast64, Ieee<float>>::type;
+
+__device__ __forceinline__ double4 ldcg4(const double4 *p) {
+  const double2 a = __ldcg(reinterpret_cast<const double2 *>(p));
+  const double2 b = __ldcg(reinterpret_cast<const double2 *>(p) + 1);
+  return make_double4(a.x, a.y, b.x, b.y);
+}
+
+// Flux of face i with the plain operators: for faces whose branch-free evaluation met an operand
+// outside its range.  Loads from L2 (the persistent kernel writes rows and records in its launch).
+template <int DISS>
+__device__ __noinline__ double4 face_flux_again(const DevMesh &m, const DevState &st, const FluxParams &fp, int i) {
+  const int2 on = m.fon[i];
+  const double4 gq = m.fg4[i];
+  const int g = on.y < m.NP ? on.y : on.x;  // a ghost neighbour uses the owner's gradients
+  const double4 *rc = reinterpret_cast<const double4 *>(st.rec + 8 * (size_t)on.x);
+  const double4 *rn = reinterpret_cast<const double4 *>(st.rec + 8 * (size_t)g);
+  Ieee<double> o;
+  return face_flux_rec<double, DISS>(o, fp.limiter == LIM_REF_MINMOD ? LIM_MINMOD : fp.limiter, ldcg4(st.q4 + on.x),
+                                     ldcg4(rc), ldcg4(rc + 1), ldcg4(st.q4 + on.y), ldcg4(rn), ldcg4(rn + 1), gq.x, gq.y,
+                                     gq.z, gq.w, m.fdy[i], fp.eflin, fp.shock_fix);
+}
+
 template <typename T, int DISS, int MINB>
-__global__ void __launch_bounds__(MINB >= 6 ? 128 : 256, MINB) k_faces(DevMesh m, DevState st, FluxParams fp) {
+__global__ void __launch_bounds__(MINB >= 6 ? 128 : 256, MINB) k_faces(const __grid_constant__ DevMesh m,
+                                                                          const __grid_constant__ DevState st,
+                                                                          const __grid_constant__ FluxParams fp) {
   pdl_enter();
   const int i = item_index(m.fblk, m.NF);
   if (i >= m.NF || step_done(st.ctl)) return;
@@ -959,8 +1064,12 @@ __global__ void __launch_bounds__(MINB >= 6 ? 128 : 256, MINB) k_faces(DevMesh m
     n1 = nphys ? rn[0] : c1;
     n2 = nphys ? rn[1] : c2;
   }
-  st.F[i] = face_flux_rec<T, DISS>(glim, c0, c1, c2, n0, n1, n2, nx, ny, dl, dx, dy, T(fp.eflin),
-                                     T(fp.shock_fix));
+  FaceOps<T> o;
+  double4 F = face_flux_rec<T, DISS>(o, glim, c0, c1, c2, n0, n1, n2, nx, ny, dl, dx, dy, T(fp.eflin), T(fp.shock_fix));
+  if constexpr (FaceOps<T>::fast) {
+    if (o.bad()) F = face_flux_again<DISS>(m, st, fp, i);
+  }
+  st.F[i] = F;
 }
 
 // Sum of the face fluxes of cell c in face order (+F on the owner side, -F on the neighbour
@@ -969,12 +1078,6 @@ __global__ void __launch_bounds__(MINB >= 6 ? 128 : 256, MINB) k_faces(DevMesh m
 // face are in flight together; only the sums are predicated on the count.
 // CG: the face fluxes were written earlier in the same launch by other thread blocks (the
 // persistent stage kernel), so they are loaded from L2 (ld.global.cg), not through L1.
-__device__ __forceinline__ double4 ldcg4(const double4 *p) {
-  const double2 a = __ldcg(reinterpret_cast<const double2 *>(p));
-  const double2 b = __ldcg(reinterpret_cast<const double2 *>(p) + 1);
-  return make_double4(a.x, a.y, b.x, b.y);
-}
-
 template <bool DEN = true, bool CG = false>
 __device__ __forceinline__ void gather_faces(const DevMesh &m, const DevState &st, int c, double R[4], double &den) {
   const int NP = m.NP, NT = m.NT;
@@ -1045,7 +1148,7 @@ __device__ __forceinline__ double err_term(double du, double u) {
 
 // Per-block partial sums (4 error terms, 4 residual squares), then the last block reduces the
 // partials in block order and applies the step epilogue (Total_Time += Min_dt, iterations++).
-__device__ __forceinline__ void reduce_err_and_epilogue(DevState &st, const double e[8], bool advance_time,
+__device__ __forceinline__ void reduce_err_and_epilogue(const DevState &st, const double e[8], bool advance_time,
                                                         double dt_for_time) {
   __shared__ double sh[8 * 32];
   double v[8];
@@ -1104,7 +1207,7 @@ __device__ __forceinline__ void load_stage_in(const DevMesh &m, const DevState &
   }
 }
 
-__device__ __forceinline__ void cell_update_in(const DevMesh &m, DevState &st, int c, int kind, double dt,
+__device__ __forceinline__ void cell_update_in(const DevMesh &m, const DevState &st, int c, int kind, double dt,
                                                const double Rk[4], const StageIn &in, int fuse_final, int keep_delu,
                                                double e[8]) {
   const int NP = m.NP, NT = m.NT;
@@ -1209,7 +1312,7 @@ __device__ __forceinline__ void cell_update_in(const DevMesh &m, DevState &st, i
   }
 }
 
-__device__ __forceinline__ void cell_update(const DevMesh &m, DevState &st, int c, int kind, double dt,
+__device__ __forceinline__ void cell_update(const DevMesh &m, const DevState &st, int c, int kind, double dt,
                                             const double Rk[4], int fuse_final, int keep_delu, double e[8]) {
   StageIn in;
   load_stage_in(m, st, c, kind, in);
@@ -1256,7 +1359,7 @@ __global__ void __launch_bounds__(kBlock) k_stage(DevMesh m, DevState st, int ki
 // next stage).  Returns the dt used.
 // stage_cell_in: the same with the stage inputs and the frozen dt already loaded (the TMA tile
 // form prefetches them into shared memory).
-__device__ __forceinline__ double stage_cell_in(const DevMesh &m, DevState &st, const BcParams &bp, int c,
+__device__ __forceinline__ double stage_cell_in(const DevMesh &m, const DevState &st, const BcParams &bp, int c,
                                                 const double R[4], double dtc, double dt_frozen, const StageIn &in,
                                                 int kind, int lts, int fuse_final, int keep_delu, int flags,
                                                 double e[8]) {
@@ -1277,7 +1380,7 @@ __device__ __forceinline__ double stage_cell_in(const DevMesh &m, DevState &st, 
   }
   return dt;
 }
-__device__ __forceinline__ double stage_cell(const DevMesh &m, DevState &st, const BcParams &bp, int c,
+__device__ __forceinline__ double stage_cell(const DevMesh &m, const DevState &st, const BcParams &bp, int c,
                                              const double R[4], double dtc, int kind, int lts, int fuse_final,
                                              int keep_delu, int flags, double e[8]) {
   StageIn in;
@@ -1291,7 +1394,7 @@ __device__ __forceinline__ double stage_cell(const DevMesh &m, DevState &st, con
 // over the grid, then the Total_Time epilogue of the loop body.  Called by every thread.
 // stage_final_reduce_sm: the same with its scratch (32 + 8 * 32 + 9 doubles) in caller-provided
 // shared memory.
-__device__ __forceinline__ void stage_final_reduce_sm(DevState &st, const double e[8], double dtu, double *scratch) {
+__device__ __forceinline__ void stage_final_reduce_sm(const DevState &st, const double e[8], double dtu, double *scratch) {
   double *sh = scratch, *sh8 = scratch + 32, *red = scratch + 32 + 8 * 32;
   const double sq = block_sums8(e, sh8);
   if (threadIdx.x < 8) st.partial[(1 + threadIdx.x) * gridDim.x + blockIdx.x] = sq;
@@ -1308,7 +1411,7 @@ __device__ __forceinline__ void stage_final_reduce_sm(DevState &st, const double
     if (te > 0.0 && t >= te) st.ctl[CTL_DONE] = 1.0;
   }
 }
-__device__ __forceinline__ void stage_final_reduce(DevState &st, const double e[8], double dtu) {
+__device__ __forceinline__ void stage_final_reduce(const DevState &st, const double e[8], double dtu) {
   __shared__ double scratch[32 + 8 * 32 + 9];
   stage_final_reduce_sm(st, e, dtu, scratch);
 }
@@ -1555,8 +1658,8 @@ __device__ __forceinline__ void grid_barrier(unsigned int *count, unsigned int *
 // registers and a small spill, 24 warps per SM; 8: 64 registers).  On a batch of 128 ramps on B200
 // the FP64 form runs fastest at 6 (25 % faster than at 4) and the FP32-flux form at 8.
 template <typename T, int DISS, int MINB>
-__global__ void __launch_bounds__(kPersistBlock, MINB) k_persistent_stage(DevMesh m, DevState st, FluxParams fp,
-                                                                       BcParams bp, int kind, int lts, int fuse_final,
+__global__ void __launch_bounds__(kPersistBlock, MINB) k_persistent_stage(const __grid_constant__ DevMesh m, const __grid_constant__ DevState st,
+                                                                       const __grid_constant__ FluxParams fp, BcParams bp, int kind, int lts, int fuse_final,
                                                                        int keep_delu, int flags, int with_dt,
                                                                        int with_bc, unsigned int test_arrivals) {
   const int NP = m.NP;
@@ -1625,8 +1728,13 @@ __global__ void __launch_bounds__(kPersistBlock, MINB) k_persistent_stage(DevMes
         n1 = nphys ? ldcg4(rn) : c1;
         n2 = nphys ? ldcg4(rn + 1) : c2;
       }
-      st.F[i] = face_flux_rec<T, DISS>(glim, c0, c1, c2, n0, n1, n2, nx, ny, dl, dx, dy, T(fp.eflin),
-                                     T(fp.shock_fix));
+      FaceOps<T> o;
+      double4 F = face_flux_rec<T, DISS>(o, glim, c0, c1, c2, n0, n1, n2, nx, ny, dl, dx, dy, T(fp.eflin),
+                                         T(fp.shock_fix));
+      if constexpr (FaceOps<T>::fast) {
+        if (o.bad()) F = face_flux_again<DISS>(m, st, fp, i);
+      }
+      st.F[i] = F;
     }
   }
   grid_barrier(bar_count, bar_gen, st.status, test_arrivals);
@@ -1727,7 +1835,8 @@ __global__ void __launch_bounds__(kPatchCells, 5) k_patch_stage(DevMesh m, DevSt
       n1r = make_double4(srec[4 * rows + ln], srec[5 * rows + ln], srec[6 * rows + ln], srec[7 * rows + ln]);
       n2r = make_double4(srec[8 * rows + ln], srec[9 * rows + ln], srec[10 * rows + ln], srec[11 * rows + ln]);
     }
-    const double4 F = face_flux_rec<double, DISS>(glim, c0r, c1r, c2r, n0r, n1r, n2r, fe.nx, fe.ny, fe.dl, fe.dx, fe.dy,
+    Ieee<double> o;
+    const double4 F = face_flux_rec<double, DISS>(o, glim, c0r, c1r, c2r, n0r, n1r, n2r, fe.nx, fe.ny, fe.dl, fe.dx, fe.dy,
                                                     fp.eflin, fp.shock_fix);
     if (so < 4) {
       sF[(so * 4 + 0) * kPatchCells + lo] = F.x;
@@ -2006,7 +2115,8 @@ __global__ void __launch_bounds__(kTileX * kTileY, 2)
     const RecV a = ro[0], b = ro[1], p = rn[0], q = rn[1];
     const double4 c1 = make_double4(a.x, a.y, a.z, a.w), c2 = make_double4(b.x, b.y, b.z, b.w);
     const double4 n1 = make_double4(p.x, p.y, p.z, p.w), n2 = make_double4(q.x, q.y, q.z, q.w);
-    sF[t] = face_flux_rec<T, DISS>(glim, c0, c1, c2, n0, n1, n2, T(gq.x), T(gq.y), T(gq.z), T(gq.w), T(gdy),
+    Ieee<T> o;
+    sF[t] = face_flux_rec<T, DISS>(o, glim, c0, c1, c2, n0, n1, n2, T(gq.x), T(gq.y), T(gq.z), T(gq.w), T(gdy),
                                    T(fp.eflin), T(fp.shock_fix));
   }
   __syncthreads();
@@ -2426,7 +2536,8 @@ __global__ void __launch_bounds__(NTHR, PRE ? 2 : 3)
     const RecV a = ro[0], b = ro[1], p = rn[0], q = rn[1];
     const double4 c1 = make_double4(a.x, a.y, a.z, a.w), c2 = make_double4(b.x, b.y, b.z, b.w);
     const double4 n1 = make_double4(p.x, p.y, p.z, p.w), n2 = make_double4(q.x, q.y, q.z, q.w);
-    const double4 F = face_flux_rec<T, DISS>(glim, c0, c1, c2, n0, n1, n2, T(g01.x), T(g01.y), T(g23.x), T(g23.y),
+    Ieee<T> o;
+    const double4 F = face_flux_rec<T, DISS>(o, glim, c0, c1, c2, n0, n1, n2, T(g01.x), T(g01.y), T(g23.x), T(g23.y),
                                              T(g45.x), T(fp.eflin), T(fp.shock_fix));
     *reinterpret_cast<double2 *>(rec) = make_double2(F.x, F.y);
     *reinterpret_cast<double2 *>(rec + 2) = make_double2(F.z, F.w);
@@ -2530,17 +2641,15 @@ __global__ void k_eval_limiter(int limiter, const double *a, const double *b, in
 // for n conserved left/right states [n][4], outward normals [n][2] and lengths [n]; T is the
 // arithmetic precision (the states are rounded to T first, as in the FP32-flux form).  Primitive
 // variables for Roe and HLLC come from the reference EOS (eos_prim).
-template <typename T>
-__global__ void k_eval_face_flux(int scheme, const double *UL, const double *UR, const double *nrm, const double *len,
-                                 int n, double *F) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n) return;
+template <typename T, typename O>
+__device__ __forceinline__ void eval_face(O &o, int scheme, const double *UL, const double *UR, const double *nrm,
+                                          const double *len, int i, double *F) {
   const T nx = T(nrm[2 * i]), ny = T(nrm[2 * i + 1]), dl = T(len[i]);
   T A[4], D[4] = {T(0.0), T(0.0), T(0.0), T(0.0)};
   const T uL[4] = {T(UL[4 * i]), T(UL[4 * i + 1]), T(UL[4 * i + 2]), T(UL[4 * i + 3])};
   const T uR[4] = {T(UR[4 * i]), T(UR[4 * i + 1]), T(UR[4 * i + 2]), T(UR[4 * i + 3])};
   if (scheme == 6) {
-    ausm_face<T>(uL, uR, nx, ny, dl, A);
+    ausm_face<T>(o, uL, uR, nx, ny, dl, A);
   } else if (scheme == 8) {
     ausm_gpu_face<T>(uL, uR, nx, ny, dl, A);
   } else {
@@ -2550,14 +2659,27 @@ __global__ void k_eval_face_flux(int scheme, const double *UL, const double *UR,
     const T qL[5] = {T(pl.rho), T(pl.u), T(pl.v), T(pl.p), T(pl.a)};
     const T qR[5] = {T(pr.rho), T(pr.u), T(pr.v), T(pr.p), T(pr.a)};
     if (scheme == 7) {
-      hllc_face<T>(qL, uL, qR, uR, nx, ny, dl, A);
+      hllc_face<T>(o, qL, uL, qR, uR, nx, ny, dl, A);
     } else {
       average_flux<T>(qL[0], qL[1], qL[2], qL[3], qR[0], qR[1], qR[2], qR[3], nx, ny, dl, A);
-      roe_1o<T>(qL[0], qL[1], qL[2], qL[3], qL[4], qR[0], qR[1], qR[2], qR[3], qR[4], nx, ny, dl, false, D);
+      roe_1o<T>(o, qL[0], qL[1], qL[2], qL[3], qL[4], qR[0], qR[1], qR[2], qR[3], qR[4], nx, ny, dl, false, D);
     }
   }
 #pragma unroll
   for (int k = 0; k < 4; k++) F[4 * i + k] = double(A[k] - D[k]);
+}
+
+template <typename T>
+__global__ void k_eval_face_flux(int scheme, const double *UL, const double *UR, const double *nrm, const double *len,
+                                 int n, double *F) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= n) return;
+  FaceOps<T> o;
+  eval_face<T>(o, scheme, UL, UR, nrm, len, i, F);
+  if (o.bad()) {
+    Ieee<T> again;
+    eval_face<T>(again, scheme, UL, UR, nrm, len, i, F);
+  }
 }
 
 // ---- AMR tagging (TagRefinableCells, src/Grid_Refine_Functions.cpp:33-63) on the device ----

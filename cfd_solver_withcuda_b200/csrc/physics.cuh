@@ -21,6 +21,122 @@ struct Prim {  // the five primitive slots the fluxes read: Primitive_Cells[c][0
   double rho, u, v, p, a;
 };
 
+// Division and square root of the flux functions, as a policy O.
+//
+// Ieee<T>: the operators themselves.  CUDA's double division and square root test for special
+// operands in a branch each, so a flux with 15 - 25 of them is that many short serial pieces the
+// compiler cannot interleave: the flux kernels were bound by that latency (FP64 pipe 32 - 51 % active).
+// With Fast64 the ROE_2O flux of 524,288 cells takes 117 us instead of 158, the Van Leer + Roe faces
+// 43.7 instead of 52.8, the HLLC faces of 1,038,240 mixed cells 62.9 instead of 73.3 (B200).
+//
+// Fast64: the same values without branches (every result is the correctly rounded one).
+//   Reciprocal: y0 = rcp.approx.ftz.f64(b) (PTX; relative error e about 2^-20), one third-order step
+//   y = y0 (1 + e + e^2).  Its error before rounding is e^3, so y = RN(1/b) unless 1/b lies next to a
+//   rounding boundary; of those b only 2^k (2 - 2^-52) matters for the quotients, and there RN(1/b),
+//   whose last mantissa bit is 1, is put in directly.
+//   Quotient: q = a y, then twice q + (a - b q) y.  The first pass leaves q within one unit in the last
+//   place, so the second residual is exact and its correction rounds correctly (P. Markstein,
+//   Computation of elementary functions on the IBM RISC System/6000, IBM J. Res. Dev. 34, 1990).
+//   Quotients by one denominator share its reciprocal.
+//   Square root: y0 = rsqrt.approx.ftz.f64(a); g = a y0 and h = y0 / 2 take the third-order step
+//   (1 + r + 3/2 r^2), r = 1/2 - g h; then g + (a - g^2) h.  sqrt(a) is nearer than that result's
+//   error to a rounding boundary only just below it (a = 1 - 2^-53, say), so the one correction left
+//   is to the next smaller number p, when a <= p g (B. Tuckerman's test).
+//
+// The steps hold for operands well inside the exponent range: numerators 0 or 2^-500 .. 2^500,
+// denominators 2^-400 .. 2^400, radicands 2^-500 .. 2^500 (positive).  Every operand's high word goes
+// into a running minimum and maximum; bad() tells that some operand was outside (infinities, NaN,
+// zero denominators, negative radicands among them), and the caller then evaluates the same item
+// again with Ieee.  Zero numerators keep their sign for positive denominators (div_signed flags them
+// for the others).
+template <typename T>
+struct Ieee {
+  static constexpr bool fast = false;
+  struct Rcp {
+    T b;
+  };
+  __device__ __forceinline__ T div(T a, T b) { return a / b; }
+  __device__ __forceinline__ T div_signed(T a, T b) { return a / b; }
+  __device__ __forceinline__ T div_gm1(T a) { return a / T(kGM1); }
+  __device__ __forceinline__ T inv(T b) { return T(1.0) / b; }
+  __device__ __forceinline__ Rcp rcp(T b) { return Rcp{b}; }
+  __device__ __forceinline__ T div(T a, const Rcp &r) { return a / r.b; }
+  __device__ __forceinline__ T root(T a) { return sqrt(a); }
+  __device__ __forceinline__ void flag() {}
+  __device__ __forceinline__ bool bad() const { return false; }
+};
+
+struct Fast64 {
+  static constexpr bool fast = true;
+  struct Rcp {
+    double b, y;
+  };
+  // High words (sign off) of 2^-500, 2^500, 2^-400, 2^400.
+  static constexpr unsigned kNumLo = (1023u - 500u) << 20, kNumHi = (1023u + 500u) << 20;
+  static constexpr unsigned kDenLo = (1023u - 400u) << 20, kDenHi = (1023u + 400u) << 20;
+  unsigned nlo = ~0u, nhi = 0u, dlo = ~0u, dhi = 0u;
+  __device__ __forceinline__ void num(double a) {
+    const unsigned h = static_cast<unsigned>(__double2hiint(a)) & 0x7fffffffu;
+    nlo = min(nlo, h - 1u);  // zero wraps to the largest value: allowed
+    nhi = max(nhi, h);
+  }
+  __device__ __forceinline__ void den(double b) {
+    const unsigned h = static_cast<unsigned>(__double2hiint(b)) & 0x7fffffffu;
+    dlo = min(dlo, h);
+    dhi = max(dhi, h);
+  }
+  __device__ __forceinline__ void flag() { dlo = 0u; }
+  __device__ __forceinline__ bool bad() const {
+    return nlo < kNumLo || nhi > kNumHi || dlo < kDenLo || dhi > kDenHi;
+  }
+  __device__ __forceinline__ Rcp rcp(double b) {
+    den(b);
+    double y;
+    asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(b));
+    const double e = fma(-b, y, 1.0);
+    y = fma(fma(e, e, e), y, y);
+    const bool ones = ((static_cast<unsigned>(__double2hiint(b)) | 0xfff00000u) &
+                       static_cast<unsigned>(__double2loint(b))) == 0xffffffffu;
+    return Rcp{b, __hiloint2double(__double2hiint(y), ones ? 1 : __double2loint(y))};
+  }
+  __device__ __forceinline__ double div(double a, const Rcp &r) {
+    num(a);
+    double q = a * r.y;
+    q = fma(-fma(r.b, q, -a), r.y, q);
+    return fma(-fma(r.b, q, -a), r.y, q);
+  }
+  __device__ __forceinline__ double div(double a, double b) { return div(a, rcp(b)); }
+  __device__ __forceinline__ double div_signed(double a, double b) {
+    if (a == 0.0) flag();
+    return div(a, b);
+  }
+  // a / (1.4 - 1.0): 1 / (1.4 - 1.0) as a sum of two doubles brings q within one unit at once.
+  __device__ __forceinline__ double div_gm1(double a) {
+    constexpr double yh = 1.0 / kGM1, yl = 0x1.0000000000005p-53;
+    num(a);
+    const double q = fma(a, yh, a * yl);
+    return fma(-fma(kGM1, q, -a), yh, q);
+  }
+  __device__ __forceinline__ double inv(double b) {
+    const Rcp r = rcp(b);
+    return fma(-fma(b, r.y, -1.0), r.y, r.y);
+  }
+  __device__ __forceinline__ double root(double a) {
+    const unsigned h = static_cast<unsigned>(__double2hiint(a));  // a set sign bit is above every bound
+    nlo = min(nlo, h);
+    nhi = max(nhi, h);
+    double y;
+    asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(a));
+    const double g0 = a * y, h0 = 0.5 * y;
+    const double r = fma(-g0, h0, 0.5);
+    const double t = fma(1.5 * r, r, r);
+    const double g1 = fma(g0, t, g0), hh = fma(h0, t, h0);
+    const double g = fma(fma(-g1, g1, a), hh, g1);
+    const double p = __longlong_as_double(__double_as_longlong(g) - 1);
+    return fma(-p, g, a) <= 0.0 ? p : g;
+  }
+};
+
 // Calculate_Primitive_Variables, src/Basic_Functions.cpp:100-156 (slots 0,1,2,4,5).
 // Returns false when the sound speed is NaN (the reference exits there, :151-155).
 __host__ __device__ inline bool eos_prim(double U0, double U1, double U2, double U3, Prim &q) {
@@ -67,27 +183,31 @@ __device__ __forceinline__ void average_flux(const T rL, const T uL, const T vL,
 // eigenvalues with Harten's fix delta = 0.1*a_Roe on the acoustic waves, right eigenvectors,
 // D = 0.5*sum|l|a r*dl.  eflin > 0 (no reference counterpart; the gradient-MUSCL form's option
 // against the carbuncle) also fixes the two linear waves, |Un| below eflin*a_Roe.
-template <typename T>
-__device__ __forceinline__ void roe_tail(const T Ru, const T Rv, const T RH, const T RVm, const T Ra, const T RoeRho,
-                                         const T Un, const T Ut, const T dP, const T dRho, const T dUn, const T dUt,
-                                         const T nx, const T ny, const T dl, T D[4], const T eflin = T(0.0)) {
+template <typename T, typename O>
+__device__ __forceinline__ void roe_tail(O &o, const T Ru, const T Rv, const T RH, const T RVm, const T Ra,
+                                         const T RoeRho, const T Un, const T Ut, const T dP, const T dRho, const T dUn,
+                                         const T dUt, const T nx, const T ny, const T dl, T D[4],
+                                         const T eflin = T(0.0)) {
   T R11 = T(1.0), R12 = Ru - nx * Ra, R13 = Rv - ny * Ra, R14 = RH - Ra * Un;
   T R21 = T(1.0), R22 = Ru, R23 = Rv, R24 = RVm;
   T R31 = T(0.0), R32 = -ny, R33 = nx, R34 = Ut;
   T R41 = T(1.0), R42 = Ru + nx * Ra, R43 = Rv + ny * Ra, R44 = RH + Ra * Un;
-  T Term2 = T(1.0) / (Ra * Ra);
+  T Term2 = o.inv(Ra * Ra);
   T a1 = T(0.5) * Term2 * (dP - RoeRho * Ra * dUn);
   T a2 = dRho - Term2 * dP;
   T a3 = RoeRho * dUt;
   T a4 = T(0.5) * Term2 * (dP + RoeRho * Ra * dUn);
   T L1 = fabs(Un - Ra), L2 = fabs(Un), L3 = fabs(Un), L4 = fabs(Un + Ra);
   T ef = T(0.1) * Ra;
-  if (L1 < ef) L1 = T(0.5) * (L1 * L1 / ef + ef);
-  if (L4 < ef) L4 = T(0.5) * (L4 * L4 / ef + ef);
+  if (L1 < ef || L4 < ef) {
+    const typename O::Rcp rf = o.rcp(ef);
+    if (L1 < ef) L1 = T(0.5) * (o.div(L1 * L1, rf) + ef);
+    if (L4 < ef) L4 = T(0.5) * (o.div(L4 * L4, rf) + ef);
+  }
   if (eflin > T(0.0)) {
     const T el = eflin * Ra;
     if (L2 < el) {
-      L2 = T(0.5) * (L2 * L2 / el + el);
+      L2 = T(0.5) * (o.div(L2 * L2, el) + el);
       L3 = L2;
     }
   }
@@ -99,27 +219,34 @@ __device__ __forceinline__ void roe_tail(const T Ru, const T Rv, const T RH, con
 
 // ROE, src/Roe_Scheme.cpp:6-256.  `degenerate` is the precomputed |n| < 1e-12 test (:71-76);
 // a ghost neighbour has already been replaced by the cell itself (:79-84) by the caller.
-template <typename T>
-__device__ __forceinline__ void roe_1o(const T rL, const T uL, const T vL, const T pL, const T cL, const T rR,
+template <typename T, typename O>
+__device__ __forceinline__ void roe_1o(O &o, const T rL, const T uL, const T vL, const T pL, const T cL, const T rR,
                                        const T uR, const T vR, const T pR, const T cR, const T nx, const T ny,
                                        const T dl, bool degenerate, T D[4], const T eflin = T(0.0)) {
   D[0] = D[1] = D[2] = D[3] = T(0.0);
-  if (degenerate) return;
-  if (rL <= T(0.0) || pL <= T(0.0) || cL <= T(0.0)) return;
+  if (O::fast) {  // the special cases are left to the caller's second evaluation
+    if (degenerate || rL <= T(0.0) || pL <= T(0.0) || cL <= T(0.0) || rR <= T(0.0) || pR <= T(0.0) || cR <= T(0.0))
+      o.flag();
+  } else {
+    if (degenerate) return;
+    if (rL <= T(0.0) || pL <= T(0.0) || cL <= T(0.0)) return;
+    if (rR <= T(0.0) || pR <= T(0.0) || cR <= T(0.0)) return;
+  }
   T VmL = T(0.5) * (uL * uL + vL * vL);
-  T HL = ((cL * cL) / T(kGM1)) + VmL;
-  if (rR <= T(0.0) || pR <= T(0.0) || cR <= T(0.0)) return;
+  T HL = o.div_gm1(cL * cL) + VmL;
   T VmR = T(0.5) * (uR * uR + vR * vR);
-  T HR = ((cR * cR) / T(kGM1)) + VmR;
-  T sL = sqrt(rL), sR = sqrt(rR);
-  T Term1 = T(1.0) / (sL + sR);
-  T RoeRho = sqrt(rL * rR);
+  T HR = o.div_gm1(cR * cR) + VmR;
+  T sL = o.root(rL), sR = o.root(rR);
+  T Term1 = o.inv(sL + sR);
+  T RoeRho = o.root(rL * rR);
   T Ru = Term1 * (uR * sR + uL * sL);
   T Rv = Term1 * (vR * sR + vL * sL);
   T RH = Term1 * (HR * sR + HL * sL);
   T RVm = T(0.5) * (Ru * Ru + Rv * Rv);
-  T Ra = sqrt(T(kGM1) * (RH - RVm));
-  if (Ra <= T(0.0)) {
+  T Ra = o.root(T(kGM1) * (RH - RVm));
+  if (O::fast) {
+    if (Ra <= T(0.0)) o.flag();
+  } else if (Ra <= T(0.0)) {
     Ra = T(0.5) * (cL + cR);
     if (Ra <= T(0.0)) return;
   }
@@ -128,37 +255,38 @@ __device__ __forceinline__ void roe_1o(const T rL, const T uL, const T vL, const
   T du = (uR - uL), dv = (vR - vL), dP = (pR - pL), dRho = (rR - rL);
   T dUn = nx * du + ny * dv;
   T dUt = -ny * du + nx * dv;
-  roe_tail<T>(Ru, Rv, RH, RVm, Ra, RoeRho, Un, Ut, dP, dRho, dUn, dUt, nx, ny, dl, D, eflin);
+  roe_tail<T>(o, Ru, Rv, RH, RVm, Ra, RoeRho, Un, Ut, dP, dRho, dUn, dUt, nx, ny, dl, D, eflin);
 }
 
 // ROE_2O, src/Roe_Scheme.cpp:257-447: Roe averages of the unreconstructed cell states, wave
 // strengths from the limited conserved jump dU (Second_Order_Limiter).
-template <typename T>
-__device__ __forceinline__ void roe_2o(const T rL, const T uL, const T vL, const T pL, const T cL, const T rR,
+template <typename T, typename O>
+__device__ __forceinline__ void roe_2o(O &o, const T rL, const T uL, const T vL, const T pL, const T cL, const T rR,
                                        const T uR, const T vR, const T pR, const T cR, const T nx, const T ny,
                                        const T dl, const T dU[4], T D[4]) {
   T VmL = T(0.5) * (uL * uL + vL * vL);
-  T HL = ((cL * cL) / T(kGM1)) + VmL;
+  T HL = o.div_gm1(cL * cL) + VmL;
   T VmR = T(0.5) * (uR * uR + vR * vR);
-  T HR = ((cR * cR) / T(kGM1)) + VmR;
-  T sR = sqrt(rR), sL = sqrt(rL);
-  T Term1 = T(1.0) / (sL + sR);
-  T RoeRho = sqrt(rL * rR);
+  T HR = o.div_gm1(cR * cR) + VmR;
+  T sR = o.root(rR), sL = o.root(rL);
+  T Term1 = o.inv(sL + sR);
+  T RoeRho = o.root(rL * rR);
   T Ru = Term1 * (uR * sR + uL * sL);
   T Rv = Term1 * (vR * sR + vL * sL);
   T RH = Term1 * (HR * sR + HL * sL);
   T RVm = T(0.5) * (Ru * Ru + Rv * Rv);
   T Un = nx * Ru + ny * Rv;
   T Ut = -ny * Ru + nx * Rv;
-  T Ra = sqrt(T(kGM1) * (RH - RVm));
-  T du = dU[1] / RoeRho - dU[0] * Ru / (RoeRho * RoeRho);
-  T dv = dU[2] / RoeRho - dU[0] * Rv / (RoeRho * RoeRho);
+  T Ra = o.root(T(kGM1) * (RH - RVm));
+  const typename O::Rcp r1 = o.rcp(RoeRho), r2 = o.rcp(RoeRho * RoeRho);
+  T du = o.div(dU[1], r1) - o.div(dU[0] * Ru, r2);
+  T dv = o.div(dU[2], r1) - o.div(dU[0] * Rv, r2);
   T dE = dU[3] - T(0.5) * RoeRho * (T(2.0) * (Ru * du + Rv * dv) + du * du + dv * dv) - T(0.5) * dU[0] * RVm;
   T dP = T(kGM1) * dE;
   T dRho = dU[0];
   T dUn = nx * du + ny * dv;
   T dUt = -ny * du + nx * dv;
-  roe_tail<T>(Ru, Rv, RH, RVm, Ra, RoeRho, Un, Ut, dP, dRho, dUn, dUt, nx, ny, dl, D);
+  roe_tail<T>(o, Ru, Rv, RH, RVm, Ra, RoeRho, Un, Ut, dP, dRho, dUn, dUt, nx, ny, dl, D);
 }
 
 // Maximum(a,b,c) / Maximum(a,b), src/Utility_Files.cpp:5-31.
@@ -206,8 +334,8 @@ __device__ __forceinline__ T min3_ref(T a, T b, T c) {
 // association order.  `plus_pl` is the sign the reference gives the left pressure term of the two
 // momentum components: + in MOVERS, MOVERS_2O, RICCA, RICCA_2O and MOVERS_NWSC, - in
 // MOVERS_NWSC_2O (src/MOVERS_NWSC.cpp:183-184).
-template <typename T>
-__device__ __forceinline__ void movers_flux_jump(const T rL, const T uL, const T vL, const T pL, const T rR,
+template <typename T, typename O>
+__device__ __forceinline__ void movers_flux_jump(O &o, const T rL, const T uL, const T vL, const T pL, const T rR,
                                                  const T uR, const T vR, const T pR, const T nx, const T ny,
                                                  const T dl, const T VnL, const T VnR, bool plus_pl, T dF[4]) {
   const T VmL = T(0.5) * (uL * uL + vL * vL);
@@ -220,23 +348,31 @@ __device__ __forceinline__ void movers_flux_jump(const T rL, const T uL, const T
     dF[1] = (rR * uR * VnR + pR * nx - rL * uL * VnL - pL * nx) * dl;
     dF[2] = (rR * vR * VnR + pR * ny - rL * vL * VnL - pL * ny) * dl;
   }
-  dF[3] = ((((pR / T(kGM1)) + rR * VmR) + pR) * VnR - (((pL / T(kGM1)) + rL * VmL) + pL) * VnL) * dl;
+  dF[3] = (((o.div_gm1(pR) + rR * VmR) + pR) * VnR - ((o.div_gm1(pL) + rL * VmL) + pL) * VnL) * dl;
 }
 
 // Conserved jump rebuilt from the two cells' primitives (src/MOVERS.cpp:208-211, src/RICCA.cpp:96-100).
-template <typename T>
-__device__ __forceinline__ void prim_jump(const T rL, const T uL, const T vL, const T pL, const T rR, const T uR,
+template <typename T, typename O>
+__device__ __forceinline__ void prim_jump(O &o, const T rL, const T uL, const T vL, const T pL, const T rR, const T uR,
                                           const T vR, const T pR, T dU[4]) {
   dU[0] = rR - rL;
   dU[1] = rR * uR - rL * uL;
   dU[2] = rR * vR - rL * vL;
-  dU[3] = ((pR / T(kGM1)) + T(0.5) * rR * (uR * uR + vR * vR)) - ((pL / T(kGM1)) + T(0.5) * rL * (uL * uL + vL * vL));
+  dU[3] = (o.div_gm1(pR) + T(0.5) * rR * (uR * uR + vR * vR)) - (o.div_gm1(pL) + T(0.5) * rL * (uL * uL + vL * vL));
 }
 
 // Condition_For_MOVERS, src/MOVERS.cpp:19-43 (epsilon 1e-10).
-template <typename T>
-__device__ __forceinline__ T movers_alpha(const T dU, const T dF, const T Lmax, const T Lmin) {
+template <typename T, typename O>
+__device__ __forceinline__ T movers_alpha(O &o, const T dU, const T dF, const T Lmax, const T Lmin) {
   const T eps = T(1e-10);
+  if (O::fast) {  // the same choices without branches
+    const bool both = fabs(dF) > eps && fabs(dU) > eps;
+    const T A = fabs(o.div(both ? dF : T(0.0), both ? fabs(dU) : T(1.0)));
+    T B = A;
+    if (A >= Lmax) B = T(sign_ref<T>(A)) * Lmax;
+    else if (A <= Lmin) B = T(sign_ref<T>(A)) * Lmin;
+    return both ? B : ((fabs(dF) < eps && fabs(dU) > eps) ? T(0.0) : Lmin);
+  }
   if (fabs(dF) < eps && fabs(dU) > eps) return T(0.0);
   if (fabs(dF) < eps && fabs(dU) < eps) return Lmin;
   if (fabs(dF) > eps && fabs(dU) > eps) {
@@ -249,10 +385,10 @@ __device__ __forceinline__ T movers_alpha(const T dU, const T dF, const T Lmax, 
 }
 
 // Entropy_Fix, src/MOVERS.cpp:7-17 (delta = 1.0 * L_Max).
-template <typename T>
-__device__ __forceinline__ T movers_entropy_fix(const T A, const T Lmax) {
+template <typename T, typename O>
+__device__ __forceinline__ T movers_entropy_fix(O &o, const T A, const T Lmax) {
   const T delta = T(1.0) * Lmax;
-  if (fabs(A) < delta) return (A * A + delta * delta) / (T(2.0) * delta);
+  if (fabs(A) < delta) return o.div(A * A + delta * delta, T(2.0) * delta);
   return Lmax;
 }
 
@@ -262,8 +398,8 @@ __device__ __forceinline__ T movers_entropy_fix(const T A, const T Lmax) {
 // (all four components at first order, the energy one at second order).  At second order the
 // reference keeps the unreconstructed primitive jump and zero sound speeds (its MOVERS_2O never
 // sets C_L, C_R).  D = 0.5 alpha dU.
-template <typename T, int ORDER>
-__device__ __forceinline__ void movers_diss(const T rL, const T uL, const T vL, const T pL, const T cL0, const T rR,
+template <typename T, int ORDER, typename O>
+__device__ __forceinline__ void movers_diss(O &o, const T rL, const T uL, const T vL, const T pL, const T cL0, const T rR,
                                             const T uR, const T vR, const T pR, const T cR0, const T UL[4],
                                             const T UR[4], const T nx, const T ny, const T dl, bool single, bool efix,
                                             T D[4]) {
@@ -272,30 +408,30 @@ __device__ __forceinline__ void movers_diss(const T rL, const T uL, const T vL, 
 #pragma unroll
     for (int k = 0; k < 4; k++) dU[k] = UR[k] - UL[k];
   } else {
-    prim_jump<T>(rL, uL, vL, pL, rR, uR, vR, pR, dU);
+    prim_jump<T>(o, rL, uL, vL, pL, rR, uR, vR, pR, dU);
   }
   const T cL = ORDER == 1 ? cL0 : T(0.0), cR = ORDER == 1 ? cR0 : T(0.0);
   const T VnL = (uL * nx + vL * ny);
   const T VnR = (uR * nx + vR * ny);
   T dF[4];
-  movers_flux_jump<T>(rL, uL, vL, pL, rR, uR, vR, pR, nx, ny, dl, VnL, VnR, true, dF);
+  movers_flux_jump<T>(o, rL, uL, vL, pL, rR, uR, vR, pR, nx, ny, dl, VnL, VnR, true, dF);
   const T S0 = fabs(VnL - cL) * dl, S1 = fabs(VnL + cL) * dl, S2 = fabs(VnL) * dl;
   const T S3 = fabs(VnR - cR) * dl, S4 = fabs(VnR + cR) * dl, S5 = fabs(VnR) * dl;
   const T Lmax = max2_ref<T>(max3_ref<T>(S0, S1, S2), max3_ref<T>(S3, S4, S5));
   const T Lmin = max2_ref<T>(min3_ref<T>(S0, S1, S2), min3_ref<T>(S3, S4, S5));
   T A[4];
-  A[3] = movers_alpha<T>(dU[3], dF[3], Lmax, Lmin);
+  A[3] = movers_alpha<T>(o, dU[3], dF[3], Lmax, Lmin);
   A[0] = A[1] = A[2] = A[3];
   if (!single) {
 #pragma unroll
-    for (int k = 0; k < 3; k++) A[k] = movers_alpha<T>(dU[k], dF[k], Lmax, Lmin);
+    for (int k = 0; k < 3; k++) A[k] = movers_alpha<T>(o, dU[k], dF[k], Lmax, Lmin);
   }
   if (efix) {
     if (ORDER == 1) {
 #pragma unroll
-      for (int k = 0; k < 3; k++) A[k] = movers_entropy_fix<T>(A[k], Lmax);
+      for (int k = 0; k < 3; k++) A[k] = movers_entropy_fix<T>(o, A[k], Lmax);
     }
-    A[3] = movers_entropy_fix<T>(A[3], Lmax);
+    A[3] = movers_entropy_fix<T>(o, A[3], Lmax);
   }
 #pragma unroll
   for (int k = 0; k < 4; k++) D[k] = T(0.5) * A[k] * dU[k];
@@ -307,31 +443,32 @@ __device__ __forceinline__ void movers_diss(const T rL, const T uL, const T vL, 
 // place, so it stays zero for the later components).  dU is the primitive-rebuilt jump at first
 // order and the limited conserved jump `dU2` (Second_Order_Limiter) at second order.
 // D = 0.5 alpha dl dU.
-template <typename T, int ORDER>
-__device__ __forceinline__ void ricca_diss(const T rL, const T uL, const T vL, const T pL, const T rR, const T uR,
+template <typename T, int ORDER, typename O>
+__device__ __forceinline__ void ricca_diss(O &o, const T rL, const T uL, const T vL, const T pL, const T rR, const T uR,
                                            const T vR, const T pR, const T nx, const T ny, const T dl, const T dU2[4],
                                            T D[4]) {
   const T VnL = uL * nx + vL * ny;
   const T VnR = uR * nx + vR * ny;
   T dU[4];
-  if (ORDER == 1) prim_jump<T>(rL, uL, vL, pL, rR, uR, vR, pR, dU);
+  if (ORDER == 1) prim_jump<T>(o, rL, uL, vL, pL, rR, uR, vR, pR, dU);
   else {
 #pragma unroll
     for (int k = 0; k < 4; k++) dU[k] = dU2[k];
   }
   T dF[4];
-  movers_flux_jump<T>(rL, uL, vL, pL, rR, uR, vR, pR, nx, ny, dl, VnL, VnR, true, dF);
+  movers_flux_jump<T>(o, rL, uL, vL, pL, rR, uR, vR, pR, nx, ny, dl, VnL, VnR, true, dF);
   T dP = fabs(pL - pR);
   const T PI = T(0.5) * (pL + pR);
   const T RI = T(0.5) * (rL + rR);
   if (dP < T(1e-8)) dP = T(0.0);
   const T aL = fabs(VnL), aR = fabs(VnR);
   const T Mx = (aL < aR) ? aR : aL;
+  const T aI = o.root(o.div(T(kGamma) * PI, RI));
 #pragma unroll
   for (int k = 0; k < 4; k++) {
     T A;
     if (fabs(dF[k]) < T(1e-8) && fabs(dU[k]) < T(1e-8)) A = T(0.5) * (aL + aR);
-    else A = Mx + T(1.0) * T(sign_ref<T>(dP)) * sqrt(T(kGamma) * PI / RI);
+    else A = Mx + T(1.0) * T(sign_ref<T>(dP)) * aI;
     D[k] = T(0.5) * A * dl * dU[k];
   }
 }
@@ -340,8 +477,8 @@ __device__ __forceinline__ void ricca_diss(const T rL, const T uL, const T vL, c
 // Condition_For_MOVERS_NWSC (:6-21): alpha_k = sign(dU_k) |dF_k| (0 across a discontinuity),
 // pressure sensor 0.21 |dp / (2 p_I)|, D = 0.5 (sensor alpha + 0.5(|V_R.n dl| + |V_L.n dl|) dU).
 // dU: conserved jump U_R - U_L at first order, the limited jump `dU2` at second order.
-template <typename T, int ORDER>
-__device__ __forceinline__ void nwsc_diss(const T rL, const T uL, const T vL, const T pL, const T rR, const T uR,
+template <typename T, int ORDER, typename O>
+__device__ __forceinline__ void nwsc_diss(O &o, const T rL, const T uL, const T vL, const T pL, const T rR, const T uR,
                                           const T vR, const T pR, const T UL[4], const T UR[4], const T nx, const T ny,
                                           const T dl, const T dU2[4], T D[4]) {
   const T VnL = (uL * nx + vL * ny);
@@ -350,7 +487,7 @@ __device__ __forceinline__ void nwsc_diss(const T rL, const T uL, const T vL, co
 #pragma unroll
   for (int k = 0; k < 4; k++) dU[k] = ORDER == 1 ? UR[k] - UL[k] : dU2[k];
   T dF[4];
-  movers_flux_jump<T>(rL, uL, vL, pL, rR, uR, vR, pR, nx, ny, dl, VnL, VnR, ORDER == 1, dF);
+  movers_flux_jump<T>(o, rL, uL, vL, pL, rR, uR, vR, pR, nx, ny, dl, VnL, VnR, ORDER == 1, dF);
   T A[4];
 #pragma unroll
   for (int k = 0; k < 4; k++) {
@@ -360,7 +497,7 @@ __device__ __forceinline__ void nwsc_diss(const T rL, const T uL, const T vL, co
   const T dP = pR - pL;
   const T PI = T(0.5) * (pR + pL);
   const T AP = T(0.5) * (fabs(VnR * dl) + fabs(VnL * dl));
-  const T Sensor = T(0.21) * fabs(dP / (T(2.0) * PI));
+  const T Sensor = T(0.21) * fabs(o.div(dP, T(2.0) * PI));
 #pragma unroll
   for (int k = 0; k < 4; k++) D[k] = T(0.5) * (Sensor * A[k] + AP * dU[k]);
 }
@@ -414,20 +551,43 @@ __device__ __forceinline__ T muscl_slope(int kind, T a, T b) {
   }
 }
 
-// Limited slope of one variable on the reference's directional stencil (src/Limiters.cpp:109-134):
+// muscl_slope of a Fast64 evaluation: the Van Leer and van Albada quotients without branches (where the
+// slope is zero the quotient is 0 / 1), the others as they are.
+template <int KIND>
+__device__ __forceinline__ double muscl_slope_fast(Fast64 &o, double a, double b) {
+  const double ab = a * b;
+  const bool on = !(fabs(b) < 1e-12) && !(ab <= 0.0);
+  if (KIND == LIM_VANLEER) return o.div(on ? 2.0 * ab : 0.0, on ? a + b : 1.0);
+  const double a2 = a * a;
+  return o.div(on ? b * (a2 + ab) : 0.0, on ? a2 + b * b : 1.0);
+}
+
+// Limited slopes of the four conserved or primitive variables on the reference's directional stencil
+// (src/Limiters.cpp:109-134):
 //   S1 = zeta*(q_c - q_N1)/d1 (across the face), S2 = zeta1*(q_N1 - q_N2)/d2 (beyond N1)
 // Reference minmod (src/Limiters.cpp:58-63): 0.5*(sgn S1 + sgn S2)*min(|S1|,|S2|).
 // phi forms: phi(S2, S1) * S1.
-template <typename T>
-__device__ __forceinline__ T limited_slope(int kind, T qc, T q1, T q2, T d1, T d2, T zeta, T zeta1) {
-  T S1 = zeta * (qc - q1) / d1;
-  T S2 = zeta1 * (q1 - q2) / d2;
-  if (kind == LIM_REF_MINMOD) {
-    T a1 = fabs(S1), b1 = fabs(S2);
-    T m = (b1 < a1) ? b1 : a1;
-    return T(0.5) * T(sign_ref<T>(S1) + sign_ref<T>(S2)) * m;
+template <typename T, typename O>
+__device__ __forceinline__ void limited_slopes(O &o, int kind, const T qc[4], const T q1[4], const T q2[4], T d1, T d2,
+                                               T zeta, T zeta1, T phi[4]) {
+  const typename O::Rcp r1 = o.rcp(d1), r2 = o.rcp(d2);
+  T S1[4], S2[4];
+#pragma unroll
+  for (int k = 0; k < 4; k++) {
+    S1[k] = o.div(zeta * (qc[k] - q1[k]), r1);
+    S2[k] = o.div(zeta1 * (q1[k] - q2[k]), r2);
   }
-  return phi_ab<T>(kind, S2, S1) * S1;
+  if (kind == LIM_REF_MINMOD) {
+#pragma unroll
+    for (int k = 0; k < 4; k++) {
+      const T a1 = fabs(S1[k]), b1 = fabs(S2[k]);
+      const T m = (b1 < a1) ? b1 : a1;
+      phi[k] = T(0.5) * T(sign_ref<T>(S1[k]) + sign_ref<T>(S2[k])) * m;
+    }
+  } else {
+#pragma unroll
+    for (int k = 0; k < 4; k++) phi[k] = phi_ab<T>(kind, S2[k], S1[k]) * S1[k];
+  }
 }
 
 }  // namespace cfdb
@@ -437,24 +597,28 @@ namespace cfdb {
 // AUSM face flux of Ausm_Flux (src/Ausm_Flux.cpp:36-160) from the two conserved states:
 // velocities and pressure from U, Roe-averaged interface sound speed, M+/- and P+/- splittings,
 // upwinded mass flux; F already multiplied by the face length.
-template <typename T>
-__device__ __forceinline__ void ausm_face(const T UL[4], const T UR[4], const T nx, const T ny, const T area, T F[4]) {
+template <typename T, typename O>
+__device__ __forceinline__ void ausm_face(O &o, const T UL[4], const T UR[4], const T nx, const T ny, const T area,
+                                          T F[4]) {
   const T rho_L = UL[0], rhou_L = UL[1], rhov_L = UL[2], rhoE_L = UL[3];
-  const T u_L = rhou_L / rho_L, v_L = rhov_L / rho_L;
+  const typename O::Rcp rL = o.rcp(rho_L);
+  const T u_L = o.div(rhou_L, rL), v_L = o.div(rhov_L, rL);
   const T p_L = T(kGM1) * (rhoE_L - T(0.5) * rho_L * (u_L * u_L + v_L * v_L));
-  const T H_L = (rhoE_L + p_L) / rho_L;
+  const T H_L = o.div(rhoE_L + p_L, rL);
   const T rho_R = UR[0], rhou_R = UR[1], rhov_R = UR[2], rhoE_R = UR[3];
-  const T u_R = rhou_R / rho_R, v_R = rhov_R / rho_R;
+  const typename O::Rcp rR = o.rcp(rho_R);
+  const T u_R = o.div(rhou_R, rR), v_R = o.div(rhov_R, rR);
   const T p_R = T(kGM1) * (rhoE_R - T(0.5) * rho_R * (u_R * u_R + v_R * v_R));
-  const T H_R = (rhoE_R + p_R) / rho_R;
+  const T H_R = o.div(rhoE_R + p_R, rR);
   const T Vn_L = u_L * nx + v_L * ny, Vn_R = u_R * nx + v_R * ny;
-  const T sqrt_rho_L = sqrt(rho_L), sqrt_rho_R = sqrt(rho_R);
-  const T inv_sqrt_sum = T(1.0) / (sqrt_rho_L + sqrt_rho_R);
+  const T sqrt_rho_L = o.root(rho_L), sqrt_rho_R = o.root(rho_R);
+  const T inv_sqrt_sum = o.inv(sqrt_rho_L + sqrt_rho_R);
   const T u_roe = (sqrt_rho_L * u_L + sqrt_rho_R * u_R) * inv_sqrt_sum;
   const T v_roe = (sqrt_rho_L * v_L + sqrt_rho_R * v_R) * inv_sqrt_sum;
   const T H_roe = (sqrt_rho_L * H_L + sqrt_rho_R * H_R) * inv_sqrt_sum;
-  const T a_roe = sqrt(T(kGM1) * (H_roe - T(0.5) * (u_roe * u_roe + v_roe * v_roe)));
-  const T M_L = Vn_L / a_roe, M_R = Vn_R / a_roe;
+  const T a_roe = o.root(T(kGM1) * (H_roe - T(0.5) * (u_roe * u_roe + v_roe * v_roe)));
+  const typename O::Rcp ra = o.rcp(a_roe);
+  const T M_L = o.div(Vn_L, ra), M_R = o.div(Vn_R, ra);
   T M_plus, M_minus, P_plus, P_minus;
   if (fabs(M_L) >= T(1.0)) M_plus = (M_L > T(0.0)) ? M_L : T(0.0);
   else M_plus = T(0.25) * (M_L + T(1.0)) * (M_L + T(1.0));
@@ -485,30 +649,38 @@ __device__ __forceinline__ void ausm_face(const T UL[4], const T UR[4], const T 
 // normal renormalised, Davis/Roe wave-speed bounds, contact speed S*, star states; zero flux for
 // a degenerate normal or a non-physical state; F multiplied by the face length.  q = (rho, u, v,
 // p, a) with the conserved U of the same cell.
-template <typename T>
-__device__ __forceinline__ void hllc_face(const T qL[5], const T UL[4], const T qR[5], const T UR[4], T nx, T ny,
+template <typename T, typename O>
+__device__ __forceinline__ void hllc_face(O &o, const T qL[5], const T UL[4], const T qR[5], const T UR[4], T nx, T ny,
                                           const T area, T F[4]) {
   F[0] = F[1] = F[2] = F[3] = T(0.0);
-  const T normal_mag = sqrt(nx * nx + ny * ny);
-  if (normal_mag < T(1e-14)) return;
-  nx /= normal_mag;
-  ny /= normal_mag;
+  const T normal_mag = o.root(nx * nx + ny * ny);
+  if (O::fast) {  // the special cases are left to the caller's second evaluation
+    if (normal_mag < T(1e-14) || qL[0] <= T(0.0) || qL[3] <= T(0.0) || qL[4] <= T(0.0) || qR[0] <= T(0.0) ||
+        qR[3] <= T(0.0) || qR[4] <= T(0.0))
+      o.flag();
+  } else {
+    if (normal_mag < T(1e-14)) return;
+    if (qL[0] <= T(0.0) || qL[3] <= T(0.0) || qL[4] <= T(0.0)) return;
+    if (qR[0] <= T(0.0) || qR[3] <= T(0.0) || qR[4] <= T(0.0)) return;
+  }
+  const typename O::Rcp rm = o.rcp(normal_mag);
+  nx = o.div(nx, rm);
+  ny = o.div(ny, rm);
   const T rho_L = qL[0], u_L = qL[1], v_L = qL[2], P_L = qL[3], a_L = qL[4];
-  if (rho_L <= T(0.0) || P_L <= T(0.0) || a_L <= T(0.0)) return;
   const T rho_R = qR[0], u_R = qR[1], v_R = qR[2], P_R = qR[3], a_R = qR[4];
-  if (rho_R <= T(0.0) || P_R <= T(0.0) || a_R <= T(0.0)) return;
   const T un_L = nx * u_L + ny * v_L, un_R = nx * u_R + ny * v_R;
-  const T sqrt_rho_L = sqrt(rho_L), sqrt_rho_R = sqrt(rho_R);
-  const T a_roe = (a_L * sqrt_rho_L + a_R * sqrt_rho_R) / (sqrt_rho_L + sqrt_rho_R);
-  const T u_roe = (u_L * sqrt_rho_L + u_R * sqrt_rho_R) / (sqrt_rho_L + sqrt_rho_R);
-  const T v_roe = (v_L * sqrt_rho_L + v_R * sqrt_rho_R) / (sqrt_rho_L + sqrt_rho_R);
+  const T sqrt_rho_L = o.root(rho_L), sqrt_rho_R = o.root(rho_R);
+  const typename O::Rcp rs = o.rcp(sqrt_rho_L + sqrt_rho_R);
+  const T a_roe = o.div(a_L * sqrt_rho_L + a_R * sqrt_rho_R, rs);
+  const T u_roe = o.div(u_L * sqrt_rho_L + u_R * sqrt_rho_R, rs);
+  const T v_roe = o.div(v_L * sqrt_rho_L + v_R * sqrt_rho_R, rs);
   const T un_roe = nx * u_roe + ny * v_roe;
   const T S_L = fmin(un_L - a_L, un_roe - a_roe);
   const T S_R = fmax(un_R + a_R, un_roe + a_roe);
   const T numer = P_R - P_L + rho_L * un_L * (S_L - un_L) - rho_R * un_R * (S_R - un_R);
   const T denom = rho_L * (S_L - un_L) - rho_R * (S_R - un_R);
   T S_star;
-  if (fabs(denom) > T(1e-14)) S_star = numer / denom;
+  if (fabs(denom) > T(1e-14)) S_star = o.div_signed(numer, denom);
   else S_star = T(0.5) * (un_L + un_R);
   T flux[4];
   if (S_L >= T(0.0)) {
@@ -528,9 +700,9 @@ __device__ __forceinline__ void hllc_face(const T qL[5], const T UL[4], const T 
     const T S_K = left ? S_L : S_R;
     const T un = nx * u + ny * v;
     const T FK[4] = {rho * un, rho * u * un + P * nx, rho * v * un + P * ny, (U[3] + P) * un};
-    const T factor = rho * (S_K - un) / (S_K - S_star);
+    const T factor = o.div_signed(rho * (S_K - un), S_K - S_star);
     const T Us[4] = {factor, factor * (u + (S_star - un) * nx), factor * (v + (S_star - un) * ny),
-                     factor * (U[3] / rho + (S_star - un) * (S_star + P / (rho * (S_K - un))))};
+                     factor * (o.div(U[3], rho) + (S_star - un) * (S_star + o.div_signed(P, rho * (S_K - un))))};
 #pragma unroll
     for (int i = 0; i < 4; i++) flux[i] = FK[i] + S_K * (Us[i] - U[i]);
   }
