@@ -397,6 +397,16 @@ struct cfd_ctx {
     cudaEvent_t a, b;
   };
   std::vector<Timed> timed;
+  // Whole pseudo-steps in one launch (launch_steps): the shape and block shares of a single solve, decided
+  // at the first multi-step call, or of a batch's active instances.
+  bool steps_known = false;
+  int steps_off = 0;      // option "one_launch_steps" 0
+  StepsShape steps{};
+  std::vector<int> bptr;  // host copy of the cells' boundary-entry offsets
+  bool t_end_set = false;
+  StepsBlock *d_steps = nullptr;         // [SMs] block shares
+  unsigned int *d_arrivals = nullptr;    // [SMs * kStepsBarrierStride] barrier counts, then the give-up flag
+  int steps_sms = 0;
   double kind_ms[9] = {0, 0, 0, 0, 0, 0, 0, 0, 0};
   long long kind_n[9] = {0, 0, 0, 0, 0, 0, 0, 0, 0};
   double *d_stage = nullptr;  // [NT*4] reference-order AoS staging rows
@@ -1151,6 +1161,7 @@ cfd_status cfd_create(const cfd_mesh_desc *d, const cfd_config *cfg, cfd_ctx **o
     for (int e = 0; e < NB; e++) bidx[fill[bnd[e].y]++] = e;
   }
 
+  ctx->bptr = bptr;
   DevMesh &m = ctx->dm;
   m.NP = NP;
   m.NT = NT;
@@ -1252,7 +1263,9 @@ cfd_status cfd_create(const cfd_mesh_desc *d, const cfd_config *cfg, cfd_ctx **o
 
   DevState &st = ctx->ds;
   const size_t dsz = sizeof(double);
-  const int nblk = std::max(std::max(flux_block_count(NP), m.npatch), ctx->tile_ok ? ctx->tm.tiles_i * ctx->tm.tiles_j : 0);
+  // (at least 512: the grids of the one-launch form)
+  const int nblk = std::max(std::max(std::max(flux_block_count(NP), m.npatch), 512),
+                            ctx->tile_ok ? ctx->tm.tiles_i * ctx->tm.tiles_j : 0);
   ctx->partial_blocks = nblk;
   if ((s = ctx_alloc(ctx, (void **)&st.U, 4 * (size_t)NT * dsz)) != CFD_OK) return bail(s);
   if ((s = ctx_alloc(ctx, (void **)&st.S, 4 * (size_t)NP * dsz)) != CFD_OK) return bail(s);
@@ -1326,7 +1339,9 @@ cfd_status cfd_create(const cfd_mesh_desc *d, const cfd_config *cfg, cfd_ctx **o
     if ((s = ctx_alloc(ctx, (void **)&ctx->pbuf[q], 5 * (size_t)NT * dsz)) != CFD_OK) return bail(s);
     if (cudaMemset(ctx->pbuf[q], 0, 5 * (size_t)NT * dsz) != cudaSuccess) return bail(fail(CFD_ERR_CUDA, "memset failed"));
   }
-  if ((s = ctx_alloc(ctx, (void **)&st.partial, 9 * (size_t)(nblk + kMaxGroups) * dsz)) != CFD_OK) return bail(s);
+  if ((s = ctx_alloc(ctx, (void **)&st.partial, std::max<size_t>(9 * (size_t)(nblk + kMaxGroups),
+                                                                 512 * (size_t)(9 + kStepsPerLaunch)) * dsz)) != CFD_OK)
+    return bail(s);
   const size_t counter_bytes = 64 + 4 * (size_t)(kMaxGroups + 1);
   if ((s = ctx_alloc(ctx, (void **)&st.counter, counter_bytes)) != CFD_OK) return bail(s);
   st.gcount = st.counter + 16;
@@ -1437,6 +1452,7 @@ cfd_status cfd_set_option(cfd_ctx *ctx, const char *name, double value) {
     ctx->fp.faces_shape = static_cast<int>(value);
   }
   else if (n == "pdl") ctx->dm.pdl = value != 0.0;
+  else if (n == "one_launch_steps") ctx->steps_off = value == 0.0;
   else if (n == "profile") ctx->profile = value != 0.0;
   else if (n == "fuse_gather") ctx->fuse_gather = value != 0.0;
   else if (n == "patch_stage") ctx->patch_stage = value != 0.0;
@@ -1544,7 +1560,58 @@ static cfd_status enqueue_steps_persistent(cfd_ctx *ctx, int n_steps) {
   return CFD_OK;
 }
 
+// Whether the pseudo-steps of this context can run as one launch: the fused face-based form with a dt
+// frozen per step, every ghost private to its owner, none of the other launch forms chosen.
+static bool one_launch_form(const cfd_ctx *ctx) {
+  const StagePlan p = stage_plan(ctx->cfg, ctx->fp.consistent);
+  return ctx->dm.NF > 0 && !ctx->steps_off && ctx->fuse_gather && ctx->use_graph && !ctx->profile && !ctx->patch_stage &&
+         !ctx->tile_stage && !ctx->fp.weno && ctx->ghost_private && p.kind0 != 0 && p.lts_mode == 1 &&
+         ctx->cfg.local_time_stepping;
+}
+
+// Decides the launch for the given instances and uploads the blocks' shares.
+static cfd_status prepare_steps(cfd_ctx *ctx, const std::vector<int4> &inst) {
+  std::vector<StepsBlock> blocks;
+  ctx->steps = inst.empty() ? StepsShape{}
+                            : steps_shape(ctx->fp, ctx->bptr.data(), inst.data(), static_cast<int>(inst.size()), blocks);
+  if (ctx->steps.blocks == 0) return CFD_OK;
+  if (!ctx->d_steps) {
+    cudaDeviceGetAttribute(&ctx->steps_sms, cudaDevAttrMultiProcessorCount, ctx->cfg.device);
+    cfd_status s;
+    const size_t n = sizeof(unsigned int) * ((size_t)ctx->steps_sms * kStepsBarrierStride + 32);
+    if ((s = ctx_alloc(ctx, (void **)&ctx->d_steps, sizeof(StepsBlock) * (size_t)ctx->steps_sms)) != CFD_OK ||
+        (s = ctx_alloc(ctx, (void **)&ctx->d_arrivals, n)) != CFD_OK)
+      return s;
+    CUDA_TRY(cudaMemsetAsync(ctx->d_arrivals, 0, n, ctx->stream));
+  }
+  CUDA_TRY(cudaMemcpyAsync(ctx->d_steps, blocks.data(), sizeof(StepsBlock) * blocks.size(), cudaMemcpyHostToDevice,
+                           ctx->stream));
+  return CFD_OK;
+}
+
+static cfd_status enqueue_steps_one_launch(cfd_ctx *ctx, int n_steps, bool batch) {
+  const StagePlan p = stage_plan(ctx->cfg, ctx->fp.consistent);
+  for (int i = 0; i < n_steps; i += kStepsPerLaunch)
+    ctx->launches += launch_steps(ctx->stream, ctx->dm, ctx->ds, ctx->fp, ctx->bp, ctx->steps, ctx->d_steps,
+                                  ctx->d_arrivals, ctx->d_arrivals + (size_t)ctx->steps_sms * kStepsBarrierStride,
+                                  std::min(kStepsPerLaunch, n_steps - i), p.n, p.kind0, ctx->keep_delu, batch ? 0 : 1,
+                                  ctx->t_end_set ? 1 : 0, ctx->persist_test_arrivals);
+  CUDA_TRY(cudaGetLastError());
+  ctx->prim_from_S = false;
+  return CFD_OK;
+}
+
 static cfd_status enqueue_steps(cfd_ctx *ctx, int n_steps) {
+  if (n_steps > 1 && !ctx->persistent && !ctx->dm.cblk && one_launch_form(ctx)) {
+    if (!ctx->steps_known) {
+      cfd_status s = prepare_steps(ctx, {make_int4(0, ctx->NP, 0, ctx->dm.NF)});
+      if (s != CFD_OK) return s;
+      ctx->steps_known = true;
+    }
+    if (ctx->steps.blocks > 0) return enqueue_steps_one_launch(ctx, n_steps, false);
+  }
+  if (ctx->dm.cblk && ctx->steps.blocks > 0 && ctx->persist_test_arrivals == 0 && one_launch_form(ctx))
+    return enqueue_steps_one_launch(ctx, n_steps, true);
   if (ctx->persistent && ctx->persist_grid > 0 && ctx->dm.NF > 0) return enqueue_steps_persistent(ctx, n_steps);
   if (ctx->use_graph && !ctx->profile && n_steps > 1) {
     if (!ctx->graph) {
@@ -1574,6 +1641,7 @@ cfd_status cfd_step(cfd_ctx *ctx, int n_steps, double t_end, cfd_step_info *info
   ctx->launches += launch_set_ctl(ctx->stream, ctx->ds, CTL_TEND, t_end);
   ctx->launches += launch_set_ctl(ctx->stream, ctx->ds, CTL_DONE, 0.0);
   CUDA_TRY(cudaGetLastError());
+  ctx->t_end_set = t_end > 0.0;  // (the device keeps the value for later asynchronous steps too)
   if (t_end > 0.0) {
     // Steps past t_end are no-ops on the device; check the done flag between chunks so that a
     // large n_steps does not queue work that will be skipped.
@@ -2154,6 +2222,12 @@ static cfd_status batch_tables(cfd_batch *b) {
   ctx->dm.n_bblk = static_cast<int>(t[2].size());
   ctx->dm.rblk = p[3];
   ctx->dm.n_rblk = static_cast<int>(t[3].size());
+  // The one-launch form's blocks over the active instances (when they are few and small enough).
+  std::vector<int4> inst;
+  for (int i = 0; i < b->n; i++)
+    if (b->active[i]) inst.push_back(make_int4(b->cs[i], b->ce[i], b->fs[i], b->fe[i]));
+  const cfd_status steps_status = prepare_steps(ctx, inst);
+  if (steps_status != CFD_OK) return steps_status;
   drop_graphs(ctx);
   CUDA_TRY(cudaStreamSynchronize(ctx->stream));
   return CFD_OK;

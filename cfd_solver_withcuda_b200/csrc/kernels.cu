@@ -5,6 +5,7 @@
 // result is deterministic and bit-identical; there are no atomics on data.  Reductions (min dt,
 // residual and error norms) use a fixed-shape warp-shuffle tree per block and a fixed-order pass
 // over the per-block partials (a last-block pass, or the two-level group pass of the last stage).
+#include <algorithm>
 #include <climits>
 #include <type_traits>
 
@@ -313,16 +314,32 @@ __global__ void k_prim_all(DevMesh m, DevState st) {
 //   fixed-p exit     src/Exit_Boundary_Conditions.cpp:8-66 (exit kind 3)
 // src_is_S: the supersonic-exit copy reads the stage state (stage-consistent forms) instead of
 // U^n; cur_is_S: the state the primitives were last computed from is the stage state.
-__device__ __forceinline__ void bc_entry(const DevMesh &m, const DevState &st, const BcParams &bp, int e, int src_is_S,
-                                         int cur_is_S) {
-  const int4 b = m.bnd[e];
-  const int kind = b.x, c = b.y, f = b.z, g = b.w;
-  const int NT = m.NT, NP = m.NP;
-  const double *prim = st.prim;
-  const double rho = prim[c], u = prim[NT + c], v = prim[2 * NT + c], p = prim[3 * NT + c];
+// Values a boundary state is formed from, read from global memory when a kind needs them.
+struct BcGlobal {
+  const DevMesh &m;
+  const DevState &st;
+  int c, f, e, src_is_S, cur_is_S;
+  const double4 *bstate;
+  const double *bexit;
+  __device__ __forceinline__ double nx() const { return m.nx[f * m.NP + c]; }
+  __device__ __forceinline__ double ny() const { return m.ny[f * m.NP + c]; }
+  __device__ __forceinline__ double a() const { return st.prim[4 * m.NT + c]; }
+  __device__ __forceinline__ double cur(int k) const {
+    return cur_is_S ? st.S[(size_t)k * m.NP + c] : st.U[(size_t)k * m.NT + c];
+  }
+  __device__ __forceinline__ double src(int k) const {
+    return src_is_S ? st.S[(size_t)k * m.NP + c] : st.U[(size_t)k * m.NT + c];
+  }
+};
+
+// Conserved ghost state G of an entry of `kind` whose cell has the primitives (rho, u, v, p); false when
+// the entry leaves its ghost alone.
+template <typename Src>
+__device__ __forceinline__ bool bc_values(const Src &s, const BcParams &bp, int kind, double rho, double u, double v,
+                                          double p, double G[4]) {
   double G0, G1, G2, G3;
   if (kind == 2 || kind == 3) {
-    const double n1 = m.nx[f * NP + c], n2 = m.ny[f * NP + c];
+    const double n1 = s.nx(), n2 = s.ny();
     double vdotn = (u * n1 + v * n2);
     double v1g = u - 2.0 * vdotn * n1;
     double v2g = v - 2.0 * vdotn * n2;
@@ -333,19 +350,17 @@ __device__ __forceinline__ void bc_entry(const DevMesh &m, const DevState &st, c
     G3 = ((p / kGM1) + rho * vmag);
   } else if (kind == 0) {
     if (bp.inlet_bc == 4) {
-      const double *Uc = cur_is_S ? st.S : st.U;
-      const int ld = cur_is_S ? NP : NT;
-      const double Ui[4] = {Uc[c], Uc[ld + c], Uc[2 * ld + c], Uc[3 * ld + c]};
+      const double Ui[4] = {s.cur(0), s.cur(1), s.cur(2), s.cur(3)};
       double Gf[4];
-      const double4 fs = m.bstate ? m.bstate[e] : make_double4(bp.inlet_rho, bp.inlet_u, bp.inlet_v, bp.inlet_p);
-      farfield_state(Ui, m.nx[f * NP + c], m.ny[f * NP + c], fs.x, fs.y, fs.z, fs.w, Gf);
+      const double4 fs = s.bstate ? s.bstate[s.e] : make_double4(bp.inlet_rho, bp.inlet_u, bp.inlet_v, bp.inlet_p);
+      farfield_state(Ui, s.nx(), s.ny(), fs.x, fs.y, fs.z, fs.w, Gf);
       G0 = Gf[0];
       G1 = Gf[1];
       G2 = Gf[2];
       G3 = Gf[3];
     } else if (bp.inlet_bc == 3) {
       // Fully prescribed inflow (rho, u, v, p), per boundary entry when given (batched solves).
-      const double4 q = m.bstate ? m.bstate[e] : make_double4(bp.inlet_rho, bp.inlet_u, bp.inlet_v, bp.inlet_p);
+      const double4 q = s.bstate ? s.bstate[s.e] : make_double4(bp.inlet_rho, bp.inlet_u, bp.inlet_v, bp.inlet_p);
       G0 = q.x;
       G1 = q.x * q.y;
       G2 = q.x * q.z;
@@ -370,11 +385,11 @@ __device__ __forceinline__ void bc_entry(const DevMesh &m, const DevState &st, c
       // H0 = a0^2/(g-1) = a^2/(g-1) + Vn^2/2 this gives
       //   (g+1)/(g-1) a^2 - 2 R+ a + (g-1)/2 R+^2 - a0^2 = 0   (larger root),
       // then Vn = R+ - 2a/(g-1), T = a^2/(g R), p = p0 (T/T0)^(g/(g-1)), rho = p/(R T).
-      const double n1 = m.nx[f * NP + c], n2 = m.ny[f * NP + c];
-      const double a_i = prim[4 * NT + c];
+      const double n1 = s.nx(), n2 = s.ny();
+      const double a_i = s.a();
       const double vn_i = u * n1 + v * n2;
       const double Rp = vn_i + 2.0 * a_i / kGM1;
-      const double p0 = m.bstate ? m.bstate[e].x : bp.inlet_p0, t0 = m.bstate ? m.bstate[e].y : bp.inlet_t0;
+      const double p0 = s.bstate ? s.bstate[s.e].x : bp.inlet_p0, t0 = s.bstate ? s.bstate[s.e].y : bp.inlet_t0;
       const double a0sq = kGamma * bp.r_gas * t0;
       const double qa = (kGamma + 1.0) / kGM1, qb = -2.0 * Rp, qc = 0.5 * kGM1 * Rp * Rp - a0sq;
       const double disc = qb * qb - 4.0 * qa * qc;
@@ -391,19 +406,16 @@ __device__ __forceinline__ void bc_entry(const DevMesh &m, const DevState &st, c
       G3 = pb / kGM1 + 0.5 * rb * (ub * ub + vb * vb);
     }
   } else {  // exit
-    if (bp.exit_bc == 1) return;
-    const double *Us = src_is_S ? st.S : st.U;
-    const int ld = src_is_S ? NP : NT;
+    if (bp.exit_bc == 1) return false;
     if (bp.exit_bc == 0) {
-      G0 = Us[c];
-      G1 = Us[ld + c];
-      G2 = Us[2 * ld + c];
-      G3 = Us[3 * ld + c];
+      G0 = s.src(0);
+      G1 = s.src(1);
+      G2 = s.src(2);
+      G3 = s.src(3);
     } else if (bp.exit_bc == 3) {
-      const double rho_Et = cur_is_S ? st.S[3 * NP + c] : st.U[3 * NT + c];
+      const double rho_Et = s.cur(3);
       double Gf[4];
-      fixed_p_exit_state(rho, u, v, p, rho_Et, m.nx[f * NP + c], m.ny[f * NP + c], m.bexit ? m.bexit[e] : bp.exit_p,
-                         Gf);
+      fixed_p_exit_state(rho, u, v, p, rho_Et, s.nx(), s.ny(), s.bexit ? s.bexit[s.e] : bp.exit_p, Gf);
       G0 = Gf[0];
       G1 = Gf[1];
       G2 = Gf[2];
@@ -411,25 +423,40 @@ __device__ __forceinline__ void bc_entry(const DevMesh &m, const DevState &st, c
     } else {
       // Static-pressure outflow: rho, V extrapolated; p prescribed when the normal Mach
       // number is subsonic, extrapolated otherwise.
-      const double n1 = m.nx[f * NP + c], n2 = m.ny[f * NP + c];
-      const double a_i = prim[4 * NT + c];
+      const double n1 = s.nx(), n2 = s.ny();
+      const double a_i = s.a();
       const double vn = u * n1 + v * n2;
-      const double pb = (vn < a_i) ? (m.bexit ? m.bexit[e] : bp.exit_p) : p;
+      const double pb = (vn < a_i) ? (s.bexit ? s.bexit[s.e] : bp.exit_p) : p;
       G0 = rho;
       G1 = rho * u;
       G2 = rho * v;
       G3 = pb / kGM1 + 0.5 * rho * (u * u + v * v);
     }
   }
-  double *U = st.U;
-  U[g] = G0;
-  U[NT + g] = G1;
-  U[2 * NT + g] = G2;
-  U[3 * NT + g] = G3;
+  G[0] = G0;
+  G[1] = G1;
+  G[2] = G2;
+  G[3] = G3;
+  return true;
+}
+
+__device__ __forceinline__ void store_ghost(const DevState &st, int NT, int g, const double G[4]) {
+#pragma unroll
+  for (int k = 0; k < 4; k++) st.U[(size_t)k * NT + g] = G[k];
   Prim q;
-  bool ok = eos_prim(G0, G1, G2, G3, q);
+  const bool ok = eos_fast(G[0], G[1], G[2], G[3], q);
   store_prim(st.prim, st.q4, NT, g, q);
   if (!ok) flag_bad(st.status, g);
+}
+
+__device__ __forceinline__ void bc_entry(const DevMesh &m, const DevState &st, const BcParams &bp, int e, int src_is_S,
+                                         int cur_is_S) {
+  const int4 b = m.bnd[e];
+  const int c = b.y, NT = m.NT;
+  const BcGlobal src{m, st, c, b.z, e, src_is_S, cur_is_S, m.bstate, m.bexit};
+  double G[4];
+  if (bc_values(src, bp, b.x, st.prim[c], st.prim[NT + c], st.prim[2 * NT + c], st.prim[3 * NT + c], G))
+    store_ghost(st, NT, b.w, G);
 }
 
 __global__ void k_bc(DevMesh m, DevState st, BcParams bp, int src_is_S, int cur_is_S) {
@@ -1078,6 +1105,32 @@ __global__ void __launch_bounds__(MINB >= 6 ? 128 : 256, MINB) k_faces(const __g
 // face are in flight together; only the sums are predicated on the count.
 // CG: the face fluxes were written earlier in the same launch by other thread blocks (the
 // persistent stage kernel), so they are loaded from L2 (ld.global.cg), not through L1.
+__device__ __forceinline__ int face_id(int e) { return e < 0 ? -e - 1 : e; }
+
+// Sum of a cell's face fluxes in face order, negated on the neighbour side.
+__device__ __forceinline__ void sum_faces(int nf, const int4 e4, const double4 F0, const double4 F1, const double4 F2,
+                                          const double4 F3, double R[4]) {
+  const int e[4] = {e4.x, e4.y, e4.z, e4.w};
+  const double4 F[4] = {F0, F1, F2, F3};
+  R[0] = R[1] = R[2] = R[3] = 0.0;
+#pragma unroll
+  for (int f = 0; f < 4; f++) {
+    if (f < nf) {
+      if (e[f] < 0) {
+        R[0] += -F[f].x;
+        R[1] += -F[f].y;
+        R[2] += -F[f].z;
+        R[3] += -F[f].w;
+      } else {
+        R[0] += F[f].x;
+        R[1] += F[f].y;
+        R[2] += F[f].z;
+        R[3] += F[f].w;
+      }
+    }
+  }
+}
+
 template <bool DEN = true, bool CG = false>
 __device__ __forceinline__ void gather_faces(const DevMesh &m, const DevState &st, int c, double R[4], double &den) {
   const int NP = m.NP, NT = m.NT;
@@ -1207,14 +1260,11 @@ __device__ __forceinline__ void load_stage_in(const DevMesh &m, const DevState &
   }
 }
 
-__device__ __forceinline__ void cell_update_in(const DevMesh &m, const DevState &st, int c, int kind, double dt,
-                                               const double Rk[4], const StageIn &in, int fuse_final, int keep_delu,
-                                               double e[8]) {
-  const int NP = m.NP, NT = m.NT;
+// out: the stage state, or (final stages, true returned) dU or U^{n+1} itself.
+__device__ __forceinline__ bool stage_values(const DevMesh &m, const DevState &st, int c, int kind, double dt,
+                                             const double Rk[4], const double Un[4], const StageIn &in, double out[4]) {
+  const int NP = m.NP;
   const double invA = in.invA;
-  double Un[4], out[4];
-#pragma unroll
-  for (int k = 0; k < 4; k++) Un[k] = in.Un[k];
   bool final_stage = false;
   if (kind == 1 || kind == 21) {
 #pragma unroll
@@ -1271,6 +1321,17 @@ __device__ __forceinline__ void cell_update_in(const DevMesh &m, const DevState 
     }
     final_stage = true;
   }
+  return final_stage;
+}
+
+__device__ __forceinline__ void cell_update_in(const DevMesh &m, const DevState &st, int c, int kind, double dt,
+                                               const double Rk[4], const StageIn &in, int fuse_final, int keep_delu,
+                                               double e[8]) {
+  const int NP = m.NP, NT = m.NT;
+  double Un[4], out[4];
+#pragma unroll
+  for (int k = 0; k < 4; k++) Un[k] = in.Un[k];
+  const bool final_stage = stage_values(m, st, c, kind, dt, Rk, Un, in, out);
   if (!final_stage) {
 #pragma unroll
     for (int k = 0; k < 4; k++) st.S[k * NP + c] = out[k];
@@ -1513,6 +1574,24 @@ __device__ __forceinline__ void gg_gradient(const DevMesh &m, const double *q, i
   g1 *= m.inv_area[c];
 }
 
+// One face's part of a cell's Green-Gauss sums g (its four variables) and, with DT, of the denominator of
+// del_t (Inviscid_Time_Step, src/Time_Step.cpp:293-329).
+template <bool DT>
+__device__ __forceinline__ void gg_face(const double qc[4], double ac, const double qn[4], double nx, double ny,
+                                        double dl, double g[8], double &den) {
+  const double wx = nx * dl, wy = ny * dl;
+#pragma unroll
+  for (int k = 0; k < 4; k++) {
+    const double qf = 0.5 * (qc[k] + qn[k]);
+    g[2 * k] += qf * wx;
+    g[2 * k + 1] += qf * wy;
+  }
+  if (DT) {
+    const double vnf = qc[1] * nx + qc[2] * ny;
+    den += (fabs(vnf) + ac) * dl;
+  }
+}
+
 // Green-Gauss gradients of (rho, u, v, p) of physical cell c from the primitive planes `prim`
 // ([5][NT]), multiplied by 1/A (g[2k], g[2k+1]: d/dx, d/dy of variable k), and with DT the
 // denominator of del_t (Inviscid_Time_Step, src/Time_Step.cpp:293-329, faces in order).  The
@@ -1553,18 +1632,7 @@ __device__ __forceinline__ void cell_gradients(const DevMesh &m, const double *p
   for (int f = 0; f < 4; f++) {
     if (f >= nf) break;
     const int idx = f * NP + c;
-    const double nxf = m.nx[idx], nyf = m.ny[idx], dlf = m.dl[idx];
-    const double wx = nxf * dlf, wy = nyf * dlf;
-#pragma unroll
-    for (int k = 0; k < 4; k++) {
-      const double qf = 0.5 * (qc[k] + qn[f][k]);
-      g[2 * k] += qf * wx;
-      g[2 * k + 1] += qf * wy;
-    }
-    if (DT) {
-      const double vnf = qc[1] * nxf + qc[2] * nyf;
-      den += (fabs(vnf) + ac) * dlf;
-    }
+    gg_face<DT>(qc, ac, qn[f], m.nx[idx], m.ny[idx], m.dl[idx], g, den);
   }
 #pragma unroll
   for (int k = 0; k < 8; k++) g[k] = g[k] * ia;
@@ -1752,6 +1820,328 @@ __global__ void __launch_bounds__(kPersistBlock, MINB) k_persistent_stage(const 
     }
   }
   if (fuse_final && final_kind(kind)) stage_final_reduce(st, e, dtu);
+}
+
+// ---- Whole pseudo-steps in one launch (small and mid-size meshes; no reference counterpart) ----
+// On a few thousand cells a pseudo-step of the separate kernels is nine launches of a few microseconds,
+// nearly all of it launch latency and chains of dependent loads (the index, the geometry it names, the
+// count that says how many faces follow ...).  Here one cooperative launch, at most a block per SM, runs
+// many pseudo-steps.  Every block keeps a fixed range of one instance's cells and faces whose geometry,
+// connectivity, boundary entries and own states stay in shared memory; only what other blocks read goes
+// through global memory: the (rho, u, v, p) rows, the gradient records and the face fluxes, one round of
+// loads per phase.  A barrier over the instance's blocks separates the phases (gradients; face fluxes;
+// gather and update): a single solve is one group of blocks, a batch one per active instance, with blocks
+// in proportion to its cells.  Values written in the launch by other blocks are read after the barrier's
+// acquire.  The operations are those of the separate kernels in the same order, so states, Min_dt and
+// Total_Time are the same bits; the norms are summed over this grid's blocks (another order).  What the
+// next step overwrites before anyone can read it (R, del_t's last evaluation, the primitive planes, the
+// norms) is formed in the launch's last step alone unless a t_end may end the run at any step.
+// (As one thread-block cluster with the hardware's cluster barrier, 2,048 cells took 25 us per
+// pseudo-step exchanging through L2 and 30 us through the cluster's shared memory.)
+struct StepsArgs {
+  int n_steps, n_stages, kind0, keep_delu;
+  int cells, faces, entries;  // shared-memory capacity per block
+  int reduce;                 // norms, Min_dt and Total_Time (single solves)
+  int may_stop;               // a t_end is set
+  const StepsBlock *blocks;
+  unsigned int *arrivals;     // [groups * kStepsBarrierStride], 0 before the launch, and the give-up flag
+  unsigned int *gave_up;
+  unsigned int test_arrivals;
+};
+
+// Barrier over the n blocks of one group: arrivals count up from 0 and every block polls the count itself,
+// so the last arrival reaches the others in one hop.  The waits are bounded like grid_barrier's: a block
+// that waits longer than kBarrierCycles records CFD_ERR_TIMEOUT and raises the give-up flag, after which
+// no block of this context waits again, so the launch always ends.
+__device__ __forceinline__ void steps_barrier(const DevState &st, const StepsArgs &a, unsigned int *count, unsigned int n,
+                                              unsigned int &target) {
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    volatile unsigned int *gave_up = a.gave_up;
+    target += n;
+    asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(count) : "memory");
+    const long long t0 = clock64();
+    for (;;) {
+      unsigned int v;
+      asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(count) : "memory");
+      if (v >= target + a.test_arrivals) break;
+      if (*gave_up) break;
+      if (clock64() - t0 > kBarrierCycles) {
+        atomicCAS(st.status, 0, 5 /* CFD_ERR_TIMEOUT */);
+        *gave_up = 1u;
+        break;
+      }
+    }
+  }
+  __syncthreads();
+}
+
+constexpr int kStepsThreads = 512;
+// Shared memory of a block: per cell 12 geometry values, 1/A, U, the primitives (5), dt; per face 5 geometry
+// values; the tables.
+__host__ __device__ __forceinline__ size_t steps_smem(int cells, int faces, int entries) {
+  return sizeof(double) * (23 * (size_t)cells + 5 * (size_t)faces) + sizeof(int4) * (2 * (size_t)cells + entries) +
+         sizeof(int2) * (size_t)faces + sizeof(int) * (2 * (size_t)cells + 1);
+}
+
+// Values a boundary state is formed from when the cell's state is in shared memory (the current state is
+// both the exit copy's source and the state the primitives came from).
+struct BcShared {
+  const double *geo, *q, *U;
+  size_t ldU;
+  int P, l, f, e;
+  const double4 *bstate;
+  const double *bexit;
+  __device__ __forceinline__ double nx() const { return geo[(3 * f) * P + l]; }
+  __device__ __forceinline__ double ny() const { return geo[(3 * f + 1) * P + l]; }
+  __device__ __forceinline__ double a() const { return q[4 * P + l]; }
+  __device__ __forceinline__ double cur(int k) const { return U[k * ldU + l]; }
+  __device__ __forceinline__ double src(int k) const { return U[k * ldU + l]; }
+};
+
+template <typename T, int DISS>
+__global__ void __launch_bounds__(kStepsThreads, 1) k_steps(const __grid_constant__ DevMesh m,
+                                                            const __grid_constant__ DevState st,
+                                                            const __grid_constant__ FluxParams fp,
+                                                            const __grid_constant__ BcParams bp,
+                                                            const __grid_constant__ StepsArgs a) {
+  extern __shared__ __align__(16) double smd[];
+  if (step_done(st.ctl)) return;
+  const int NP = m.NP, NT = m.NT, P = a.cells, Q = a.faces;
+  const StepsBlock blk = a.blocks[blockIdx.x];
+  const int2 cr = make_int2(blk.c0, blk.c1), fr = make_int2(blk.f0, blk.f1);
+  unsigned int *const count = a.arrivals + (size_t)blk.group * kStepsBarrierStride;
+  const int nc = cr.y - cr.x, nfc = fr.y - fr.x, tid = threadIdx.x;
+  double *geo = smd, *ia = geo + 12 * P, *sU = ia + P, *sq = sU + 4 * P, *sdt = sq + 5 * P, *fg = sdt + P;
+  int4 *nb4 = reinterpret_cast<int4 *>(fg + 5 * Q);  // neighbour rows (the cell itself in unused slots)
+  int4 *cf4 = nb4 + P;                               // face slots
+  int4 *be = cf4 + P;                                // boundary entries: kind, face, ghost, id
+  int2 *fon = reinterpret_cast<int2 *>(be + a.entries);
+  int *bo = reinterpret_cast<int *>(fon + Q), *nf = bo + P + 1;  // first entry of each cell; face counts
+  unsigned int arrivals = 0;
+  const int e0 = nc > 0 ? m.bptr[cr.x] : 0;
+  for (int l = tid; l < nc; l += blockDim.x) {
+    const int c = cr.x + l;
+#pragma unroll
+    for (int f = 0; f < 4; f++) {
+      const size_t idx = (size_t)f * NP + c;
+      geo[(3 * f) * P + l] = m.nx[idx];
+      geo[(3 * f + 1) * P + l] = m.ny[idx];
+      geo[(3 * f + 2) * P + l] = m.dl[idx];
+    }
+    ia[l] = m.inv_area[c];
+#pragma unroll
+    for (int k = 0; k < 4; k++) sU[k * P + l] = st.U[(size_t)k * NT + c];
+    const double4 v = st.q4[c];
+    sq[l] = v.x;
+    sq[P + l] = v.y;
+    sq[2 * P + l] = v.z;
+    sq[3 * P + l] = v.w;
+    sq[4 * P + l] = st.prim[4 * (size_t)NT + c];
+    int4 n = m.nbr4[c];
+    n.x = n.x >= 0 && n.x < NT ? n.x : c;
+    n.y = n.y >= 0 && n.y < NT ? n.y : c;
+    n.z = n.z >= 0 && n.z < NT ? n.z : c;
+    n.w = n.w >= 0 && n.w < NT ? n.w : c;
+    nb4[l] = n;
+    cf4[l] = m.cface4[c];
+    nf[l] = m.nf[c];
+    const int b0 = m.bptr[c] - e0, b1 = m.bptr[c + 1] - e0;
+    bo[l] = b0;
+    if (l == nc - 1) bo[nc] = b1;
+    for (int i = b0; i < b1; i++) {
+      const int e = m.bidx[e0 + i];
+      const int4 b = m.bnd[e];
+      be[i] = make_int4(b.x, b.z, b.w, e);
+    }
+  }
+  for (int l = tid; l < nfc; l += blockDim.x) {
+    const int i = fr.x + l;
+    const double4 g = m.fg4[i];
+    fg[l] = g.x;
+    fg[Q + l] = g.y;
+    fg[2 * Q + l] = g.z;
+    fg[3 * Q + l] = g.w;
+    fg[4 * Q + l] = m.fdy[i];
+    fon[l] = m.fon[i];
+  }
+  __syncthreads();
+  // Ghost states of cell l's entries from its current state (Ucur, leading dimension ldU: U or the stage
+  // state).
+  auto ghosts = [&](int l, const double *Ucur, size_t ldU) {
+    for (int i = bo[l]; i < bo[l + 1]; i++) {
+      const int4 b = be[i];
+      const BcShared src{geo, sq, Ucur, ldU, P, l, b.y, b.w, m.bstate, m.bexit};
+      double G[4];
+      if (bc_values(src, bp, b.x, sq[l], sq[P + l], sq[2 * P + l], sq[3 * P + l], G)) store_ghost(st, NT, b.z, G);
+    }
+  };
+  const int glim = fp.limiter == LIM_REF_MINMOD ? LIM_MINMOD : fp.limiter;
+  __shared__ double sh_min[32], fmin_sh[kStepsPerLaunch];
+  double *step_min = st.partial + 9 * (size_t)gridDim.x;  // [gridDim.x][n_steps] block minima of the frozen dt
+  int step = 0;
+  for (; step < a.n_steps; step++) {
+    const bool full = step == a.n_steps - 1 || a.may_stop;  // this step's R, norms, ... can be read
+    for (int k = 0; k < a.n_stages; k++) {
+      const int kind = a.kind0 + k;
+      const bool last = k == a.n_stages - 1, with_dt = k == 0 || (last && full);
+      for (int l = tid; l < nc; l += blockDim.x) {
+        const int c = cr.x + l;
+        if (k == 0) ghosts(l, sU, P);
+        const int4 n = nb4[l];
+        const double4 v[4] = {st.q4[n.x], st.q4[n.y], st.q4[n.z], st.q4[n.w]};
+        double qn[4][4], nx[4], ny[4], dl[4];
+#pragma unroll
+        for (int f = 0; f < 4; f++) {
+          qn[f][0] = v[f].x;
+          qn[f][1] = v[f].y;
+          qn[f][2] = v[f].z;
+          qn[f][3] = v[f].w;
+          nx[f] = geo[(3 * f) * P + l];
+          ny[f] = geo[(3 * f + 1) * P + l];
+          dl[f] = geo[(3 * f + 2) * P + l];
+        }
+        const double qc[4] = {sq[l], sq[P + l], sq[2 * P + l], sq[3 * P + l]};
+        double g[8] = {0, 0, 0, 0, 0, 0, 0, 0}, den = 0.0;
+        const int cnt = nf[l];
+        const double ac = sq[4 * P + l];
+#pragma unroll
+        for (int f = 0; f < 4; f++)
+          if (f < cnt) gg_face<true>(qc, ac, qn[f], nx[f], ny[f], dl[f], g, den);
+#pragma unroll
+        for (int q = 0; q < 8; q++) g[q] *= ia[l];
+        if (sizeof(T) == sizeof(float)) {
+          float4 *r = st.recf + 2 * (size_t)c;
+          r[0] = make_float4(float(g[0]), float(g[1]), float(g[2]), float(g[3]));
+          r[1] = make_float4(float(g[4]), float(g[5]), float(g[6]), float(g[7]));
+        } else {
+          double4 *r = reinterpret_cast<double4 *>(st.rec + 8 * (size_t)c);
+          r[0] = make_double4(g[0], g[1], g[2], g[3]);
+          r[1] = make_double4(g[4], g[5], g[6], g[7]);
+        }
+        if (with_dt) {
+          const double dt = cell_dt_a(fp, m.area[c], den);
+          if (k == 0) sdt[l] = dt;
+          if (last) st.dtc[c] = dt;
+        }
+      }
+      steps_barrier(st, a, count, blk.blocks, arrivals);
+      for (int l = tid; l < nfc; l += blockDim.x) {
+        const int2 on = fon[l];
+        const int gn = on.y < NP ? on.y : on.x;  // a ghost neighbour uses the owner's gradients
+        const double4 c0 = st.q4[on.x], n0 = st.q4[on.y];
+        double4 c1, c2, n1, n2;
+        if (sizeof(T) == sizeof(float)) {
+          const float4 x = st.recf[2 * (size_t)on.x], y = st.recf[2 * (size_t)on.x + 1];
+          const float4 z = st.recf[2 * (size_t)gn], w = st.recf[2 * (size_t)gn + 1];
+          c1 = make_double4(x.x, x.y, x.z, x.w);
+          c2 = make_double4(y.x, y.y, y.z, y.w);
+          n1 = make_double4(z.x, z.y, z.z, z.w);
+          n2 = make_double4(w.x, w.y, w.z, w.w);
+        } else {
+          const double4 *rc = reinterpret_cast<const double4 *>(st.rec + 8 * (size_t)on.x);
+          const double4 *rn = reinterpret_cast<const double4 *>(st.rec + 8 * (size_t)gn);
+          c1 = rc[0];
+          c2 = rc[1];
+          n1 = rn[0];
+          n2 = rn[1];
+        }
+        FaceOps<T> o;
+        double4 F = face_flux_rec<T, DISS>(o, glim, c0, c1, c2, n0, n1, n2, T(fg[l]), T(fg[Q + l]), T(fg[2 * Q + l]),
+                                           T(fg[3 * Q + l]), T(fg[4 * Q + l]), T(fp.eflin), T(fp.shock_fix));
+        if constexpr (FaceOps<T>::fast) {
+          if (o.bad()) F = face_flux_again<DISS>(m, st, fp, fr.x + l);
+        }
+        st.F[fr.x + l] = F;
+      }
+      steps_barrier(st, a, count, blk.blocks, arrivals);
+      double dtu = 1e308 * 10.0;
+      double e[8] = {0, 0, 0, 0, 0, 0, 0, 0};
+      for (int l = tid; l < nc; l += blockDim.x) {
+        const int c = cr.x + l;
+        const int4 e4 = cf4[l];
+        double R[4];
+        sum_faces(nf[l], e4, st.F[face_id(e4.x)], st.F[face_id(e4.y)], st.F[face_id(e4.z)], st.F[face_id(e4.w)], R);
+        StageIn si;
+        si.invA = ia[l];
+        double Un[4], out[4];
+#pragma unroll
+        for (int q = 0; q < 4; q++) {
+          Un[q] = sU[q * P + l];
+          si.Sk[q] = st.S[(size_t)q * NP + c];
+        }
+        const double dt = sdt[l];
+        dtu = dt < dtu ? dt : dtu;
+        const bool fin = stage_values(m, st, c, kind, dt, R, Un, si, out);
+        if (fin) {
+          const bool direct = direct_kind(kind);
+#pragma unroll
+          for (int q = 0; q < 4; q++) {
+            const double du = direct ? out[q] - Un[q] : out[q];
+            const double nu = direct ? out[q] : Un[q] + out[q];
+            if (full) {
+              e[q] += err_term(du, Un[q]);
+              e[4 + q] += R[q] * R[q];
+              st.R[(size_t)q * NP + c] = R[q];
+              if (a.keep_delu) st.dU[(size_t)q * NP + c] = du;
+              st.U[(size_t)q * NT + c] = nu;
+            }
+            out[q] = nu;
+          }
+        }
+#pragma unroll
+        for (int q = 0; q < 4; q++) {
+          if (fin) sU[q * P + l] = out[q];
+          else st.S[(size_t)q * NP + c] = out[q];
+        }
+        Prim w;
+        const bool ok = eos_fast(out[0], out[1], out[2], out[3], w);
+        if (!ok) flag_bad(st.status, c);
+        sq[l] = w.rho;
+        sq[P + l] = w.u;
+        sq[2 * P + l] = w.v;
+        sq[3 * P + l] = w.p;
+        sq[4 * P + l] = w.a;
+        if (fin && full) store_prim(st.prim, st.q4, NT, c, w);
+        else st.q4[c] = make_double4(w.rho, w.u, w.v, w.p);
+        if (!fin) ghosts(l, st.S + cr.x, NP);
+        else if (full) st.dtk[c] = dt;
+      }
+      if (last && a.reduce) {
+        if (a.may_stop) {
+          stage_final_reduce(st, e, dtu);
+        } else if (step < a.n_steps - 1) {
+          const double bm = block_min(dtu, sh_min);
+          if (tid == 0) step_min[(size_t)blockIdx.x * a.n_steps + step] = bm;
+        } else {
+          // The earlier steps' Total_Time increments, in step order, before this step's own.
+          steps_barrier(st, a, count, blk.blocks, arrivals);
+          if (blockIdx.x == 0) {
+            for (int s0 = tid; s0 < a.n_steps - 1; s0 += blockDim.x) {
+              double v = 1e308 * 10.0;
+#pragma unroll 8
+              for (int i = 0; i < (int)gridDim.x; i++) {
+                const double w = step_min[(size_t)i * a.n_steps + s0];
+                v = w < v ? w : v;
+              }
+              fmin_sh[s0] = v;
+            }
+            __syncthreads();
+            if (tid == 0) {
+              double t = st.ctl[CTL_TOTAL_TIME];
+              for (int s0 = 0; s0 < a.n_steps - 1; s0++) t += fmin_sh[s0];
+              st.ctl[CTL_TOTAL_TIME] = t;
+              st.ctl[CTL_ITER] += double(a.n_steps - 1);
+            }
+          }
+          steps_barrier(st, a, count, blk.blocks, arrivals);
+          stage_final_reduce(st, e, dtu);
+        }
+      }
+      steps_barrier(st, a, count, blk.blocks, arrivals);
+    }
+    if (a.may_stop && step_done(st.ctl)) break;  // the same flag in every block
+  }
 }
 
 // Patch form of one stage of the face-based per-cell-dt forms: one thread block per patch of up
@@ -3260,6 +3650,100 @@ int launch_persistent_stage(cudaStream_t s, const DevMesh &m, DevState &st, cons
   BcParams bb = bp;
   void *args[] = {&mm, &ss, &ff, &bb, &kind, &lts, &fuse_final, &keep_delu, &flags, &with_dt, &with_bc, &test_arrivals};
   cudaLaunchCooperativeKernel(reinterpret_cast<const void *>(k), dim3(grid), dim3(kPersistBlock), args, 0, s);
+  return 1;
+}
+
+template <typename T>
+void *steps_kernel_t(const FluxParams &fp) {
+  switch (face_scheme(fp)) {
+    case 103: return reinterpret_cast<void *>(k_steps<T, 103>);
+    case 6: return reinterpret_cast<void *>(k_steps<T, 6>);
+    case 7: return reinterpret_cast<void *>(k_steps<T, 7>);
+    case 8: return reinterpret_cast<void *>(k_steps<T, 8>);
+    default: return reinterpret_cast<void *>(k_steps<T, 3>);
+  }
+}
+void *steps_kernel(const FluxParams &fp) { return fp.precision == 1 ? steps_kernel_t<float>(fp) : steps_kernel_t<double>(fp); }
+
+int device_sms() {
+  int dev = 0, sms = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
+    return 0;
+  return sms;
+}
+
+// Threads of a block whose widest phase has n items, in whole warps; at least four (reduce_rows takes
+// three of the nine reduced quantities per warp).
+int steps_threads(int n) {
+  const int t = (n + 31) & ~31;
+  return t < 128 ? 128 : (t > kStepsThreads ? kStepsThreads : t);
+}
+
+// This block's share of the items [begin, end): equal ranges of whole warps.
+static int2 block_share(int begin, int end, int rank, int blocks) {
+  const int per = (((end - begin + blocks - 1) / blocks) + 31) & ~31;
+  const int lo = std::min(begin + rank * per, end);
+  return make_int2(lo, std::min(lo + per, end));
+}
+
+StepsShape steps_shape(const FluxParams &fp, const int *bptr, const int4 *inst, int instances,
+                       std::vector<StepsBlock> &blocks) {
+  StepsShape sh{};
+  blocks.clear();
+  const int sms = device_sms();
+  int dev = 0, optin = 0, coop = 0;
+  if (sms <= 0 || instances < 1 || instances > sms || cudaGetDevice(&dev) != cudaSuccess ||
+      cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev) != cudaSuccess ||
+      cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev) != cudaSuccess || !coop)
+    return sh;
+  long long total = 0;
+  for (int i = 0; i < instances; i++) total += inst[i].y - inst[i].x;
+  if (total <= 0 || total > kStepsCells) return sh;
+  // Blocks in proportion to the cells, at least one each and no more than hold a warp of cells.
+  for (int i = 0; i < instances; i++) {
+    const int n = inst[i].y - inst[i].x;
+    int nb = static_cast<int>((long long)(sms - instances) * n / total) + 1;
+    nb = std::min(nb, (n + 31) / 32);
+    for (int r = 0; r < nb; r++) {
+      const int2 c = block_share(inst[i].x, inst[i].y, r, nb), f = block_share(inst[i].z, inst[i].w, r, nb);
+      blocks.push_back(StepsBlock{c.x, c.y, f.x, f.y, i, nb});
+      sh.cells = std::max(sh.cells, c.y - c.x);
+      sh.faces = std::max(sh.faces, f.y - f.x);
+      sh.entries = std::max(sh.entries, c.y > c.x ? bptr[c.y] - bptr[c.x] : 0);
+    }
+  }
+  sh.cells = (sh.cells + 3) & ~3;  // keeps the int4 tables behind the doubles aligned
+  sh.faces = (sh.faces + 3) & ~3;
+  const size_t sm = steps_smem(sh.cells, sh.faces, sh.entries);
+  const int room = optin - 4096;  // static shared memory of the reductions
+  const int threads = steps_threads(sh.faces);
+  int per_sm = 0;
+  void *k = steps_kernel(fp);
+  if (sm <= (size_t)room &&
+      cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, room) == cudaSuccess &&
+      cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k, threads, sm) == cudaSuccess && per_sm >= 1 &&
+      (int)blocks.size() <= sms) {
+    sh.blocks = static_cast<int>(blocks.size());
+    sh.threads = threads;
+    sh.groups = instances;
+  }
+  cudaGetLastError();
+  return sh;
+}
+
+int launch_steps(cudaStream_t s, const DevMesh &m, const DevState &st, const FluxParams &fp, const BcParams &bp,
+                 const StepsShape &sh, const StepsBlock *blocks, unsigned int *arrivals, unsigned int *gave_up, int n_steps,
+                 int n_stages, int kind0, int keep_delu, int reduce, int may_stop, unsigned int test_arrivals) {
+  DevMesh mm = m;
+  DevState ss = st;
+  FluxParams ff = fp;
+  BcParams bb = bp;
+  StepsArgs a{n_steps, n_stages, kind0,    keep_delu, sh.cells, sh.faces, sh.entries,
+              reduce,  may_stop, blocks,   arrivals,  gave_up,  test_arrivals};
+  void *args[] = {&mm, &ss, &ff, &bb, &a};
+  cudaMemsetAsync(arrivals, 0, sizeof(unsigned int) * (size_t)sh.groups * kStepsBarrierStride, s);
+  cudaLaunchCooperativeKernel(steps_kernel(fp), dim3(sh.blocks), dim3(sh.threads), args,
+                              steps_smem(sh.cells, sh.faces, sh.entries), s);
   return 1;
 }
 

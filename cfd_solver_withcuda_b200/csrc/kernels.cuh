@@ -107,7 +107,7 @@ struct DevState {
   double4 *F;    // [NF] face fluxes (face-based forms)
   // reduction / control block (see CtrlIdx)
   double *ctl;
-  double *partial;     // [(nblk_max + kMaxGroups) * 9]
+  double *partial;     // [(nblk_max + kMaxGroups) * 9], at least 512 * (9 + kStepsPerLaunch)
   unsigned int *counter;
   unsigned int *gcount;  // [kMaxGroups + 1] group and top counters of two-level reductions
   int *status;         // [0] status code, [1] first bad cell (device order)
@@ -211,6 +211,26 @@ int persistent_grid(const FluxParams &fp);
 int launch_persistent_stage(cudaStream_t s, const DevMesh &m, DevState &st, const FluxParams &fp,
                             const BcParams &bp, int kind, int lts, int fuse_final, int keep_delu, int flags,
                             int with_dt, int with_bc, int grid, unsigned int test_arrivals);
+// Whole pseudo-steps of the face-based forms with a dt frozen per step in one cooperative launch (k_steps).
+// steps_shape: the launch for `instances` solves over the cell and face ranges inst[i] (x, y; z, w), and
+// its blocks' shares; blocks = 0 when the separate kernels are the faster ones or the launch is not
+// available.  bptr: the cells' boundary-entry offsets (host copy).  cells, faces, entries: shared-memory
+// capacity per block.
+struct StepsBlock {
+  int c0, c1, f0, f1;  // cells and faces of this block
+  int group, blocks;   // its barrier group (instance) and the group's blocks
+};
+struct StepsShape {
+  int blocks, threads, groups, cells, faces, entries;
+};
+constexpr int kStepsCells = 98304;       // most cells of one launch, all instances together
+constexpr int kStepsPerLaunch = 128;     // bounds a launch's run time to a few milliseconds
+constexpr int kStepsBarrierStride = 32;  // a group's arrival count has its own 128 bytes
+StepsShape steps_shape(const FluxParams &fp, const int *bptr, const int4 *inst, int instances,
+                       std::vector<StepsBlock> &blocks);
+int launch_steps(cudaStream_t s, const DevMesh &m, const DevState &st, const FluxParams &fp, const BcParams &bp,
+                 const StepsShape &sh, const StepsBlock *blocks, unsigned int *arrivals, unsigned int *gave_up, int n_steps,
+                 int n_stages, int kind0, int keep_delu, int reduce, int may_stop, unsigned int test_arrivals);
 int launch_gather(cudaStream_t s, const DevMesh &m, DevState &st, const FluxParams &fp);
 // Fused gather + stage update of the per-cell-dt forms; del_t comes from the gradient pass
 // (launch_muscl_gradients with with_dt).  flags: bit 1 the owner thread writes its ghosts for the

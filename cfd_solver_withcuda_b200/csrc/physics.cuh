@@ -157,6 +157,25 @@ __host__ __device__ inline bool eos_prim(double U0, double U1, double U2, double
   return !(C != C);
 }
 
+// eos_prim with the branch-free operations (the same bits).
+__device__ __forceinline__ bool eos_fast(double U0, double U1, double U2, double U3, Prim &q) {
+  Fast64 o;
+  const double inv = o.inv(U0);
+  double v1 = U1 * inv, v2 = U2 * inv;
+  if (fabs(v1) <= 1e-10) v1 = 0.0;
+  if (fabs(v2) <= 1e-10) v2 = 0.0;
+  const double vmag = (v1 * v1 + v2 * v2);
+  const double P = kGM1 * (U3 - 0.5 * U0 * vmag);
+  const double C = o.root(kGamma * P * inv);
+  if (o.bad()) return eos_prim(U0, U1, U2, U3, q);
+  q.rho = U0;
+  q.u = v1;
+  q.v = v2;
+  q.p = P;
+  q.a = C;
+  return true;
+}
+
 // Calculate_Face_Average_Flux, src/Average_Interface_Flux.cpp:20-82 (wall flag is never set on
 // the reference path, src/Initialize.cpp:100).
 template <typename T>

@@ -240,6 +240,9 @@ cfd_status cfd_sync(cfd_ctx *ctx, cfd_step_info *info);
  * one CUDA graph per RK stage; default 0; the batched solves' form, see cfd_batch_set_option),
  * "persist_minb" (the persistent kernel's register budget: built for 4, 6 or 8 resident blocks per
  * SM; default 0: 6 in FP64 and 8 in the FP32-flux form, the faster of each on B200),
+ * "one_launch_steps" (multi-step calls of the face-based forms with a per-cell dt frozen per step, of at
+ * most 98,304 cells -- a batch's active instances together -- run many pseudo-steps in one cooperative
+ * launch; default 1, 0: the separate kernels),
  * "barrier_timeout_test" (a test of the bounded barriers: every barrier of the persistent form
  * waits for `value` more blocks than it has, so each wait runs out and the step reports
  * CFD_ERR_TIMEOUT; default 0),
@@ -255,8 +258,8 @@ cfd_status cfd_sync(cfd_ctx *ctx, cfd_step_info *info);
  * apply (or, for 2-4, the device offers no tensor copies) setting it is CFD_ERR_BAD_ARG),
  * "tile_prefetch" (tile forms 2-4: each block also prefetches into L2 the inputs of the tile that
  * starts one wave later; default 0).
- * None of the options changes a state bit (the persistent form sums the error norms in another
- * order). */
+ * None of the options changes a state bit (the persistent and one-launch forms sum the error norms in
+ * another order). */
 cfd_status cfd_set_option(cfd_ctx *ctx, const char *name, double value);
 /* Times every combination of the options above that applies to this configuration over `steps`
  * pseudo-steps of the context's own mesh and state, keeps the fastest and restores the state
