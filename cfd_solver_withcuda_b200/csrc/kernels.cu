@@ -72,6 +72,41 @@ void launch_k(const DevMesh &m, void (*k)(KArgs...), unsigned grid, unsigned blo
   launch_ks(m, k, grid, block, 0, s, args...);
 }
 
+// 32-byte loads and stores of sm_100 (32-byte aligned global addresses).  A warp's rows, records and fluxes
+// lie 32 or 64 bytes apart, so as pairs of 16-byte accesses every access touches each of its lines half
+// used, and the kernels that gather them were bound by the L1's passes over those lines.  The volatile
+// form keeps its place among the thread's stores.
+__device__ __forceinline__ double4 ld32(const double4 *p) {
+  double4 v;
+  asm("ld.global.v4.f64 {%0, %1, %2, %3}, [%4];" : "=d"(v.x), "=d"(v.y), "=d"(v.z), "=d"(v.w) : "l"(p));
+  return v;
+}
+__device__ __forceinline__ double4 ld32_ordered(const double4 *p) {
+  double4 v;
+  asm volatile("ld.global.v4.f64 {%0, %1, %2, %3}, [%4];"
+               : "=d"(v.x), "=d"(v.y), "=d"(v.z), "=d"(v.w)
+               : "l"(p)
+               : "memory");
+  return v;
+}
+__device__ __forceinline__ void st32(double4 *p, const double4 v) {
+  asm volatile("st.global.v4.f64 [%0], {%1, %2, %3, %4};" ::"l"(p), "d"(v.x), "d"(v.y), "d"(v.z), "d"(v.w) : "memory");
+}
+// Eight floats (a cell's FP32 gradients) as two double4.
+__device__ __forceinline__ void ld32f(const float4 *p, double4 &a, double4 &b) {
+  float v[8];
+  asm("ld.global.v8.f32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+      : "=f"(v[0]), "=f"(v[1]), "=f"(v[2]), "=f"(v[3]), "=f"(v[4]), "=f"(v[5]), "=f"(v[6]), "=f"(v[7])
+      : "l"(p));
+  a = make_double4(v[0], v[1], v[2], v[3]);
+  b = make_double4(v[4], v[5], v[6], v[7]);
+}
+__device__ __forceinline__ void st32f(float4 *p, const double g[8]) {
+  asm volatile("st.global.v8.f32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"(p), "f"(float(g[0])), "f"(float(g[1])),
+               "f"(float(g[2])), "f"(float(g[3])), "f"(float(g[4])), "f"(float(g[5])), "f"(float(g[6])), "f"(float(g[7]))
+               : "memory");
+}
+
 // Item handled by this thread: from the block's work-list range when a list is given (n when the
 // thread is past the range's end), else the plain global index.
 __device__ __forceinline__ int item_index(const int2 *blk, int n) {
@@ -94,7 +129,7 @@ __device__ __forceinline__ void store_prim(double *prim, double4 *q4, int NT, in
   prim[2 * NT + c] = q.v;
   prim[3 * NT + c] = q.p;
   prim[4 * NT + c] = q.a;
-  if (q4) q4[c] = make_double4(q.rho, q.u, q.v, q.p);
+  if (q4) st32(q4 + c, make_double4(q.rho, q.u, q.v, q.p));
 }
 
 __device__ __forceinline__ double warp_min(double v) {
@@ -925,62 +960,85 @@ __global__ void __launch_bounds__(kFluxBlock) k_weno(DevMesh m, DevState st, Flu
 // fp.eflin > 0).
 // Flux of one unique face from the owner's record (c0: rho, u, v, p; c1, c2: gradients) and the
 // neighbour's (n0, n1, n2), face normal (nx, ny), length dl and centre-to-centre vector (dx, dy).
-template <typename T, int DISS, typename O>
-__device__ __forceinline__ double4 face_flux_rec(O &o, int glim, const double4 c0, const double4 c1, const double4 c2,
-                                                 const double4 n0, const double4 n1, const double4 n2, const T nx,
-                                                 const T ny, const T dl, const T dx, const T dy, const T eflin,
-                                                 const T shock_fix = T(0.0)) {
+// FaceIn: what the flux needs of the two cells: the states, D+ and the two upwind differences per
+// variable, and (DISS 103) whether the pressure gradients mark a shock.
+template <typename T>
+struct FaceIn {
+  T qc[4], qn[4], dp[4], dmc[4], dmn[4];
+  bool shock;
+};
+template <typename T, int DISS>
+__device__ __forceinline__ void face_in(const double4 c0, const double4 c1, const double4 c2, const double4 n0,
+                                        const double4 n1, const double4 n2, const T dx, const T dy, const T shock_fix,
+                                        FaceIn<T> &in) {
   const T qc[4] = {T(c0.x), T(c0.y), T(c0.z), T(c0.w)};
   const T qn[4] = {T(n0.x), T(n0.y), T(n0.z), T(n0.w)};
   const T gc[8] = {T(c1.x), T(c1.y), T(c1.z), T(c1.w), T(c2.x), T(c2.y), T(c2.z), T(c2.w)};
   const T gn[8] = {T(n1.x), T(n1.y), T(n1.z), T(n1.w), T(n2.x), T(n2.y), T(n2.z), T(n2.w)};
-  T qL[4], qR[4], dp[4], dmc[4], dmn[4];
 #pragma unroll
   for (int k = 0; k < 4; k++) {
-    dp[k] = qn[k] - qc[k];
-    dmc[k] = T(2.0) * (gc[2 * k] * dx + gc[2 * k + 1] * dy) - dp[k];
-    dmn[k] = T(2.0) * (gn[2 * k] * dx + gn[2 * k + 1] * dy) - dp[k];
+    in.qc[k] = qc[k];
+    in.qn[k] = qn[k];
+    in.dp[k] = qn[k] - qc[k];
+    in.dmc[k] = T(2.0) * (gc[2 * k] * dx + gc[2 * k + 1] * dy) - in.dp[k];
+    in.dmn[k] = T(2.0) * (gn[2 * k] * dx + gn[2 * k + 1] * dy) - in.dp[k];
   }
+  in.shock = false;
+  if (DISS == 103 && shock_fix > T(0.0)) {
+    // Shock sensor of the hybrid: |grad p|^2 |d|^2 > (shock_fix p)^2 in either cell.
+    const T d2 = dx * dx + dy * dy;
+    const T gpc = gc[6] * gc[6] + gc[7] * gc[7], gpn = gn[6] * gn[6] + gn[7] * gn[7];
+    const T tc = shock_fix * qc[3], tn = shock_fix * qn[3];
+    in.shock = gpc * d2 > tc * tc || gpn * d2 > tn * tn;
+  }
+}
+
+template <int KIND>
+__device__ __forceinline__ void half_slopes(Fast64 &o, const FaceIn<double> &in, double qL[4], double qR[4]) {
+#pragma unroll
+  for (int k = 0; k < 4; k++) {
+    qL[k] = in.qc[k] + muscl_half_slope<KIND>(o, in.dmc[k], in.dp[k]);
+    qR[k] = in.qn[k] - muscl_half_slope<KIND>(o, in.dmn[k], in.dp[k]);
+  }
+}
+
+template <typename T, int DISS, typename O>
+__device__ __forceinline__ double4 face_flux_in(O &o, int glim, const FaceIn<T> &in, const T nx, const T ny, const T dl,
+                                                const T eflin) {
+  T qL[4], qR[4];
   // The slopes.  Fast64: one branch on the limiter for all eight, so that their divisions interleave.
   bool limited = false;
   if constexpr (O::fast) {
-    if (glim == LIM_VANLEER) {
-      limited = true;
+    limited = true;
+    if (glim == LIM_VANLEER) half_slopes<LIM_VANLEER>(o, in, qL, qR);
+    else if (glim == LIM_VANALBADA) half_slopes<LIM_VANALBADA>(o, in, qL, qR);
+    else if (glim == LIM_MINMOD) half_slopes<LIM_MINMOD>(o, in, qL, qR);
+    else limited = false;
+    // Non-positive densities or pressures (an integer test; NaN is flagged by the roots below).
+    if (limited) {
+      const bool badL = __double2hiint(qL[0]) <= 0 || __double2hiint(qL[3]) <= 0;
+      const bool badR = __double2hiint(qR[0]) <= 0 || __double2hiint(qR[3]) <= 0;
 #pragma unroll
       for (int k = 0; k < 4; k++) {
-        qL[k] = qc[k] + 0.5 * muscl_slope_fast<LIM_VANLEER>(o, dmc[k], dp[k]);
-        qR[k] = qn[k] - 0.5 * muscl_slope_fast<LIM_VANLEER>(o, dmn[k], dp[k]);
-      }
-    } else if (glim == LIM_VANALBADA) {
-      limited = true;
-#pragma unroll
-      for (int k = 0; k < 4; k++) {
-        qL[k] = qc[k] + 0.5 * muscl_slope_fast<LIM_VANALBADA>(o, dmc[k], dp[k]);
-        qR[k] = qn[k] - 0.5 * muscl_slope_fast<LIM_VANALBADA>(o, dmn[k], dp[k]);
-      }
-    } else if (glim == LIM_MINMOD) {
-      limited = true;
-#pragma unroll
-      for (int k = 0; k < 4; k++) {
-        qL[k] = qc[k] + 0.5 * muscl_slope<T>(LIM_MINMOD, dmc[k], dp[k]);
-        qR[k] = qn[k] - 0.5 * muscl_slope<T>(LIM_MINMOD, dmn[k], dp[k]);
+        qL[k] = badL ? in.qc[k] : qL[k];
+        qR[k] = badR ? in.qn[k] : qR[k];
       }
     }
   }
   if (!limited) {
 #pragma unroll
     for (int k = 0; k < 4; k++) {
-      qL[k] = qc[k] + T(0.5) * muscl_slope<T>(glim, dmc[k], dp[k]);
-      qR[k] = qn[k] - T(0.5) * muscl_slope<T>(glim, dmn[k], dp[k]);
+      qL[k] = in.qc[k] + T(0.5) * muscl_slope<T>(glim, in.dmc[k], in.dp[k]);
+      qR[k] = in.qn[k] - T(0.5) * muscl_slope<T>(glim, in.dmn[k], in.dp[k]);
     }
-  }
-  if (!(qL[0] > T(0.0)) || !(qL[3] > T(0.0))) {
+    if (!(qL[0] > T(0.0)) || !(qL[3] > T(0.0))) {
 #pragma unroll
-    for (int k = 0; k < 4; k++) qL[k] = qc[k];
-  }
-  if (!(qR[0] > T(0.0)) || !(qR[3] > T(0.0))) {
+      for (int k = 0; k < 4; k++) qL[k] = in.qc[k];
+    }
+    if (!(qR[0] > T(0.0)) || !(qR[3] > T(0.0))) {
 #pragma unroll
-    for (int k = 0; k < 4; k++) qR[k] = qn[k];
+      for (int k = 0; k < 4; k++) qR[k] = in.qn[k];
+    }
   }
   const T aL = o.root(o.div(T(kGamma) * qL[3], qL[0])), aR = o.root(o.div(T(kGamma) * qR[3], qR[0]));
   T A[4], D[4] = {T(0.0), T(0.0), T(0.0), T(0.0)};
@@ -988,14 +1046,7 @@ __device__ __forceinline__ double4 face_flux_rec(O &o, int glim, const double4 c
   // hybrid), a separate instance so that the plain form keeps its register footprint.
   if (DISS == 3 || DISS == 103) {
     average_flux<T>(qL[0], qL[1], qL[2], qL[3], qR[0], qR[1], qR[2], qR[3], nx, ny, dl, A);
-    // Shock sensor of the hybrid: |grad p|^2 |d|^2 > (shock_fix p)^2 in either cell.
-    bool rusanov = false;
-    if (DISS == 103 && shock_fix > T(0.0)) {
-      const T d2 = dx * dx + dy * dy;
-      const T gpc = gc[6] * gc[6] + gc[7] * gc[7], gpn = gn[6] * gn[6] + gn[7] * gn[7];
-      const T tc = shock_fix * qc[3], tn = shock_fix * qn[3];
-      rusanov = gpc * d2 > tc * tc || gpn * d2 > tn * tn;
-    }
+    const bool rusanov = DISS == 103 && in.shock;
     if (rusanov) {
       const T vnL = qL[1] * nx + qL[2] * ny, vnR = qR[1] * nx + qR[2] * ny;
       const T sL = fabs(vnL) + aL, sR = fabs(vnR) + aR;
@@ -1026,6 +1077,16 @@ __device__ __forceinline__ double4 face_flux_rec(O &o, int glim, const double4 c
     }
   }
   return make_double4(double(A[0] - D[0]), double(A[1] - D[1]), double(A[2] - D[2]), double(A[3] - D[3]));
+}
+
+template <typename T, int DISS, typename O>
+__device__ __forceinline__ double4 face_flux_rec(O &o, int glim, const double4 c0, const double4 c1, const double4 c2,
+                                                 const double4 n0, const double4 n1, const double4 n2, const T nx,
+                                                 const T ny, const T dl, const T dx, const T dy, const T eflin,
+                                                 const T shock_fix = T(0.0)) {
+  FaceIn<T> in;
+  face_in<T, DISS>(c0, c1, c2, n0, n1, n2, dx, dy, shock_fix, in);
+  return face_flux_in<T, DISS>(o, glim, in, nx, ny, dl, eflin);
 }
 
 // Division policy of the face kernels: the branch-free double operations, or plain float ones.
@@ -1064,39 +1125,29 @@ __global__ void __launch_bounds__(MINB >= 6 ? 128 : 256, MINB) k_faces(const __g
   const int2 on = m.fon[i];
   const int c = on.x, N = on.y;
   const int glim = fp.limiter == LIM_REF_MINMOD ? LIM_MINMOD : fp.limiter;
-  const double4 gq = m.fg4[i];
+  const double4 gq = ld32(m.fg4 + i);
   const T nx = T(gq.x), ny = T(gq.y), dl = T(gq.z), dx = T(gq.w), dy = T(m.fdy[i]);
-  const double4 c0 = st.q4[c], n0 = st.q4[N];
-  const bool nphys = N < NP;
+  const double4 c0 = ld32(st.q4 + c), n0 = ld32(st.q4 + N);
+  const int G = N < NP ? N : c;  // a ghost neighbour uses the owner's gradients
   double4 c1, c2, n1, n2;
   if (sizeof(T) == sizeof(float)) {
     // FP32-flux form: 32-byte float records (the values face_flux_rec would round to anyway).
-    const float4 *rc = st.recf + 2 * (size_t)c, *rn = st.recf + 2 * (size_t)N;
-    const float4 a = rc[0], b = rc[1];
-    c1 = make_double4(a.x, a.y, a.z, a.w);
-    c2 = make_double4(b.x, b.y, b.z, b.w);
-    if (nphys) {
-      const float4 p = rn[0], q = rn[1];
-      n1 = make_double4(p.x, p.y, p.z, p.w);
-      n2 = make_double4(q.x, q.y, q.z, q.w);
-    } else {
-      n1 = c1;
-      n2 = c2;
-    }
+    ld32f(st.recf + 2 * (size_t)c, c1, c2);
+    ld32f(st.recf + 2 * (size_t)G, n1, n2);
   } else {
     const double4 *rc = reinterpret_cast<const double4 *>(st.rec + 8 * (size_t)c);
-    const double4 *rn = reinterpret_cast<const double4 *>(st.rec + 8 * (size_t)N);
-    c1 = rc[0];
-    c2 = rc[1];
-    n1 = nphys ? rn[0] : c1;
-    n2 = nphys ? rn[1] : c2;
+    const double4 *rn = reinterpret_cast<const double4 *>(st.rec + 8 * (size_t)G);
+    c1 = ld32(rc);
+    c2 = ld32(rc + 1);
+    n1 = ld32(rn);
+    n2 = ld32(rn + 1);
   }
   FaceOps<T> o;
   double4 F = face_flux_rec<T, DISS>(o, glim, c0, c1, c2, n0, n1, n2, nx, ny, dl, dx, dy, T(fp.eflin), T(fp.shock_fix));
   if constexpr (FaceOps<T>::fast) {
     if (o.bad()) F = face_flux_again<DISS>(m, st, fp, i);
   }
-  st.F[i] = F;
+  st32(st.F + i, F);
 }
 
 // Sum of the face fluxes of cell c in face order (+F on the owner side, -F on the neighbour
@@ -1143,7 +1194,7 @@ __device__ __forceinline__ void gather_faces(const DevMesh &m, const DevState &s
 #pragma unroll
   for (int f = 0; f < 4; f++) {
     const int id = e[f] < 0 ? -e[f] - 1 : e[f];
-    F[f] = CG ? ldcg4(st.F + id) : st.F[id];
+    F[f] = CG ? ldcg4(st.F + id) : ld32(st.F + id);
   }
   R[0] = R[1] = R[2] = R[3] = 0.0;
   den = 0.0;
@@ -1615,7 +1666,7 @@ __device__ __forceinline__ void cell_gradients(const DevMesh &m, const double *p
 #pragma unroll
   for (int f = 0; f < 4; f++) {
     if (Q4) {
-      const double4 v = q4[nb[f]];
+      const double4 v = ld32_ordered(q4 + nb[f]);
       qn[f][0] = v.x;
       qn[f][1] = v.y;
       qn[f][2] = v.z;
@@ -1659,18 +1710,16 @@ __global__ void __launch_bounds__(kBlock, 4) k_muscl_gradients(DevMesh m, DevSta
       const int b0 = m.bptr[c], b1 = m.bptr[c + 1];
       for (int i = b0; i < b1; i++) bc_entry(m, st, bp, m.bidx[i], 0, 0);
     }
-    const double4 v = st.q4[c];
+    const double4 v = ld32_ordered(st.q4 + c);
     const double qc[4] = {v.x, v.y, v.z, v.w};
     double g[8], den;
     cell_gradients<DT, true>(m, st.prim, st.q4, c, qc, g, den);
     if (st.recf) {
-      float4 *r = st.recf + 2 * (size_t)c;
-      r[0] = make_float4(float(g[0]), float(g[1]), float(g[2]), float(g[3]));
-      r[1] = make_float4(float(g[4]), float(g[5]), float(g[6]), float(g[7]));
+      st32f(st.recf + 2 * (size_t)c, g);
     } else {
       double4 *r = reinterpret_cast<double4 *>(st.rec + 8 * (size_t)c);
-      r[0] = make_double4(g[0], g[1], g[2], g[3]);
-      r[1] = make_double4(g[4], g[5], g[6], g[7]);
+      st32(r, make_double4(g[0], g[1], g[2], g[3]));
+      st32(r + 1, make_double4(g[4], g[5], g[6], g[7]));
     }
     if (DT) st.dtc[c] = cell_dt(m, fp, c, den);
   }
@@ -1989,7 +2038,8 @@ __global__ void __launch_bounds__(kStepsThreads, 1) k_steps(const __grid_constan
         const int c = cr.x + l;
         if (k == 0) ghosts(l, sU, P);
         const int4 n = nb4[l];
-        const double4 v[4] = {st.q4[n.x], st.q4[n.y], st.q4[n.z], st.q4[n.w]};
+        const double4 v[4] = {ld32_ordered(st.q4 + n.x), ld32_ordered(st.q4 + n.y), ld32_ordered(st.q4 + n.z),
+                              ld32_ordered(st.q4 + n.w)};
         double qn[4][4], nx[4], ny[4], dl[4];
 #pragma unroll
         for (int f = 0; f < 4; f++) {
@@ -2011,13 +2061,11 @@ __global__ void __launch_bounds__(kStepsThreads, 1) k_steps(const __grid_constan
 #pragma unroll
         for (int q = 0; q < 8; q++) g[q] *= ia[l];
         if (sizeof(T) == sizeof(float)) {
-          float4 *r = st.recf + 2 * (size_t)c;
-          r[0] = make_float4(float(g[0]), float(g[1]), float(g[2]), float(g[3]));
-          r[1] = make_float4(float(g[4]), float(g[5]), float(g[6]), float(g[7]));
+          st32f(st.recf + 2 * (size_t)c, g);
         } else {
           double4 *r = reinterpret_cast<double4 *>(st.rec + 8 * (size_t)c);
-          r[0] = make_double4(g[0], g[1], g[2], g[3]);
-          r[1] = make_double4(g[4], g[5], g[6], g[7]);
+          st32(r, make_double4(g[0], g[1], g[2], g[3]));
+          st32(r + 1, make_double4(g[4], g[5], g[6], g[7]));
         }
         if (with_dt) {
           const double dt = cell_dt_a(fp, m.area[c], den);
@@ -2029,7 +2077,7 @@ __global__ void __launch_bounds__(kStepsThreads, 1) k_steps(const __grid_constan
       for (int l = tid; l < nfc; l += blockDim.x) {
         const int2 on = fon[l];
         const int gn = on.y < NP ? on.y : on.x;  // a ghost neighbour uses the owner's gradients
-        const double4 c0 = st.q4[on.x], n0 = st.q4[on.y];
+        const double4 c0 = ld32_ordered(st.q4 + on.x), n0 = ld32_ordered(st.q4 + on.y);
         double4 c1, c2, n1, n2;
         if (sizeof(T) == sizeof(float)) {
           const float4 x = st.recf[2 * (size_t)on.x], y = st.recf[2 * (size_t)on.x + 1];
@@ -2041,10 +2089,10 @@ __global__ void __launch_bounds__(kStepsThreads, 1) k_steps(const __grid_constan
         } else {
           const double4 *rc = reinterpret_cast<const double4 *>(st.rec + 8 * (size_t)on.x);
           const double4 *rn = reinterpret_cast<const double4 *>(st.rec + 8 * (size_t)gn);
-          c1 = rc[0];
-          c2 = rc[1];
-          n1 = rn[0];
-          n2 = rn[1];
+          c1 = ld32_ordered(rc);
+          c2 = ld32_ordered(rc + 1);
+          n1 = ld32_ordered(rn);
+          n2 = ld32_ordered(rn + 1);
         }
         FaceOps<T> o;
         double4 F = face_flux_rec<T, DISS>(o, glim, c0, c1, c2, n0, n1, n2, T(fg[l]), T(fg[Q + l]), T(fg[2 * Q + l]),
@@ -2052,7 +2100,7 @@ __global__ void __launch_bounds__(kStepsThreads, 1) k_steps(const __grid_constan
         if constexpr (FaceOps<T>::fast) {
           if (o.bad()) F = face_flux_again<DISS>(m, st, fp, fr.x + l);
         }
-        st.F[fr.x + l] = F;
+        st32(st.F + fr.x + l, F);
       }
       steps_barrier(st, a, count, blk.blocks, arrivals);
       double dtu = 1e308 * 10.0;
@@ -2061,7 +2109,8 @@ __global__ void __launch_bounds__(kStepsThreads, 1) k_steps(const __grid_constan
         const int c = cr.x + l;
         const int4 e4 = cf4[l];
         double R[4];
-        sum_faces(nf[l], e4, st.F[face_id(e4.x)], st.F[face_id(e4.y)], st.F[face_id(e4.z)], st.F[face_id(e4.w)], R);
+        sum_faces(nf[l], e4, ld32_ordered(st.F + face_id(e4.x)), ld32_ordered(st.F + face_id(e4.y)),
+                  ld32_ordered(st.F + face_id(e4.z)), ld32_ordered(st.F + face_id(e4.w)), R);
         StageIn si;
         si.invA = ia[l];
         double Un[4], out[4];
@@ -2103,7 +2152,7 @@ __global__ void __launch_bounds__(kStepsThreads, 1) k_steps(const __grid_constan
         sq[3 * P + l] = w.p;
         sq[4 * P + l] = w.a;
         if (fin && full) store_prim(st.prim, st.q4, NT, c, w);
-        else st.q4[c] = make_double4(w.rho, w.u, w.v, w.p);
+        else st32(st.q4 + c, make_double4(w.rho, w.u, w.v, w.p));
         if (!fin) ghosts(l, st.S + cr.x, NP);
         else if (full) st.dtk[c] = dt;
       }

@@ -63,6 +63,7 @@ struct Ieee {
   __device__ __forceinline__ T div(T a, const Rcp &r) { return a / r.b; }
   __device__ __forceinline__ T root(T a) { return sqrt(a); }
   __device__ __forceinline__ void flag() {}
+  __device__ __forceinline__ void need_positive(T) {}
   __device__ __forceinline__ bool bad() const { return false; }
 };
 
@@ -85,7 +86,18 @@ struct Fast64 {
     dlo = min(dlo, h);
     dhi = max(dhi, h);
   }
+  // Numerators known to be 0 or positive.
+  __device__ __forceinline__ void num_pos(double a) {
+    const unsigned h = static_cast<unsigned>(__double2hiint(a));
+    nlo = min(nlo, h - 1u);
+    nhi = max(nhi, h);
+  }
   __device__ __forceinline__ void flag() { dlo = 0u; }
+  // Flags values that are not positive (their sign bit or a zero high word; NaN is flagged where it is
+  // used).
+  __device__ __forceinline__ void need_positive(double a) {
+    if (__double2hiint(a) <= 0) dlo = 0u;
+  }
   __device__ __forceinline__ bool bad() const {
     return nlo < kNumLo || nhi > kNumHi || dlo < kDenLo || dhi > kDenHi;
   }
@@ -99,11 +111,18 @@ struct Fast64 {
                        static_cast<unsigned>(__double2loint(b))) == 0xffffffffu;
     return Rcp{b, __hiloint2double(__double2hiint(y), ones ? 1 : __double2loint(y))};
   }
-  __device__ __forceinline__ double div(double a, const Rcp &r) {
-    num(a);
+  __device__ __forceinline__ double quotient(double a, const Rcp &r) {
     double q = a * r.y;
     q = fma(-fma(r.b, q, -a), r.y, q);
     return fma(-fma(r.b, q, -a), r.y, q);
+  }
+  __device__ __forceinline__ double div(double a, const Rcp &r) {
+    num(a);
+    return quotient(a, r);
+  }
+  __device__ __forceinline__ double div_pos(double a, double b) {
+    num_pos(a);
+    return quotient(a, rcp(b));
   }
   __device__ __forceinline__ double div(double a, double b) { return div(a, rcp(b)); }
   __device__ __forceinline__ double div_signed(double a, double b) {
@@ -133,7 +152,7 @@ struct Fast64 {
     const double g1 = fma(g0, t, g0), hh = fma(h0, t, h0);
     const double g = fma(fma(-g1, g1, a), hh, g1);
     const double p = __longlong_as_double(__double_as_longlong(g) - 1);
-    return fma(-p, g, a) <= 0.0 ? p : g;
+    return __double2hiint(fma(-p, g, a)) <= 0 ? p : g;  // <= 0 (far above the subnormal range otherwise)
   }
 };
 
@@ -243,9 +262,12 @@ __device__ __forceinline__ void roe_1o(O &o, const T rL, const T uL, const T vL,
                                        const T uR, const T vR, const T pR, const T cR, const T nx, const T ny,
                                        const T dl, bool degenerate, T D[4], const T eflin = T(0.0)) {
   D[0] = D[1] = D[2] = D[3] = T(0.0);
-  if (O::fast) {  // the special cases are left to the caller's second evaluation
-    if (degenerate || rL <= T(0.0) || pL <= T(0.0) || cL <= T(0.0) || rR <= T(0.0) || pR <= T(0.0) || cR <= T(0.0))
-      o.flag();
+  if (O::fast) {  // the special cases are left to the caller's second evaluation (root() flags the densities)
+    if (degenerate) o.flag();
+    o.need_positive(pL);
+    o.need_positive(cL);
+    o.need_positive(pR);
+    o.need_positive(cR);
   } else {
     if (degenerate) return;
     if (rL <= T(0.0) || pL <= T(0.0) || cL <= T(0.0)) return;
@@ -264,7 +286,7 @@ __device__ __forceinline__ void roe_1o(O &o, const T rL, const T uL, const T vL,
   T RVm = T(0.5) * (Ru * Ru + Rv * Rv);
   T Ra = o.root(T(kGM1) * (RH - RVm));
   if (O::fast) {
-    if (Ra <= T(0.0)) o.flag();
+    o.need_positive(Ra);
   } else if (Ra <= T(0.0)) {
     Ra = T(0.5) * (cL + cR);
     if (Ra <= T(0.0)) return;
@@ -570,15 +592,19 @@ __device__ __forceinline__ T muscl_slope(int kind, T a, T b) {
   }
 }
 
-// muscl_slope of a Fast64 evaluation: the Van Leer and van Albada quotients without branches (where the
-// slope is zero the quotient is 0 / 1), the others as they are.
+// Half of muscl_slope of a Fast64 evaluation: the Van Leer and van Albada quotients without branches (where
+// the slope is zero the quotient is 0 / 1), the others as they are.  Halving Van Leer's 2ab / (a + b)
+// cancels its 2: both are exact.  ab > 0 is read off its high word (products below 2^-1042 count as 0).
 template <int KIND>
-__device__ __forceinline__ double muscl_slope_fast(Fast64 &o, double a, double b) {
-  const double ab = a * b;
-  const bool on = !(fabs(b) < 1e-12) && !(ab <= 0.0);
-  if (KIND == LIM_VANLEER) return o.div(on ? 2.0 * ab : 0.0, on ? a + b : 1.0);
-  const double a2 = a * a;
-  return o.div(on ? b * (a2 + ab) : 0.0, on ? a2 + b * b : 1.0);
+__device__ __forceinline__ double muscl_half_slope(Fast64 &o, double a, double b) {
+  if (KIND == LIM_VANLEER || KIND == LIM_VANALBADA) {
+    const double ab = a * b;
+    const bool on = !(fabs(b) < 1e-12) && __double2hiint(ab) > 0;
+    if (KIND == LIM_VANLEER) return o.div_pos(on ? ab : 0.0, on ? a + b : 1.0);
+    const double a2 = a * a;
+    return 0.5 * o.div(on ? b * (a2 + ab) : 0.0, on ? a2 + b * b : 1.0);
+  }
+  return 0.5 * muscl_slope<double>(KIND, a, b);
 }
 
 // Limited slopes of the four conserved or primitive variables on the reference's directional stencil
@@ -674,9 +700,11 @@ __device__ __forceinline__ void hllc_face(O &o, const T qL[5], const T UL[4], co
   F[0] = F[1] = F[2] = F[3] = T(0.0);
   const T normal_mag = o.root(nx * nx + ny * ny);
   if (O::fast) {  // the special cases are left to the caller's second evaluation
-    if (normal_mag < T(1e-14) || qL[0] <= T(0.0) || qL[3] <= T(0.0) || qL[4] <= T(0.0) || qR[0] <= T(0.0) ||
-        qR[3] <= T(0.0) || qR[4] <= T(0.0))
-      o.flag();
+    if (normal_mag < T(1e-14)) o.flag();
+    o.need_positive(qL[3]);
+    o.need_positive(qL[4]);
+    o.need_positive(qR[3]);
+    o.need_positive(qR[4]);
   } else {
     if (normal_mag < T(1e-14)) return;
     if (qL[0] <= T(0.0) || qL[3] <= T(0.0) || qL[4] <= T(0.0)) return;
