@@ -360,6 +360,9 @@ struct cfd_ctx {
   double *pbuf[2] = {nullptr, nullptr};  // stage primitives of the patch form ([5][NT] each)
   cudaGraphExec_t graph = nullptr;
   int graph_launches = 0;
+  // The pseudo-step whose unreadable outputs are left out (every step but a call's last one).
+  cudaGraphExec_t lean_graph = nullptr;
+  int lean_graph_launches = 0;
   // Persistent batched form (option "persistent"): one cooperative launch per RK stage, one
   // CUDA graph per stage; persist_grid = co-resident blocks used; persist_test_arrivals = barrier
   // arrivals that never come (option "barrier_timeout_test", a test of the timeout path).
@@ -480,6 +483,8 @@ int stage_lts(const StagePlan &p, const cfd_config &c, int k) {
 void drop_graphs(cfd_ctx *ctx) {
   if (ctx->graph) cudaGraphExecDestroy(ctx->graph);
   ctx->graph = nullptr;
+  if (ctx->lean_graph) cudaGraphExecDestroy(ctx->lean_graph);
+  ctx->lean_graph = nullptr;
   for (int k = 0; k < 4; k++) {
     if (ctx->stage_graph[k]) cudaGraphExecDestroy(ctx->stage_graph[k]);
     ctx->stage_graph[k] = nullptr;
@@ -491,7 +496,9 @@ void drop_graphs(cfd_ctx *ctx) {
 // boundary conditions, the residual (face-based forms: gradients, face fluxes, gather) and the
 // update.  ghosts_written carries "the previous stage's owner threads wrote this stage's ghosts"
 // from stage to stage (false before stage 0).
-int enqueue_stage(cfd_ctx *ctx, int k, bool fuse_final, bool &ghosts_written) {
+// full: the step's outputs can be read after it; false (a step that another one of the same call
+// follows): the residual, the primitive planes, del_t's last evaluation and the norms are left out.
+int enqueue_stage(cfd_ctx *ctx, int k, bool fuse_final, bool full, bool &ghosts_written) {
   const cfd_config &c = ctx->cfg;
   cudaStream_t s = ctx->stream;
   DevMesh &m = ctx->dm;
@@ -562,7 +569,9 @@ int enqueue_stage(cfd_ctx *ctx, int k, bool fuse_final, bool &ghosts_written) {
     const bool fused = ctx->fuse_gather && (lts == 1 || lts == 2);
     // del_t is formed where a stage uses it (lts 1, or the first stage, which freezes it) and
     // at the last stage, whose value is the Cells[].del_t a download returns.
-    const bool with_dt = fused && (lts == 1 || k == 0 || k == p.n - 1);
+    // Lean stages need every stage fused with a frozen dt, and ghosts that the gradient pass can form.
+    const bool lean = fused && fuse_final && p.lts_mode == 1 && ctx->ghost_private && (k < p.n - 1 || !full);
+    const bool with_dt = fused && (lts == 1 || k == 0 || (k == p.n - 1 && full));
     if (fused && ctx->persistent && ctx->persist_grid > 0) {
       TimedScope ts(ctx, TK_PERSIST);
       const bool bc_next = k < p.n - 1;
@@ -581,7 +590,8 @@ int enqueue_stage(cfd_ctx *ctx, int k, bool fuse_final, bool &ghosts_written) {
       TimedScope ts(ctx, TK_GATHER_STAGE);
       const bool bc_next = k < p.n - 1;
       const int flags = (bc_next ? 2 : 0) | (p.src_S ? 4 : 0);
-      n += launch_gather_stage(s, m, st, ctx->fp, ctx->bp, kind, lts, fin, ctx->keep_delu, flags);
+      if (lean) n += launch_gather_lean(s, m, st, ctx->bp, kind, flags, k == p.n - 2 && full);
+      else n += launch_gather_stage(s, m, st, ctx->fp, ctx->bp, kind, lts, fin, ctx->keep_delu, flags);
       ghosts_written = bc_next;
     } else {
       { TimedScope ts(ctx, TK_FLUX); n += launch_gather(s, m, st, ctx->fp); }
@@ -595,11 +605,11 @@ int enqueue_stage(cfd_ctx *ctx, int k, bool fuse_final, bool &ghosts_written) {
 }
 
 // Launch sequence of one pseudo-step: its stages in order.
-int enqueue_step(cfd_ctx *ctx, bool fuse_final) {
+int enqueue_step(cfd_ctx *ctx, bool fuse_final, bool full = true) {
   const StagePlan p = stage_plan(ctx->cfg, ctx->fp.consistent);
   bool ghosts_written = false;
   int n = 0;
-  for (int k = 0; k < p.n; k++) n += enqueue_stage(ctx, k, fuse_final, ghosts_written);
+  for (int k = 0; k < p.n; k++) n += enqueue_stage(ctx, k, fuse_final, full, ghosts_written);
   return n;
 }
 
@@ -1216,6 +1226,17 @@ cfd_status cfd_create(const cfd_mesh_desc *d, const cfd_config *cfg, cfd_ctx **o
   }
 
   m.wave_blocks = gather_stage_wave_blocks();
+  m.lean_blocks = gather_lean_wave_blocks();
+  if (m.NF > 0) {
+    std::vector<uint8_t> nfb(NP);
+    for (int i = 0; i < NP; i++) nfb[i] = static_cast<uint8_t>(nf[i] | (bptr[i + 1] > bptr[i] ? kHasEntries : 0));
+    if ((s = ctx_upload(ctx, const_cast<uint8_t **>(&m.nfb), nfb)) != CFD_OK) return bail(s);
+    double2 *gw = nullptr;
+    if ((s = ctx_alloc(ctx, (void **)&gw, 4 * (size_t)NP * sizeof(double2))) != CFD_OK) return bail(s);
+    launch_face_weights(ctx->stream, m, gw);
+    if (cudaGetLastError() != cudaSuccess) return bail(fail(CFD_ERR_CUDA, "face weights"));
+    m.gw = gw;
+  }
   if (tile_tables && tile_prepare()) {
     TileMesh &tm = ctx->tm;
     tm.ni = blk.ni;
@@ -1531,7 +1552,7 @@ static cfd_status enqueue_steps_persistent(cfd_ctx *ctx, int n_steps) {
     for (int k = 0; k < p.n && ctx->stage_graphs_ok; k++) {
       cudaGraph_t g;
       CUDA_TRY(cudaStreamBeginCapture(ctx->stream, cudaStreamCaptureModeThreadLocal));
-      ctx->stage_graph_launches[k] = enqueue_stage(ctx, k, true, gw);
+      ctx->stage_graph_launches[k] = enqueue_stage(ctx, k, true, true, gw);
       cudaError_t e = cudaStreamEndCapture(ctx->stream, &g);
       if (e == cudaSuccess) {
         e = cudaGraphInstantiate(&ctx->stage_graph[k], g, 0);
@@ -1613,23 +1634,30 @@ static cfd_status enqueue_steps(cfd_ctx *ctx, int n_steps) {
   if (ctx->dm.cblk && ctx->steps.blocks > 0 && ctx->persist_test_arrivals == 0 && one_launch_form(ctx))
     return enqueue_steps_one_launch(ctx, n_steps, true);
   if (ctx->persistent && ctx->persist_grid > 0 && ctx->dm.NF > 0) return enqueue_steps_persistent(ctx, n_steps);
+  // Every step but the last leaves out what the next one overwrites, unless a t_end may make any the last.
+  const int lean = ctx->t_end_set ? 0 : n_steps - 1;
   if (ctx->use_graph && !ctx->profile && n_steps > 1) {
-    if (!ctx->graph) {
+    auto capture = [&](bool full, cudaGraphExec_t *exec, int *launches) -> cfd_status {
+      if (*exec) return CFD_OK;
       cudaGraph_t g;
       CUDA_TRY(cudaStreamBeginCapture(ctx->stream, cudaStreamCaptureModeThreadLocal));
-      ctx->graph_launches = enqueue_step(ctx, true);
+      *launches = enqueue_step(ctx, true, full);
       cudaError_t e = cudaStreamEndCapture(ctx->stream, &g);
       if (e != cudaSuccess) return fail(CFD_ERR_CUDA, std::string("graph capture: ") + cudaGetErrorString(e));
-      e = cudaGraphInstantiate(&ctx->graph, g, 0);
+      e = cudaGraphInstantiate(exec, g, 0);
       cudaGraphDestroy(g);
       if (e != cudaSuccess) return fail(CFD_ERR_CUDA, std::string("graph instantiate: ") + cudaGetErrorString(e));
-    }
+      return CFD_OK;
+    };
+    cfd_status s;
+    if ((s = capture(true, &ctx->graph, &ctx->graph_launches)) != CFD_OK) return s;
+    if (lean > 0 && (s = capture(false, &ctx->lean_graph, &ctx->lean_graph_launches)) != CFD_OK) return s;
     for (int i = 0; i < n_steps; i++) {
-      CUDA_TRY(cudaGraphLaunch(ctx->graph, ctx->stream));
-      ctx->launches += ctx->graph_launches;
+      CUDA_TRY(cudaGraphLaunch(i < lean ? ctx->lean_graph : ctx->graph, ctx->stream));
+      ctx->launches += i < lean ? ctx->lean_graph_launches : ctx->graph_launches;
     }
   } else {
-    for (int i = 0; i < n_steps; i++) ctx->launches += enqueue_step(ctx, true);
+    for (int i = 0; i < n_steps; i++) ctx->launches += enqueue_step(ctx, true, i >= lean);
   }
   CUDA_TRY(cudaGetLastError());
   ctx->prim_from_S = false;

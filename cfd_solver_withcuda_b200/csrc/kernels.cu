@@ -494,6 +494,16 @@ __device__ __forceinline__ void bc_entry(const DevMesh &m, const DevState &st, c
     store_ghost(st, NT, b.w, G);
 }
 
+// The same from the cell's (rho, u, v, p) row: between pseudo-steps whose primitive planes are not stored
+// only the sound speed's plane is current.
+__device__ __forceinline__ void bc_entry_row(const DevMesh &m, const DevState &st, const BcParams &bp, int e,
+                                             const double4 q) {
+  const int4 b = m.bnd[e];
+  const BcGlobal src{m, st, b.y, b.z, e, 0, 0, m.bstate, m.bexit};
+  double G[4];
+  if (bc_values(src, bp, b.x, q.x, q.y, q.z, q.w, G)) store_ghost(st, m.NT, b.w, G);
+}
+
 __global__ void k_bc(DevMesh m, DevState st, BcParams bp, int src_is_S, int cur_is_S) {
   pdl_enter();
   const int e = item_index(m.bblk, m.NB);
@@ -1570,6 +1580,104 @@ __global__ void __launch_bounds__(kFluxBlock, 6) k_gather_stage(DevMesh m, DevSt
   if (fuse_final && final_kind(kind)) stage_final_reduce(st, e, dtu);
 }
 
+// Values a boundary state is formed from right after the cell's update: the state in registers.
+struct BcRegs {
+  const DevMesh &m;
+  int c, f, e;
+  double av;
+  const double *W, *X;  // current state, exit-copy source
+  const double4 *bstate;
+  const double *bexit;
+  __device__ __forceinline__ double nx() const { return m.nx[f * m.NP + c]; }
+  __device__ __forceinline__ double ny() const { return m.ny[f * m.NP + c]; }
+  __device__ __forceinline__ double a() const { return av; }
+  __device__ __forceinline__ double cur(int k) const { return W[k]; }
+  __device__ __forceinline__ double src(int k) const { return X[k]; }
+};
+
+// k_gather_stage for the stages whose residual, primitive planes and norms nobody can read before they
+// are formed again: every stage but the last, and the last stage of every pseudo-step but the last of a
+// call without t_end.  It leaves out those stores (R 32 bytes, three or four primitive planes of 8, dU)
+// and, in the last stage, all of the reduction but the step's Min_dt; the rows q4, the states, the frozen
+// dt, the sound speed (where the next gradient pass forms del_t) and the ghosts stay.  Bound by its
+// memory traffic: 204 - 236 bytes per cell and the fluxes.
+// MODE 0: not the last stage; 1: the last stage (one wave of blocks strides over the cells when there are
+// no work lists).
+template <int MODE>
+__global__ void __launch_bounds__(kFluxBlock, 7) k_gather_lean(DevMesh m, DevState st, BcParams bp, int kind, int flags,
+                                                              int store_a) {
+  pdl_enter();
+  const int NP = m.NP, NT = m.NT;
+  if (step_done(st.ctl)) return;
+  double dtu = 1e308 * 10.0;
+  const int step = (MODE == 1 && !m.cblk) ? gridDim.x * blockDim.x : NP;
+  for (int c = item_index(m.cblk, NP); c < NP; c += step) {
+    const int info = m.nfb[c];
+    const int4 e4 = m.cface4[c];
+    const double4 F0 = st.F[face_id(e4.x)], F1 = st.F[face_id(e4.y)], F2 = st.F[face_id(e4.z)], F3 = st.F[face_id(e4.w)];
+    StageIn in;
+    load_stage_in(m, st, c, kind, in);
+    const bool first = first_kind(kind);
+    const double dt = first ? st.dtc[c] : st.dtk[c];
+    double R[4], out[4];
+    sum_faces(info & 7, e4, F0, F1, F2, F3, R);
+    const bool fin = stage_values(m, st, c, kind, dt, R, in.Un, in, out);
+    if (first) st.dtk[c] = dt;
+    if (MODE == 1 && fin && !direct_kind(kind)) {
+#pragma unroll
+      for (int k = 0; k < 4; k++) out[k] = in.Un[k] + out[k];
+    }
+#pragma unroll
+    for (int k = 0; k < 4; k++) {
+      if (MODE == 1) st.U[(size_t)k * NT + c] = out[k];
+      else st.S[(size_t)k * NP + c] = out[k];
+    }
+    Prim q;
+    const bool ok = eos_prim(out[0], out[1], out[2], out[3], q);
+    st32(st.q4 + c, make_double4(q.rho, q.u, q.v, q.p));
+    if (MODE == 1 || store_a) st.prim[4 * (size_t)NT + c] = q.a;
+    if (!ok) flag_bad(st.status, c);
+    if (MODE == 0 && (info & kHasEntries)) {
+      const int b0 = m.bptr[c], b1 = m.bptr[c + 1];
+      for (int i = b0; i < b1; i++) {
+        const int e = m.bidx[i];
+        const int4 b = m.bnd[e];
+        const BcRegs src{m, c, b.z, e, q.a, out, (flags & 4) ? out : in.Un, m.bstate, m.bexit};
+        double G[4];
+        if (bc_values(src, bp, b.x, q.rho, q.u, q.v, q.p, G)) store_ghost(st, NT, b.w, G);
+      }
+    }
+    if (MODE == 1) dtu = dt < dtu ? dt : dtu;
+  }
+  if (MODE == 1) {
+    __shared__ double sh[32];
+    const double bm = block_min(dtu, sh);
+    if (threadIdx.x == 0) st.partial[blockIdx.x] = bm;
+    if (last_block(st.counter)) {
+      double v = 1e308 * 10.0;
+#pragma unroll 8
+      for (int i = threadIdx.x; i < (int)gridDim.x; i += kFluxBlock) {
+        const double w = __ldcg(&st.partial[i]);
+        v = w < v ? w : v;
+      }
+      v = block_min(v, sh);
+      if (threadIdx.x == 0) {
+        st.ctl[CTL_DTMIN] = v;
+        st.ctl[CTL_DTSTEP] = v;
+        st.ctl[CTL_TOTAL_TIME] += v;
+        st.ctl[CTL_ITER] += 1.0;
+        *st.counter = 0u;
+      }
+    }
+  }
+}
+
+// Weights of the gradient passes: (nx dl, ny dl) of every face slot.
+__global__ void k_face_weights(DevMesh m, double2 *gw) {
+  const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (i < 4 * (size_t)m.NP) gw[i] = make_double2(m.nx[i] * m.dl[i], m.ny[i] * m.dl[i]);
+}
+
 // Estimate_Error alone (src/Error_Estimate_Update.cpp:10-28).
 __global__ void __launch_bounds__(kBlock) k_error(DevMesh m, DevState st) {
   const int NP = m.NP, NT = m.NT;
@@ -1689,6 +1797,36 @@ __device__ __forceinline__ void cell_gradients(const DevMesh &m, const double *p
   for (int k = 0; k < 8; k++) g[k] = g[k] * ia;
 }
 
+// The gradients alone, from the faces' weights (nx dl, ny dl; the products cell_gradients forms, made once
+// with the context): 64 bytes of geometry per cell instead of 96.
+__device__ __forceinline__ void cell_gradients_w(const DevMesh &m, const double4 *q4, int c, const double qc[4],
+                                                 double g[8]) {
+  const int NP = m.NP, NT = m.NT;
+  const int nf = m.nfb[c] & 7;
+  const int4 n4 = m.nbr4[c];
+  const double ia = m.inv_area[c];
+  const int nr[4] = {n4.x, n4.y, n4.z, n4.w};
+  double4 v[4];
+#pragma unroll
+  for (int f = 0; f < 4; f++) v[f] = ld32_ordered(q4 + ((nr[f] >= 0 && nr[f] < NT) ? nr[f] : c));
+#pragma unroll
+  for (int k = 0; k < 8; k++) g[k] = 0.0;
+#pragma unroll
+  for (int f = 0; f < 4; f++) {
+    if (f >= nf) break;
+    const double2 w = m.gw[(size_t)f * NP + c];
+    const double qn[4] = {v[f].x, v[f].y, v[f].z, v[f].w};
+#pragma unroll
+    for (int k = 0; k < 4; k++) {
+      const double qf = 0.5 * (qc[k] + qn[k]);
+      g[2 * k] += qf * w.x;
+      g[2 * k + 1] += qf * w.y;
+    }
+  }
+#pragma unroll
+  for (int k = 0; k < 8; k++) g[k] = g[k] * ia;
+}
+
 // Gradient records of the face-based forms: the Green-Gauss gradients of (rho, u, v, p) of every
 // physical cell, the face value being the mean of the two cell values (a ghost neighbour's value
 // carries the boundary state); the states themselves are read from q4.  Work-list entries cover
@@ -1703,17 +1841,19 @@ __global__ void __launch_bounds__(kBlock, 4) k_muscl_gradients(DevMesh m, DevSta
                                                                int with_bc) {
   pdl_enter();
   const int c = item_index(m.rblk, m.NT);
-  const int NP = m.NP, NT = m.NT;
+  const int NP = m.NP;
   if (step_done(st.ctl)) return;
   if (c < NP) {
-    if (with_bc) {
+    if (with_bc && (m.nfb[c] & kHasEntries)) {
+      const double4 q = ld32_ordered(st.q4 + c);
       const int b0 = m.bptr[c], b1 = m.bptr[c + 1];
-      for (int i = b0; i < b1; i++) bc_entry(m, st, bp, m.bidx[i], 0, 0);
+      for (int i = b0; i < b1; i++) bc_entry_row(m, st, bp, m.bidx[i], q);
     }
     const double4 v = ld32_ordered(st.q4 + c);
     const double qc[4] = {v.x, v.y, v.z, v.w};
     double g[8], den;
-    cell_gradients<DT, true>(m, st.prim, st.q4, c, qc, g, den);
+    if (DT) cell_gradients<true, true>(m, st.prim, st.q4, c, qc, g, den);
+    else cell_gradients_w(m, st.q4, c, qc, g);
     if (st.recf) {
       st32f(st.recf + 2 * (size_t)c, g);
     } else {
@@ -1723,7 +1863,6 @@ __global__ void __launch_bounds__(kBlock, 4) k_muscl_gradients(DevMesh m, DevSta
     }
     if (DT) st.dtc[c] = cell_dt(m, fp, c, den);
   }
-  (void)NT;
 }
 
 // ---- Persistent form of one stage for batched solves (no reference counterpart) ----
@@ -3414,6 +3553,8 @@ int launch_faces(cudaStream_t s, const DevMesh &m, DevState &st, const FluxParam
   return 1;
 }
 
+int device_sms();
+
 int gather_stage_wave_blocks() {
   int dev = 0, sms = 0, per_sm = 0;
   if (cudaGetDevice(&dev) != cudaSuccess) return 0;
@@ -3431,6 +3572,31 @@ int launch_gather_stage(cudaStream_t s, const DevMesh &m, DevState &st, const Fl
              flags);
   else
     launch_k(m, k_gather_stage<false>, g, kFluxBlock, s, m, st, fp, bp, kind, lts, fuse_final, keep_delu, flags);
+  return 1;
+}
+
+// stage: 0 not the last, 1 the last.
+int launch_gather_lean(cudaStream_t s, const DevMesh &m, const DevState &st, const BcParams &bp, int kind, int flags,
+                       int store_a) {
+  const int g = m.cblk ? m.n_cblk : nblk(m.NP, kFluxBlock);
+  if (g == 0) return 0;
+  if (final_kind(kind))
+    launch_k(m, k_gather_lean<1>, !m.cblk && m.lean_blocks > 0 ? std::min(g, m.lean_blocks) : g, kFluxBlock, s, m, st, bp,
+             kind, flags, store_a);
+  else launch_k(m, k_gather_lean<0>, g, kFluxBlock, s, m, st, bp, kind, flags, store_a);
+  return 1;
+}
+
+int gather_lean_wave_blocks() {
+  int per_sm = 0;
+  const int sms = device_sms();
+  if (sms <= 0 || cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_gather_lean<1>, kFluxBlock, 0) != cudaSuccess)
+    return 0;
+  return sms * per_sm;
+}
+
+int launch_face_weights(cudaStream_t s, const DevMesh &m, double2 *gw) {
+  k_face_weights<<<(unsigned)((4 * (size_t)m.NP + kBlock - 1) / kBlock), kBlock, 0, s>>>(m, gw);
   return 1;
 }
 

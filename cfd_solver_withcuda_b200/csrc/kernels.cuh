@@ -73,6 +73,9 @@ struct DevMesh {
   // Blocks of k_gather_stage resident on the whole device at once (SMs x blocks per SM): the grid
   // of its reducing stage (0 = one block per 128 cells).
   int wave_blocks;
+  int lean_blocks;      // the same for k_gather_lean's last stage
+  const uint8_t *nfb;   // [NP] face count, kHasEntries when the cell has boundary entries
+  const double2 *gw;    // [4][NP] nx dl, ny dl (face-based forms)
   // L2 access-policy window given to every launch (null / 0: none): the (rho, u, v, p) rows and the
   // face-flux array that follows them, kept as persisting lines between the kernels of a stage.
   void *l2_base;
@@ -83,6 +86,7 @@ struct DevMesh {
 };
 
 constexpr int kPatchCells = 128;
+constexpr int kHasEntries = 128;  // bit of DevMesh::nfb
 
 constexpr int kWorkCellBlock = 128;
 constexpr int kMaxGroups = 256;  // block groups of the two-level grid reductions
@@ -237,6 +241,12 @@ int launch_gather(cudaStream_t s, const DevMesh &m, DevState &st, const FluxPara
 // next stage (non-final stages), bit 2 that next stage's supersonic-exit copy reads the stage state.
 int launch_gather_stage(cudaStream_t s, const DevMesh &m, DevState &st, const FluxParams &fp, const BcParams &bp,
                         int kind, int lts, int fuse_final, int keep_delu, int flags);
+// The same without the outputs that are formed again before anyone can read them (see k_gather_lean);
+// lts 2 forms only.  store_a: the next stage's gradient pass forms del_t.
+int launch_gather_lean(cudaStream_t s, const DevMesh &m, const DevState &st, const BcParams &bp, int kind, int flags,
+                       int store_a);
+int gather_lean_wave_blocks();
+int launch_face_weights(cudaStream_t s, const DevMesh &m, double2 *gw);
 // Patch form of one stage (gradients, face fluxes, gather and stage update in one kernel): reads
 // the primitives `prim_in` and writes the stage's primitives and ghosts to st.prim, which must be a
 // different buffer (blocks read their halo cells' primitives while others write theirs).  Same
