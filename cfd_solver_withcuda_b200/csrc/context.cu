@@ -529,6 +529,8 @@ int enqueue_stage(cfd_ctx *ctx, int k, bool fuse_final, bool full, bool &ghosts_
     n += launch_bc(s, m, st, ctx->bp, k > 0 && p.src_S, k > 0);
   }
   ghosts_written = false;
+  // The stage kernels' owner threads write the next stage's ghosts.
+  const int ghosts = k < p.n - 1 ? kStageGhosts | (p.src_S ? kStageExitS : 0) : 0;
   if (tile) {
     TimedScope ts(ctx, TK_TILE);
     const bool bc_next = k < p.n - 1;
@@ -595,19 +597,30 @@ int enqueue_stage(cfd_ctx *ctx, int k, bool fuse_final, bool full, bool &ghosts_
       ghosts_written = bc_next;
     } else {
       { TimedScope ts(ctx, TK_FLUX); n += launch_gather(s, m, st, ctx->fp); }
-      { TimedScope ts(ctx, TK_STAGE); n += launch_stage(s, m, st, kind, lts, fin, ctx->keep_delu); }
+      { TimedScope ts(ctx, TK_STAGE); n += launch_stage(s, m, st, ctx->bp, kind, lts, fin, ctx->keep_delu, ghosts); }
+      ghosts_written = k < p.n - 1;
     }
     return n;
   }
-  { TimedScope ts(ctx, TK_FLUX); n += launch_flux(s, m, st, ctx->fp, k > 0); }
-  { TimedScope ts(ctx, TK_STAGE); n += launch_stage(s, m, st, kind, lts, fin, ctx->keep_delu); }
+  // Per-cell forms.  Min_dt is formed where a stage, the step's time or a download uses it, del_t likewise.
+  const bool last = k == p.n - 1;
+  int want = 0;
+  if (lts == 0 || k == 0 || (last && full)) want = kWantDt | kWantMin;
+  if (lts == 1 && !(last && full)) want = kWantDt;
+  { TimedScope ts(ctx, TK_FLUX); n += launch_flux(s, m, st, ctx->fp, k > 0, want); }
+  // The last stage of a step that another one follows also writes that step's first ghosts.
+  const int flags = last ? (full || !fuse_final ? 0 : kStageNextStep | kStageNoNorms) : ghosts;
+  {
+    TimedScope ts(ctx, TK_STAGE);
+    n += launch_stage(s, m, st, ctx->bp, kind, lts, fin, last && !full ? 0 : ctx->keep_delu, flags);
+  }
+  ghosts_written = flags != 0;
   return n;
 }
 
-// Launch sequence of one pseudo-step: its stages in order.
-int enqueue_step(cfd_ctx *ctx, bool fuse_final, bool full = true) {
+// Launch sequence of one pseudo-step: its stages in order.  ghosts_written: the first stage's ghosts are there.
+int enqueue_step(cfd_ctx *ctx, bool fuse_final, bool full = true, bool ghosts_written = false) {
   const StagePlan p = stage_plan(ctx->cfg, ctx->fp.consistent);
-  bool ghosts_written = false;
   int n = 0;
   for (int k = 0; k < p.n; k++) n += enqueue_stage(ctx, k, fuse_final, full, ghosts_written);
   return n;
@@ -1386,7 +1399,7 @@ cfd_status cfd_create(const cfd_mesh_desc *d, const cfd_config *cfg, cfd_ctx **o
   fp.limiter = cfg->limiter;
   fp.recon_prim = cfg->reconstruct_primitive;
   fp.muscl = cfg->muscl && cfg->is_second_order;
-  fp.lanes = 1;
+  fp.lanes = flux_lanes_for(NP);
   fp.faces_shape = 3;
   // WENO (Is_WENO): Explicit_Method falls back to the 1O/2O residual when any cell is not a quad
   // (src/Numerical_Method.cpp:31-55); Runge_Kutta_Method keeps WENO (zero flux on those cells).
@@ -1636,12 +1649,18 @@ static cfd_status enqueue_steps(cfd_ctx *ctx, int n_steps) {
   if (ctx->persistent && ctx->persist_grid > 0 && ctx->dm.NF > 0) return enqueue_steps_persistent(ctx, n_steps);
   // Every step but the last leaves out what the next one overwrites, unless a t_end may make any the last.
   const int lean = ctx->t_end_set ? 0 : n_steps - 1;
+  // Per-cell forms: such a step also leaves the next one's ghosts, so only the first needs them formed here.
+  const bool ghosts = ctx->dm.NF == 0;
+  if (lean > 0 && ghosts) {
+    TimedScope ts(ctx, TK_BC);
+    ctx->launches += launch_bc(ctx->stream, ctx->dm, ctx->ds, ctx->bp, 0, 0);
+  }
   if (ctx->use_graph && !ctx->profile && n_steps > 1) {
     auto capture = [&](bool full, cudaGraphExec_t *exec, int *launches) -> cfd_status {
       if (*exec) return CFD_OK;
       cudaGraph_t g;
       CUDA_TRY(cudaStreamBeginCapture(ctx->stream, cudaStreamCaptureModeThreadLocal));
-      *launches = enqueue_step(ctx, true, full);
+      *launches = enqueue_step(ctx, true, full, !full && ghosts);
       cudaError_t e = cudaStreamEndCapture(ctx->stream, &g);
       if (e != cudaSuccess) return fail(CFD_ERR_CUDA, std::string("graph capture: ") + cudaGetErrorString(e));
       e = cudaGraphInstantiate(exec, g, 0);
@@ -1657,7 +1676,7 @@ static cfd_status enqueue_steps(cfd_ctx *ctx, int n_steps) {
       ctx->launches += i < lean ? ctx->lean_graph_launches : ctx->graph_launches;
     }
   } else {
-    for (int i = 0; i < n_steps; i++) ctx->launches += enqueue_step(ctx, true, i >= lean);
+    for (int i = 0; i < n_steps; i++) ctx->launches += enqueue_step(ctx, true, i >= lean, i < lean && ghosts);
   }
   CUDA_TRY(cudaGetLastError());
   ctx->prim_from_S = false;
@@ -1760,7 +1779,7 @@ cfd_status cfd_explicit_method(cfd_ctx *ctx) {
   cfd_status s = sync_status(ctx, nullptr);
   if (s != CFD_OK) return s;
   if (!(ctx->h_ctl[CTL_DTMIN] > 0.0)) return fail(CFD_ERR_DT_NONPOSITIVE, "Min_dt is not positive");
-  ctx->launches += launch_stage(ctx->stream, ctx->dm, ctx->ds, 0, 0, 0, 1);
+  ctx->launches += launch_stage(ctx->stream, ctx->dm, ctx->ds, ctx->bp, 0, 0, 0, 1, 0);
   CUDA_TRY(cudaGetLastError());
   return sync_status(ctx, nullptr);
 }
@@ -1771,9 +1790,9 @@ cfd_status cfd_runge_kutta_method(cfd_ctx *ctx) {
   StagePlan p = stage_plan(c, ctx->fp.consistent);
   if (p.kind0 == 0) p = {3, 1, ctx->fp.consistent, 0};  // the reference's RK3 on an explicit config
   for (int k = 0; k < p.n; k++) {
-    if (k > 0) ctx->launches += launch_bc(ctx->stream, ctx->dm, ctx->ds, ctx->bp, p.src_S, 1);
     ctx->launches += launch_flux(ctx->stream, ctx->dm, ctx->ds, ctx->fp, k > 0);
-    ctx->launches += launch_stage(ctx->stream, ctx->dm, ctx->ds, p.kind0 + k, stage_lts(p, c, k), 0, 1);
+    ctx->launches += launch_stage(ctx->stream, ctx->dm, ctx->ds, ctx->bp, p.kind0 + k, stage_lts(p, c, k), 0, 1,
+                                  k < p.n - 1 ? kStageGhosts | (p.src_S ? kStageExitS : 0) : 0);
   }
   CUDA_TRY(cudaGetLastError());
   ctx->prim_from_S = true;

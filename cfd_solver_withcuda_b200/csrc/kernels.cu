@@ -706,16 +706,20 @@ __device__ __noinline__ double4 face_contrib_again(const DevMesh &m, const DevSt
 
 // Evaluate_Cell_Net_Flux_1O/2O (src/Net_Flux.cpp:46-129) + Evaluate_Time_Step (src/Time_Step.cpp:293-359)
 // fused, one thread per cell: faces in order, Net += avg - diss; then del_t; block min + Min_dt.
-// MINB: minimum resident blocks per SM the register allocation is made for (1: unconstrained;
-// the second-order forms with the directional limiter are also built for 6 and 8 for more resident
-// warps; the autotuner picks, the results are the same bits).  SRC_S false: the conserved states
-// come from U only (the caller knows no stage state is read), which saves the per-load choice
-// between U and the stage state.  The divisions and square roots are the branch-free ones (Fast64),
-// so the four faces' chains interleave; a cell with an operand outside their range is evaluated again.
-template <int DISS, int ORDER, int MINB = 1, bool SRC_S = true>
+// MINB: minimum resident blocks per SM the register allocation is made for (6; the second-order forms
+// with the directional limiter are also built for 8 and unconstrained, the autotuner picks; the results
+// are the same bits).  SRC_S false: the conserved states come from U only (the caller knows no stage
+// state is read), which saves the per-load choice between U and the stage state.  The divisions and
+// square roots are the branch-free ones (Fast64), whose chains interleave within a face, so the face
+// loop is not unrolled: unrolled, the kernels took 124 - 136 registers (12 - 16 warps per SM) and ROE
+// 101 us, ROE_2O 117 us on 524,288 cells, against 73 and 106 us in a loop at 80 (B200).  A cell with an
+// operand outside their range is evaluated again.
+// want (FluxWant bits): del_t is stored, and Min_dt formed, only for evaluations whose value is used.
+template <int DISS, int ORDER, int MINB = 6, bool SRC_S = true>
 __global__ void __launch_bounds__(kFluxBlock, MINB) k_flux(const __grid_constant__ DevMesh m,
                                                            const __grid_constant__ DevState st,
-                                                           const __grid_constant__ FluxParams fp, int src_is_S) {
+                                                           const __grid_constant__ FluxParams fp, int src_is_S,
+                                                           int want) {
   __shared__ double sh[32];
   const int NP = m.NP, NT = m.NT;
   const int c = blockIdx.x * blockDim.x + threadIdx.x;
@@ -730,17 +734,15 @@ __global__ void __launch_bounds__(kFluxBlock, MINB) k_flux(const __grid_constant
     double N0 = 0.0, N1s = 0.0, N2s = 0.0, N3s = 0.0;
     double den = 0.0;
     Fast64 o;
-#pragma unroll
-    for (int f = 0; f < 4; f++) {
-      if (f < nf) {
-        double X[4], t;
-        face_contrib<DISS, ORDER>(o, m, st, fp, us, q, c, f, X, t);
-        N0 += X[0];
-        N1s += X[1];
-        N2s += X[2];
-        N3s += X[3];
-        den += t;
-      }
+#pragma unroll 1
+    for (int f = 0; f < nf; f++) {
+      double X[4], t;
+      face_contrib<DISS, ORDER>(o, m, st, fp, us, q, c, f, X, t);
+      N0 += X[0];
+      N1s += X[1];
+      N2s += X[2];
+      N3s += X[3];
+      den += t;
     }
     if (o.bad()) {
       N0 = N1s = N2s = N3s = 0.0;
@@ -752,14 +754,16 @@ __global__ void __launch_bounds__(kFluxBlock, MINB) k_flux(const __grid_constant
         N3s += X.w;
       }
     }
-    dt = cell_dt(m, fp, c, den);
     st.R[c] = N0;
     st.R[NP + c] = N1s;
     st.R[2 * NP + c] = N2s;
     st.R[3 * NP + c] = N3s;
-    st.dtc[c] = dt;
+    if (want) {
+      dt = cell_dt(m, fp, c, den);
+      st.dtc[c] = dt;
+    }
   }
-  if (done) return;
+  if (done || !(want & kWantMin)) return;
   min_dt_epilogue(st, dt, sh);
 }
 
@@ -770,7 +774,8 @@ __global__ void __launch_bounds__(kFluxBlock, MINB) k_flux(const __grid_constant
 template <int DISS, int ORDER>
 __global__ void __launch_bounds__(kFlux4Block) k_flux4(const __grid_constant__ DevMesh m,
                                                        const __grid_constant__ DevState st,
-                                                       const __grid_constant__ FluxParams fp, int src_is_S) {
+                                                       const __grid_constant__ FluxParams fp, int src_is_S,
+                                                       int want) {
   __shared__ double sh[32];
   const int NP = m.NP, NT = m.NT;
   const int gid = blockIdx.x * blockDim.x + threadIdx.x;
@@ -817,12 +822,14 @@ __global__ void __launch_bounds__(kFlux4Block) k_flux4(const __grid_constant__ D
         den += T[d - 1];
       }
     }
-    dt = cell_dt(m, fp, c, den);
 #pragma unroll
     for (int k = 0; k < 4; k++) st.R[k * NP + c] = R[k];
-    st.dtc[c] = dt;
+    if (want) {
+      dt = cell_dt(m, fp, c, den);
+      st.dtc[c] = dt;
+    }
   }
-  min_dt_epilogue(st, dt, sh);
+  if (want & kWantMin) min_dt_epilogue(st, dt, sh);
 }
 
 // Evaluate_Cell_Net_Flux_WENO, src/WENO2D.cpp:395-456, one thread per cell.  Quad cells only
@@ -1443,8 +1450,12 @@ __device__ __forceinline__ void cell_update(const DevMesh &m, const DevState &st
 
 // lts: 0 Min_dt, 1 Cell::del_t (reference stage 1 only), 2 dt frozen per cell at the first stage,
 // 3 Min_dt frozen at the first stage.
-__global__ void __launch_bounds__(kBlock) k_stage(DevMesh m, DevState st, int kind, int lts, int fuse_final,
-                                                  int keep_delu) {
+// flags (StageFlags): the owner thread writes its ghosts for the next evaluation, with kStageNextStep those
+// of the next pseudo-step's first one; kStageNoNorms leaves the norms out.  Bound by its traffic (168 - 232
+// bytes per cell) and, on small meshes, by the launch: the ghost writes save a k_bc launch per stage (5.5 us
+// on 524,288 cells), the missing norms 10 us of the last stage's 22 there.
+__global__ void __launch_bounds__(kBlock) k_stage(DevMesh m, DevState st, BcParams bp, int kind, int lts,
+                                                  int fuse_final, int keep_delu, int flags) {
   const int NP = m.NP;
   const int c = item_index(m.cblk, NP);
   const bool done = step_done(st.ctl);
@@ -1465,12 +1476,24 @@ __global__ void __launch_bounds__(kBlock) k_stage(DevMesh m, DevState st, int ki
 #pragma unroll
     for (int k = 0; k < 4; k++) Rk[k] = st.R[k * NP + c];
     cell_update(m, st, c, kind, dt, Rk, fuse_final, keep_delu, e);
+    if (flags & (kStageGhosts | kStageNextStep)) {
+      const int b0 = m.bptr[c], b1 = m.bptr[c + 1];
+      const int cur_S = (flags & kStageGhosts) ? 1 : 0;
+      for (int i = b0; i < b1; i++) bc_entry(m, st, bp, m.bidx[i], (cur_S && (flags & kStageExitS)) ? 1 : 0, cur_S);
+    }
   }
   if (first_kind(kind) && blockIdx.x == 0 && threadIdx.x == 0 && !done) st.ctl[CTL_DTSTEP] = dtmin;
   if (fuse_final && final_kind(kind)) {
     if (done) return;
     const double dt_time = (lts >= 2) ? st.ctl[CTL_DTSTEP] : dtmin;
-    reduce_err_and_epilogue(st, e, true, dt_time);
+    if (flags & kStageNoNorms) {  // only without t_end
+      if (blockIdx.x == 0 && threadIdx.x == 0) {
+        st.ctl[CTL_TOTAL_TIME] += dt_time;
+        st.ctl[CTL_ITER] += 1.0;
+      }
+    } else {
+      reduce_err_and_epilogue(st, e, true, dt_time);
+    }
   }
 }
 
@@ -1604,7 +1627,7 @@ struct BcRegs {
 // MODE 0: not the last stage; 1: the last stage (one wave of blocks strides over the cells when there are
 // no work lists).
 template <int MODE>
-__global__ void __launch_bounds__(kFluxBlock, 7) k_gather_lean(DevMesh m, DevState st, BcParams bp, int kind, int flags,
+__global__ void __launch_bounds__(kFluxBlock, 6) k_gather_lean(DevMesh m, DevState st, BcParams bp, int kind, int flags,
                                                               int store_a) {
   pdl_enter();
   const int NP = m.NP, NT = m.NT;
@@ -3434,32 +3457,34 @@ int launch_lax_friedrichs(cudaStream_t s, const DevMesh &m, DevState &st, const 
 // integrators, and the first stage of every form), else the one that picks U or the stage state
 // per cell.  Same bits either way.
 template <int DISS, int ORDER>
-void launch_flux_src(int g, cudaStream_t s, const DevMesh &m, DevState &st, const FluxParams &fp, int src_is_S) {
-  if (fp.consistent && src_is_S) k_flux<DISS, ORDER, 1, true><<<g, kFluxBlock, 0, s>>>(m, st, fp, src_is_S);
-  else k_flux<DISS, ORDER, 1, false><<<g, kFluxBlock, 0, s>>>(m, st, fp, src_is_S);
+void launch_flux_src(int g, cudaStream_t s, const DevMesh &m, DevState &st, const FluxParams &fp, int src_is_S,
+                     int want) {
+  if (fp.consistent && src_is_S) k_flux<DISS, ORDER, 6, true><<<g, kFluxBlock, 0, s>>>(m, st, fp, src_is_S, want);
+  else k_flux<DISS, ORDER, 6, false><<<g, kFluxBlock, 0, s>>>(m, st, fp, src_is_S, want);
 }
 
 // The second-order per-cell forms with the directional limiter (ROE_2O, RICCA_2O, MOVERS_NWSC_2O):
 // one build per register budget (minimum resident blocks of 128 threads per SM: 1 unconstrained,
 // 6 or 8), chosen by fp.flux_minb; every build gives the same bits.
 template <int DISS>
-void launch_flux_limited(int g, cudaStream_t s, const DevMesh &m, DevState &st, const FluxParams &fp, int src_is_S) {
+void launch_flux_limited(int g, cudaStream_t s, const DevMesh &m, DevState &st, const FluxParams &fp, int src_is_S,
+                         int want) {
   if (!(fp.consistent && src_is_S)) {
     switch (fp.flux_minb) {
-      case 6: k_flux<DISS, 2, 6, false><<<g, kFluxBlock, 0, s>>>(m, st, fp, src_is_S); break;
-      case 8: k_flux<DISS, 2, 8, false><<<g, kFluxBlock, 0, s>>>(m, st, fp, src_is_S); break;
-      default: k_flux<DISS, 2, 1, false><<<g, kFluxBlock, 0, s>>>(m, st, fp, src_is_S); break;
+      case 1: k_flux<DISS, 2, 1, false><<<g, kFluxBlock, 0, s>>>(m, st, fp, src_is_S, want); break;
+      case 8: k_flux<DISS, 2, 8, false><<<g, kFluxBlock, 0, s>>>(m, st, fp, src_is_S, want); break;
+      default: k_flux<DISS, 2, 6, false><<<g, kFluxBlock, 0, s>>>(m, st, fp, src_is_S, want); break;
     }
     return;
   }
   switch (fp.flux_minb) {
-    case 6: k_flux<DISS, 2, 6><<<g, kFluxBlock, 0, s>>>(m, st, fp, src_is_S); break;
-    case 8: k_flux<DISS, 2, 8><<<g, kFluxBlock, 0, s>>>(m, st, fp, src_is_S); break;
-    default: k_flux<DISS, 2><<<g, kFluxBlock, 0, s>>>(m, st, fp, src_is_S); break;
+    case 1: k_flux<DISS, 2, 1><<<g, kFluxBlock, 0, s>>>(m, st, fp, src_is_S, want); break;
+    case 8: k_flux<DISS, 2, 8><<<g, kFluxBlock, 0, s>>>(m, st, fp, src_is_S, want); break;
+    default: k_flux<DISS, 2, 6><<<g, kFluxBlock, 0, s>>>(m, st, fp, src_is_S, want); break;
   }
 }
 
-int launch_flux(cudaStream_t s, const DevMesh &m, DevState &st, const FluxParams &fp, int src_is_S) {
+int launch_flux(cudaStream_t s, const DevMesh &m, DevState &st, const FluxParams &fp, int src_is_S, int want) {
   int n = 0;
   if (fp.second_order && fp.muscl) n += launch_muscl_gradients(s, m, st, fp, 0);
   if (fp.second_order && fp.muscl && m.NF > 0) {
@@ -3474,37 +3499,38 @@ int launch_flux(cudaStream_t s, const DevMesh &m, DevState &st, const FluxParams
   }
   if (fp.lanes == 1) {
     const int g = nblk(m.NP, kFluxBlock);
-    if (fp.dissipation == 3 && !fp.second_order) k_flux<3, 1><<<g, kFluxBlock, 0, s>>>(m, st, fp, src_is_S);
-    else if (fp.dissipation == 2 && !fp.second_order) launch_flux_src<2, 1>(g, s, m, st, fp, src_is_S);
-    else if (fp.dissipation == 2) launch_flux_src<2, 2>(g, s, m, st, fp, src_is_S);
-    else if (fp.dissipation == 4 && !fp.second_order) k_flux<4, 1><<<g, kFluxBlock, 0, s>>>(m, st, fp, src_is_S);
-    else if (fp.dissipation == 5 && !fp.second_order) launch_flux_src<5, 1>(g, s, m, st, fp, src_is_S);
-    else if (fp.dissipation == 6) launch_flux_src<6, 1>(g, s, m, st, fp, src_is_S);
-    else if (fp.dissipation == 7) launch_flux_src<7, 1>(g, s, m, st, fp, src_is_S);
-    else if (fp.dissipation == 3) launch_flux_limited<3>(g, s, m, st, fp, src_is_S);
-    else if (fp.dissipation == 4) launch_flux_limited<4>(g, s, m, st, fp, src_is_S);
-    else if (fp.dissipation == 5) launch_flux_limited<5>(g, s, m, st, fp, src_is_S);
-    else launch_flux_src<1, 1>(g, s, m, st, fp, src_is_S);
+    if (fp.dissipation == 3 && !fp.second_order) k_flux<3, 1><<<g, kFluxBlock, 0, s>>>(m, st, fp, src_is_S, want);
+    else if (fp.dissipation == 2 && !fp.second_order) launch_flux_src<2, 1>(g, s, m, st, fp, src_is_S, want);
+    else if (fp.dissipation == 2) launch_flux_src<2, 2>(g, s, m, st, fp, src_is_S, want);
+    else if (fp.dissipation == 4 && !fp.second_order) k_flux<4, 1><<<g, kFluxBlock, 0, s>>>(m, st, fp, src_is_S, want);
+    else if (fp.dissipation == 5 && !fp.second_order) launch_flux_src<5, 1>(g, s, m, st, fp, src_is_S, want);
+    else if (fp.dissipation == 6) launch_flux_src<6, 1>(g, s, m, st, fp, src_is_S, want);
+    else if (fp.dissipation == 7) launch_flux_src<7, 1>(g, s, m, st, fp, src_is_S, want);
+    else if (fp.dissipation == 3) launch_flux_limited<3>(g, s, m, st, fp, src_is_S, want);
+    else if (fp.dissipation == 4) launch_flux_limited<4>(g, s, m, st, fp, src_is_S, want);
+    else if (fp.dissipation == 5) launch_flux_limited<5>(g, s, m, st, fp, src_is_S, want);
+    else launch_flux_src<1, 1>(g, s, m, st, fp, src_is_S, want);
   } else {
     const int g = nblk(4 * m.NP, kFlux4Block);
-    if (fp.dissipation == 3 && !fp.second_order) k_flux4<3, 1><<<g, kFlux4Block, 0, s>>>(m, st, fp, src_is_S);
-    else if (fp.dissipation == 2 && !fp.second_order) k_flux4<2, 1><<<g, kFlux4Block, 0, s>>>(m, st, fp, src_is_S);
-    else if (fp.dissipation == 2) k_flux4<2, 2><<<g, kFlux4Block, 0, s>>>(m, st, fp, src_is_S);
-    else if (fp.dissipation == 4 && !fp.second_order) k_flux4<4, 1><<<g, kFlux4Block, 0, s>>>(m, st, fp, src_is_S);
-    else if (fp.dissipation == 4) k_flux4<4, 2><<<g, kFlux4Block, 0, s>>>(m, st, fp, src_is_S);
-    else if (fp.dissipation == 5 && !fp.second_order) k_flux4<5, 1><<<g, kFlux4Block, 0, s>>>(m, st, fp, src_is_S);
-    else if (fp.dissipation == 5) k_flux4<5, 2><<<g, kFlux4Block, 0, s>>>(m, st, fp, src_is_S);
-    else if (fp.dissipation == 6) k_flux4<6, 1><<<g, kFlux4Block, 0, s>>>(m, st, fp, src_is_S);
-    else if (fp.dissipation == 7) k_flux4<7, 1><<<g, kFlux4Block, 0, s>>>(m, st, fp, src_is_S);
-    else if (fp.dissipation == 3) k_flux4<3, 2><<<g, kFlux4Block, 0, s>>>(m, st, fp, src_is_S);
-    else k_flux4<1, 1><<<g, kFlux4Block, 0, s>>>(m, st, fp, src_is_S);
+    if (fp.dissipation == 3 && !fp.second_order) k_flux4<3, 1><<<g, kFlux4Block, 0, s>>>(m, st, fp, src_is_S, want);
+    else if (fp.dissipation == 2 && !fp.second_order) k_flux4<2, 1><<<g, kFlux4Block, 0, s>>>(m, st, fp, src_is_S, want);
+    else if (fp.dissipation == 2) k_flux4<2, 2><<<g, kFlux4Block, 0, s>>>(m, st, fp, src_is_S, want);
+    else if (fp.dissipation == 4 && !fp.second_order) k_flux4<4, 1><<<g, kFlux4Block, 0, s>>>(m, st, fp, src_is_S, want);
+    else if (fp.dissipation == 4) k_flux4<4, 2><<<g, kFlux4Block, 0, s>>>(m, st, fp, src_is_S, want);
+    else if (fp.dissipation == 5 && !fp.second_order) k_flux4<5, 1><<<g, kFlux4Block, 0, s>>>(m, st, fp, src_is_S, want);
+    else if (fp.dissipation == 5) k_flux4<5, 2><<<g, kFlux4Block, 0, s>>>(m, st, fp, src_is_S, want);
+    else if (fp.dissipation == 6) k_flux4<6, 1><<<g, kFlux4Block, 0, s>>>(m, st, fp, src_is_S, want);
+    else if (fp.dissipation == 7) k_flux4<7, 1><<<g, kFlux4Block, 0, s>>>(m, st, fp, src_is_S, want);
+    else if (fp.dissipation == 3) k_flux4<3, 2><<<g, kFlux4Block, 0, s>>>(m, st, fp, src_is_S, want);
+    else k_flux4<1, 1><<<g, kFlux4Block, 0, s>>>(m, st, fp, src_is_S, want);
   }
   return n + 1;
 }
 
-int launch_stage(cudaStream_t s, const DevMesh &m, DevState &st, int kind, int lts, int fuse_final, int keep_delu) {
-  if (m.cblk) k_stage<<<m.n_cblk, kWorkCellBlock, 0, s>>>(m, st, kind, lts, fuse_final, keep_delu);
-  else k_stage<<<nblk(m.NP, kBlock), kBlock, 0, s>>>(m, st, kind, lts, fuse_final, keep_delu);
+int launch_stage(cudaStream_t s, const DevMesh &m, DevState &st, const BcParams &bp, int kind, int lts, int fuse_final,
+                 int keep_delu, int flags) {
+  if (m.cblk) k_stage<<<m.n_cblk, kWorkCellBlock, 0, s>>>(m, st, bp, kind, lts, fuse_final, keep_delu, flags);
+  else k_stage<<<nblk(m.NP, kBlock), kBlock, 0, s>>>(m, st, bp, kind, lts, fuse_final, keep_delu, flags);
   return 1;
 }
 
@@ -3886,6 +3912,13 @@ int device_sms() {
     return 0;
   return sms;
 }
+
+// Threads per cell of the per-cell flux kernel: four while they fit five blocks of 128 per SM, so that a
+// small mesh still fills the chip and the four faces' chains run side by side.  Per pseudo-step of three
+// stages (four lanes against one, LLF / ROE / ROE_2O / HLLC, B200): 27 / 29 / 29 / 30 us against
+// 34 / 40 / 46 / 36 at 3,200 cells, 33 / 36 / 44 / 38 against 36 / 42 / 48 / 38 at 20,000,
+// 47 / 52 / 62 / 52 against 37 / 48 / 56 / 44 at 45,451.
+int flux_lanes_for(int cells) { return 4LL * cells <= 640LL * device_sms() ? 4 : 1; }
 
 // Threads of a block whose widest phase has n items, in whole warps; at least four (reduce_rows takes
 // three of the nine reduced quantities per warp).

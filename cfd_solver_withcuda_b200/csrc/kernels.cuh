@@ -138,8 +138,8 @@ struct FluxParams {
   int limiter;
   int recon_prim;
   int muscl;            // 0 reference stencil, 1 Green-Gauss-gradient MUSCL
-  int lanes;            // threads per cell in the flux kernel: 1 or 4
-  int flux_minb = 1;    // one-lane limited second-order kernels built for 1, 6 or 8 resident blocks per SM
+  int lanes;            // threads per cell in the flux kernel: 1 or 4 (default by flux_lanes_for)
+  int flux_minb = 6;    // one-lane limited second-order kernels built for 1, 6 or 8 resident blocks per SM
   int persist_minb = 0;  // persistent stage kernel built for 4, 6 or 8 resident blocks per SM (0: 6 in
                          // FP64, 8 in the FP32-flux form)
   int faces_shape;      // face kernel launch: 0 256 threads, 1 256 threads at <= 80 registers, 2 128 threads
@@ -197,13 +197,22 @@ struct TileMaps {
 // kernels launched.
 int launch_prim_all(cudaStream_t s, const DevMesh &m, DevState &st);
 int launch_bc(cudaStream_t s, const DevMesh &m, DevState &st, const BcParams &bp, int stage_src_is_S, int cur_is_S);
-int launch_flux(cudaStream_t s, const DevMesh &m, DevState &st, const FluxParams &fp, int stage_src_is_S);
+// What a per-cell flux evaluation leaves besides the residual: del_t, and Min_dt from it.
+enum FluxWant { kWantDt = 1, kWantMin = 2 };
+int launch_flux(cudaStream_t s, const DevMesh &m, DevState &st, const FluxParams &fp, int stage_src_is_S,
+                int want = kWantDt | kWantMin);
+int flux_lanes_for(int cells);
 // Lax_Fedrichs over cells grouped by wavefront level (cells[level_start[l] .. level_start[l+1])).
 int launch_lax_friedrichs(cudaStream_t s, const DevMesh &m, DevState &st, const int *cells,
                           const std::vector<int> &level_start);
 // kind: 1,2,3 = reference RK3 stages; 0 = Explicit; 11..14 = RK4 stages; fuse_final = apply
 // Estimate_Error + Update in the last stage's kernel.
-int launch_stage(cudaStream_t s, const DevMesh &m, DevState &st, int kind, int lts, int fuse_final, int keep_delu);
+// flags: write the ghost states of the next stage from the owner threads (kStageGhosts; kStageExitS: the
+// supersonic-exit copy reads the stage state), or those of the next pseudo-step's first stage
+// (kStageNextStep, last stage); leave out the norms (kStageNoNorms, last stage, no t_end).
+enum StageFlags { kStageGhosts = 2, kStageExitS = 4, kStageNextStep = 8, kStageNoNorms = 16 };
+int launch_stage(cudaStream_t s, const DevMesh &m, DevState &st, const BcParams &bp, int kind, int lts, int fuse_final,
+                 int keep_delu, int flags);
 // Face-based forms with a per-cell stage dt (lts 1 or 2): gradients, face fluxes and the fused
 // gather + stage update.
 int launch_faces(cudaStream_t s, const DevMesh &m, DevState &st, const FluxParams &fp);
