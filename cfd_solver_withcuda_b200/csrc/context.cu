@@ -374,7 +374,7 @@ struct cfd_ctx {
   cudaGraphExec_t stage_graph[4] = {nullptr, nullptr, nullptr, nullptr};
   int stage_graph_launches[4] = {0, 0, 0, 0};
   int n_stage_graphs = 0;
-  double *h_ctl = nullptr;  // pinned mirror of the control block
+  double *h_ctl = nullptr;  // pinned mirror of the control block and the two status words behind it
   int *d_perm = nullptr;    // device copy of perm
   int *d_lf_cells = nullptr;       // Lax_Fedrichs: device cells grouped by wavefront level
   std::vector<int> lf_level_start;  // first entry of each level in d_lf_cells, plus the end
@@ -627,11 +627,11 @@ int enqueue_step(cfd_ctx *ctx, bool fuse_final, bool full = true, bool ghosts_wr
 }
 
 cfd_status sync_status(cfd_ctx *ctx, cfd_step_info *info) {
-  CUDA_TRY(cudaMemcpyAsync(ctx->h_ctl, ctx->ds.ctl, sizeof(double) * CTL_SIZE, cudaMemcpyDeviceToHost, ctx->stream));
-  int h_status[2];
-  CUDA_TRY(cudaMemcpyAsync(h_status, ctx->ds.status, sizeof(h_status), cudaMemcpyDeviceToHost, ctx->stream));
+  CUDA_TRY(cudaMemcpyAsync(ctx->h_ctl, ctx->ds.ctl, sizeof(double) * (CTL_SIZE + 1), cudaMemcpyDeviceToHost, ctx->stream));
   CUDA_TRY(cudaStreamSynchronize(ctx->stream));
   CUDA_TRY(cudaGetLastError());
+  int h_status[2];
+  std::memcpy(h_status, ctx->h_ctl + CTL_SIZE, sizeof(h_status));
   cfd_status st = static_cast<cfd_status>(h_status[0]);
   int bad = -1;
   if (st == CFD_ERR_NONPHYSICAL && h_status[1] != INT_MAX) {
@@ -876,7 +876,7 @@ cfd_status cfd_create(const cfd_mesh_desc *d, const cfd_config *cfg, cfd_ctx **o
       return bail(fail(CFD_ERR_CUDA, "stream creation failed"));
     ctx->own_stream = true;
   }
-  if (cudaMallocHost(reinterpret_cast<void **>(&ctx->h_ctl), sizeof(double) * CTL_SIZE) != cudaSuccess)
+  if (cudaMallocHost(reinterpret_cast<void **>(&ctx->h_ctl), sizeof(double) * (CTL_SIZE + 1)) != cudaSuccess)
     return bail(fail(CFD_ERR_CUDA, "pinned allocation failed"));
 
   // Renumbering (reverse Cuthill-McKee over physical cells; ghosts keep their ids).
@@ -1324,7 +1324,7 @@ cfd_status cfd_create(const cfd_mesh_desc *d, const cfd_config *cfg, cfd_ctx **o
   if (m.NF > 0 && !st.F) {
     if ((s = ctx_alloc(ctx, (void **)&st.F, 4 * (size_t)m.NF * dsz)) != CFD_OK) return bail(s);
   }
-  if ((s = ctx_alloc(ctx, (void **)&st.ctl, CTL_SIZE * dsz)) != CFD_OK) return bail(s);
+  if ((s = ctx_alloc(ctx, (void **)&st.ctl, (CTL_SIZE + 8) * dsz)) != CFD_OK) return bail(s);
   // Face-based forms: the (rho, u, v, p) rows and the face fluxes, one allocation (rows first), are
   // kept in L2 as persisting lines: the gather writes the rows that the gradient and face kernels
   // read next, and the face kernel writes the fluxes the gather reads right after.  The device's
@@ -1379,7 +1379,7 @@ cfd_status cfd_create(const cfd_mesh_desc *d, const cfd_config *cfg, cfd_ctx **o
   const size_t counter_bytes = 64 + 4 * (size_t)(kMaxGroups + 1);
   if ((s = ctx_alloc(ctx, (void **)&st.counter, counter_bytes)) != CFD_OK) return bail(s);
   st.gcount = st.counter + 16;
-  if ((s = ctx_alloc(ctx, (void **)&st.status, 64)) != CFD_OK) return bail(s);
+  st.status = reinterpret_cast<int *>(st.ctl + CTL_SIZE);  // behind the control block: one copy brings both
   if (cudaMemset(st.U, 0, 4 * (size_t)NT * dsz) != cudaSuccess || cudaMemset(st.S, 0, 4 * (size_t)NP * dsz) != cudaSuccess ||
       cudaMemset(st.prim, 0, 5 * (size_t)NT * dsz) != cudaSuccess || cudaMemset(st.R, 0, 4 * (size_t)NP * dsz) != cudaSuccess ||
       cudaMemset(st.dtc, 0, (size_t)NP * dsz) != cudaSuccess || cudaMemset(st.dU, 0, 4 * (size_t)NP * dsz) != cudaSuccess ||
@@ -1400,6 +1400,7 @@ cfd_status cfd_create(const cfd_mesh_desc *d, const cfd_config *cfg, cfd_ctx **o
   fp.recon_prim = cfg->reconstruct_primitive;
   fp.muscl = cfg->muscl && cfg->is_second_order;
   fp.lanes = flux_lanes_for(NP);
+  ctx->dm.pdl = pdl_for(NP);
   fp.faces_shape = 3;
   // WENO (Is_WENO): Explicit_Method falls back to the 1O/2O residual when any cell is not a quad
   // (src/Numerical_Method.cpp:31-55); Runge_Kutta_Method keeps WENO (zero flux on those cells).

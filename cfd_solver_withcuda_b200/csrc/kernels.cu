@@ -720,6 +720,7 @@ __global__ void __launch_bounds__(kFluxBlock, MINB) k_flux(const __grid_constant
                                                            const __grid_constant__ DevState st,
                                                            const __grid_constant__ FluxParams fp, int src_is_S,
                                                            int want) {
+  pdl_enter();
   __shared__ double sh[32];
   const int NP = m.NP, NT = m.NT;
   const int c = blockIdx.x * blockDim.x + threadIdx.x;
@@ -776,6 +777,7 @@ __global__ void __launch_bounds__(kFlux4Block) k_flux4(const __grid_constant__ D
                                                        const __grid_constant__ DevState st,
                                                        const __grid_constant__ FluxParams fp, int src_is_S,
                                                        int want) {
+  pdl_enter();
   __shared__ double sh[32];
   const int NP = m.NP, NT = m.NT;
   const int gid = blockIdx.x * blockDim.x + threadIdx.x;
@@ -1456,6 +1458,7 @@ __device__ __forceinline__ void cell_update(const DevMesh &m, const DevState &st
 // on 524,288 cells), the missing norms 10 us of the last stage's 22 there.
 __global__ void __launch_bounds__(kBlock) k_stage(DevMesh m, DevState st, BcParams bp, int kind, int lts,
                                                   int fuse_final, int keep_delu, int flags) {
+  pdl_enter();
   const int NP = m.NP;
   const int c = item_index(m.cblk, NP);
   const bool done = step_done(st.ctl);
@@ -3459,8 +3462,8 @@ int launch_lax_friedrichs(cudaStream_t s, const DevMesh &m, DevState &st, const 
 template <int DISS, int ORDER>
 void launch_flux_src(int g, cudaStream_t s, const DevMesh &m, DevState &st, const FluxParams &fp, int src_is_S,
                      int want) {
-  if (fp.consistent && src_is_S) k_flux<DISS, ORDER, 6, true><<<g, kFluxBlock, 0, s>>>(m, st, fp, src_is_S, want);
-  else k_flux<DISS, ORDER, 6, false><<<g, kFluxBlock, 0, s>>>(m, st, fp, src_is_S, want);
+  if (fp.consistent && src_is_S) launch_k(m, k_flux<DISS, ORDER, 6, true>, g, kFluxBlock, s, m, st, fp, src_is_S, want);
+  else launch_k(m, k_flux<DISS, ORDER, 6, false>, g, kFluxBlock, s, m, st, fp, src_is_S, want);
 }
 
 // The second-order per-cell forms with the directional limiter (ROE_2O, RICCA_2O, MOVERS_NWSC_2O):
@@ -3471,16 +3474,16 @@ void launch_flux_limited(int g, cudaStream_t s, const DevMesh &m, DevState &st, 
                          int want) {
   if (!(fp.consistent && src_is_S)) {
     switch (fp.flux_minb) {
-      case 1: k_flux<DISS, 2, 1, false><<<g, kFluxBlock, 0, s>>>(m, st, fp, src_is_S, want); break;
-      case 8: k_flux<DISS, 2, 8, false><<<g, kFluxBlock, 0, s>>>(m, st, fp, src_is_S, want); break;
-      default: k_flux<DISS, 2, 6, false><<<g, kFluxBlock, 0, s>>>(m, st, fp, src_is_S, want); break;
+      case 1: launch_k(m, k_flux<DISS, 2, 1, false>, g, kFluxBlock, s, m, st, fp, src_is_S, want); break;
+      case 8: launch_k(m, k_flux<DISS, 2, 8, false>, g, kFluxBlock, s, m, st, fp, src_is_S, want); break;
+      default: launch_k(m, k_flux<DISS, 2, 6, false>, g, kFluxBlock, s, m, st, fp, src_is_S, want); break;
     }
     return;
   }
   switch (fp.flux_minb) {
-    case 1: k_flux<DISS, 2, 1><<<g, kFluxBlock, 0, s>>>(m, st, fp, src_is_S, want); break;
-    case 8: k_flux<DISS, 2, 8><<<g, kFluxBlock, 0, s>>>(m, st, fp, src_is_S, want); break;
-    default: k_flux<DISS, 2, 6><<<g, kFluxBlock, 0, s>>>(m, st, fp, src_is_S, want); break;
+    case 1: launch_k(m, k_flux<DISS, 2, 1>, g, kFluxBlock, s, m, st, fp, src_is_S, want); break;
+    case 8: launch_k(m, k_flux<DISS, 2, 8>, g, kFluxBlock, s, m, st, fp, src_is_S, want); break;
+    default: launch_k(m, k_flux<DISS, 2, 6>, g, kFluxBlock, s, m, st, fp, src_is_S, want); break;
   }
 }
 
@@ -3499,10 +3502,10 @@ int launch_flux(cudaStream_t s, const DevMesh &m, DevState &st, const FluxParams
   }
   if (fp.lanes == 1) {
     const int g = nblk(m.NP, kFluxBlock);
-    if (fp.dissipation == 3 && !fp.second_order) k_flux<3, 1><<<g, kFluxBlock, 0, s>>>(m, st, fp, src_is_S, want);
+    if (fp.dissipation == 3 && !fp.second_order) launch_k(m, k_flux<3, 1>, g, kFluxBlock, s, m, st, fp, src_is_S, want);
     else if (fp.dissipation == 2 && !fp.second_order) launch_flux_src<2, 1>(g, s, m, st, fp, src_is_S, want);
     else if (fp.dissipation == 2) launch_flux_src<2, 2>(g, s, m, st, fp, src_is_S, want);
-    else if (fp.dissipation == 4 && !fp.second_order) k_flux<4, 1><<<g, kFluxBlock, 0, s>>>(m, st, fp, src_is_S, want);
+    else if (fp.dissipation == 4 && !fp.second_order) launch_k(m, k_flux<4, 1>, g, kFluxBlock, s, m, st, fp, src_is_S, want);
     else if (fp.dissipation == 5 && !fp.second_order) launch_flux_src<5, 1>(g, s, m, st, fp, src_is_S, want);
     else if (fp.dissipation == 6) launch_flux_src<6, 1>(g, s, m, st, fp, src_is_S, want);
     else if (fp.dissipation == 7) launch_flux_src<7, 1>(g, s, m, st, fp, src_is_S, want);
@@ -3512,25 +3515,25 @@ int launch_flux(cudaStream_t s, const DevMesh &m, DevState &st, const FluxParams
     else launch_flux_src<1, 1>(g, s, m, st, fp, src_is_S, want);
   } else {
     const int g = nblk(4 * m.NP, kFlux4Block);
-    if (fp.dissipation == 3 && !fp.second_order) k_flux4<3, 1><<<g, kFlux4Block, 0, s>>>(m, st, fp, src_is_S, want);
-    else if (fp.dissipation == 2 && !fp.second_order) k_flux4<2, 1><<<g, kFlux4Block, 0, s>>>(m, st, fp, src_is_S, want);
-    else if (fp.dissipation == 2) k_flux4<2, 2><<<g, kFlux4Block, 0, s>>>(m, st, fp, src_is_S, want);
-    else if (fp.dissipation == 4 && !fp.second_order) k_flux4<4, 1><<<g, kFlux4Block, 0, s>>>(m, st, fp, src_is_S, want);
-    else if (fp.dissipation == 4) k_flux4<4, 2><<<g, kFlux4Block, 0, s>>>(m, st, fp, src_is_S, want);
-    else if (fp.dissipation == 5 && !fp.second_order) k_flux4<5, 1><<<g, kFlux4Block, 0, s>>>(m, st, fp, src_is_S, want);
-    else if (fp.dissipation == 5) k_flux4<5, 2><<<g, kFlux4Block, 0, s>>>(m, st, fp, src_is_S, want);
-    else if (fp.dissipation == 6) k_flux4<6, 1><<<g, kFlux4Block, 0, s>>>(m, st, fp, src_is_S, want);
-    else if (fp.dissipation == 7) k_flux4<7, 1><<<g, kFlux4Block, 0, s>>>(m, st, fp, src_is_S, want);
-    else if (fp.dissipation == 3) k_flux4<3, 2><<<g, kFlux4Block, 0, s>>>(m, st, fp, src_is_S, want);
-    else k_flux4<1, 1><<<g, kFlux4Block, 0, s>>>(m, st, fp, src_is_S, want);
+    if (fp.dissipation == 3 && !fp.second_order) launch_k(m, k_flux4<3, 1>, g, kFlux4Block, s, m, st, fp, src_is_S, want);
+    else if (fp.dissipation == 2 && !fp.second_order) launch_k(m, k_flux4<2, 1>, g, kFlux4Block, s, m, st, fp, src_is_S, want);
+    else if (fp.dissipation == 2) launch_k(m, k_flux4<2, 2>, g, kFlux4Block, s, m, st, fp, src_is_S, want);
+    else if (fp.dissipation == 4 && !fp.second_order) launch_k(m, k_flux4<4, 1>, g, kFlux4Block, s, m, st, fp, src_is_S, want);
+    else if (fp.dissipation == 4) launch_k(m, k_flux4<4, 2>, g, kFlux4Block, s, m, st, fp, src_is_S, want);
+    else if (fp.dissipation == 5 && !fp.second_order) launch_k(m, k_flux4<5, 1>, g, kFlux4Block, s, m, st, fp, src_is_S, want);
+    else if (fp.dissipation == 5) launch_k(m, k_flux4<5, 2>, g, kFlux4Block, s, m, st, fp, src_is_S, want);
+    else if (fp.dissipation == 6) launch_k(m, k_flux4<6, 1>, g, kFlux4Block, s, m, st, fp, src_is_S, want);
+    else if (fp.dissipation == 7) launch_k(m, k_flux4<7, 1>, g, kFlux4Block, s, m, st, fp, src_is_S, want);
+    else if (fp.dissipation == 3) launch_k(m, k_flux4<3, 2>, g, kFlux4Block, s, m, st, fp, src_is_S, want);
+    else launch_k(m, k_flux4<1, 1>, g, kFlux4Block, s, m, st, fp, src_is_S, want);
   }
   return n + 1;
 }
 
 int launch_stage(cudaStream_t s, const DevMesh &m, DevState &st, const BcParams &bp, int kind, int lts, int fuse_final,
                  int keep_delu, int flags) {
-  if (m.cblk) k_stage<<<m.n_cblk, kWorkCellBlock, 0, s>>>(m, st, bp, kind, lts, fuse_final, keep_delu, flags);
-  else k_stage<<<nblk(m.NP, kBlock), kBlock, 0, s>>>(m, st, bp, kind, lts, fuse_final, keep_delu, flags);
+  if (m.cblk) launch_k(m, k_stage, m.n_cblk, kWorkCellBlock, s, m, st, bp, kind, lts, fuse_final, keep_delu, flags);
+  else launch_k(m, k_stage, nblk(m.NP, kBlock), kBlock, s, m, st, bp, kind, lts, fuse_final, keep_delu, flags);
   return 1;
 }
 
@@ -3919,6 +3922,12 @@ int device_sms() {
 // 34 / 40 / 46 / 36 at 3,200 cells, 33 / 36 / 44 / 38 against 36 / 42 / 48 / 38 at 20,000,
 // 47 / 52 / 62 / 52 against 37 / 48 / 56 / 44 at 45,451.
 int flux_lanes_for(int cells) { return 4LL * cells <= 640LL * device_sms() ? 4 : 1; }
+
+// Programmatic dependent launch pays from two waves of the six-blocks-per-SM kernels on: per pseudo-step at
+// 524,288 cells 252 -> 249 us (gradient MUSCL), 225 -> 220 (FP32-flux), 358 -> 355 (ROE_2O), 239 -> 235
+// (LLF).  Below, blocks that start while the previous kernel still holds part of the chip are spread unevenly
+// over the SMs: ROE_2O at 45,451 cells 57 -> 64 us, at 11,250 35.4 -> 35.4 (B200).
+int pdl_for(int cells) { return cells >= 2LL * 6 * kFluxBlock * device_sms() ? 1 : 0; }
 
 // Threads of a block whose widest phase has n items, in whole warps; at least four (reduce_rows takes
 // three of the nine reduced quantities per warp).

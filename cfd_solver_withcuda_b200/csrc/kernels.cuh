@@ -202,6 +202,7 @@ enum FluxWant { kWantDt = 1, kWantMin = 2 };
 int launch_flux(cudaStream_t s, const DevMesh &m, DevState &st, const FluxParams &fp, int stage_src_is_S,
                 int want = kWantDt | kWantMin);
 int flux_lanes_for(int cells);
+int pdl_for(int cells);
 // Lax_Fedrichs over cells grouped by wavefront level (cells[level_start[l] .. level_start[l+1])).
 int launch_lax_friedrichs(cudaStream_t s, const DevMesh &m, DevState &st, const int *cells,
                           const std::vector<int> &level_start);

@@ -226,7 +226,8 @@ cfd_status cfd_sync(cfd_ctx *ctx, cfd_step_info *info);
  * "flux_lanes" (threads per cell of the per-cell flux kernel, 1 or 4, default 4 up to 160 cells per SM, else 1),
  * "flux_minb" (the one-lane second-order kernels with the directional limiter -- ROE_2O, RICCA_2O,
  * MOVERS_NWSC_2O -- register-capped for 1 (uncapped), 6 or 8 resident blocks per SM, default 6),
- * "pdl" (launch the kernels of a pseudo-step with programmatic dependent launch, default 0),
+ * "pdl" (launch the kernels of a pseudo-step with programmatic dependent launch, default 1 from 1,536
+ * cells per SM on, else 0),
  * "patch_stage" (with reorder 3, the face-based forms with a per-cell dt frozen per step run each
  * stage as one kernel: a thread block per 128-cell patch computes the records, face fluxes, gather
  * and update of its cells in shared memory; default 0, tried by cfd_autotune),
