@@ -404,6 +404,8 @@ struct cfd_ctx {
   // at the first multi-step call, or of a batch's active instances.
   bool steps_known = false;
   int steps_off = 0;      // option "one_launch_steps" 0
+  int cell_steps = -1;    // k_cell_steps available (-1: not asked yet)
+  unsigned int *d_cell_steps = nullptr;
   StepsShape steps{};
   std::vector<int> bptr;  // host copy of the cells' boundary-entry offsets
   bool t_end_set = false;
@@ -1649,12 +1651,32 @@ static cfd_status enqueue_steps(cfd_ctx *ctx, int n_steps) {
     return enqueue_steps_one_launch(ctx, n_steps, true);
   if (ctx->persistent && ctx->persist_grid > 0 && ctx->dm.NF > 0) return enqueue_steps_persistent(ctx, n_steps);
   // Every step but the last leaves out what the next one overwrites, unless a t_end may make any the last.
-  const int lean = ctx->t_end_set ? 0 : n_steps - 1;
+  int lean = ctx->t_end_set ? 0 : n_steps - 1;
   // Per-cell forms: such a step also leaves the next one's ghosts, so only the first needs them formed here.
   const bool ghosts = ctx->dm.NF == 0;
   if (lean > 0 && ghosts) {
     TimedScope ts(ctx, TK_BC);
     ctx->launches += launch_bc(ctx->stream, ctx->dm, ctx->ds, ctx->bp, 0, 0);
+  }
+  // Small ones run them in one launch.
+  if (lean > 0 && ghosts && ctx->fp.lanes == 4 && !ctx->steps_off && ctx->use_graph && !ctx->profile && !ctx->fp.weno &&
+      !ctx->dm.cblk) {
+    if (ctx->cell_steps < 0) {
+      const size_t n = 3 * kStepsBarrierStride * sizeof(unsigned int);
+      cfd_status s = ctx_alloc(ctx, (void **)&ctx->d_cell_steps, n);
+      if (s != CFD_OK) return s;
+      CUDA_TRY(cudaMemsetAsync(ctx->d_cell_steps, 0, n, ctx->stream));
+      ctx->cell_steps = cell_steps_available(ctx->fp, ctx->NP) ? 1 : 0;
+    }
+    if (ctx->cell_steps > 0) {
+      const StagePlan p = stage_plan(ctx->cfg, ctx->fp.consistent);
+      for (int i = 0; i < lean; i += kStepsPerLaunch)
+        ctx->launches += launch_cell_steps(ctx->stream, ctx->dm, ctx->ds, ctx->fp, ctx->bp, ctx->d_cell_steps,
+                                           std::min(kStepsPerLaunch, lean - i), p.n, p.kind0, stage_lts(p, ctx->cfg, 0),
+                                           stage_lts(p, ctx->cfg, 1), p.src_S, ctx->persist_test_arrivals);
+      n_steps = 1;
+      lean = 0;
+    }
   }
   if (ctx->use_graph && !ctx->profile && n_steps > 1) {
     auto capture = [&](bool full, cudaGraphExec_t *exec, int *launches) -> cfd_status {

@@ -544,18 +544,38 @@ __device__ __forceinline__ void load_cell(const DevMesh &m, const DevState &st, 
   q.degen = m.degen[c];
 }
 
+// Geometry of face f of cell c.
+struct FaceGeo {
+  int N, n2;
+  double nx, ny, dl, d1, d2;
+};
+template <int DISS, int ORDER>
+__device__ __forceinline__ FaceGeo load_face(const DevMesh &m, int c, int f) {
+  const int idx = f * m.NP + c;
+  FaceGeo g;
+  g.N = m.nbr[idx];
+  g.nx = m.nx[idx];
+  g.ny = m.ny[idx];
+  g.dl = m.dl[idx];
+  if (ORDER == 2 && DISS != 2) {
+    g.n2 = m.n2[idx];
+    g.d1 = m.d1l[idx];
+    g.d2 = m.d2l[idx];
+  }
+  return g;
+}
+
 // Contribution of face f of cell c: X = avg - diss (Calculate_Flux_For_All_Faces,
 // src/Net_Flux.cpp:18-43) and the del_t term (|V.n| + a) dl (src/Time_Step.cpp:326-336).
 template <int DISS, int ORDER, typename O>
 __device__ __forceinline__ void face_contrib(O &o, const DevMesh &m, const DevState &st, const FluxParams &fp,
-                                             const USrc &us, const CellState &q, int c, int f, double X[4],
+                                             const USrc &us, const CellState &q, const FaceGeo &g, int f, double X[4],
                                              double &t) {
   const int NP = m.NP, NT = m.NT;
   const double *prim = st.prim;
   const double rc = q.rc, uc = q.uc, vc = q.vc, pc = q.pc, ac = q.ac;
-  const int idx = f * NP + c;
-  const int N = m.nbr[idx];
-  const double nx = m.nx[idx], ny = m.ny[idx], dl = m.dl[idx];
+  const int N = g.N;
+  const double nx = g.nx, ny = g.ny, dl = g.dl;
   const double rn = prim[N], un = prim[NT + N], vn = prim[2 * NT + N], pn = prim[3 * NT + N], an = prim[4 * NT + N];
   double A[4], D[4];
   if (DISS != 6 && DISS != 7) average_flux<double>(rc, uc, vc, pc, rn, un, vn, pn, nx, ny, dl, A);
@@ -565,8 +585,8 @@ __device__ __forceinline__ void face_contrib(O &o, const DevMesh &m, const DevSt
     else
       roe_1o<double>(o, rc, uc, vc, pc, ac, rn, un, vn, pn, an, nx, ny, dl, (q.degen >> f) & 1, D);
   } else if (DISS == 3 && ORDER == 2) {
-    const int n2 = m.n2[idx];
-    const double d1 = m.d1l[idx], d2 = m.d2l[idx];
+    const int n2 = g.n2;
+    const double d1 = g.d1, d2 = g.d2;
     double dU[4], phi[4];
     if (!fp.recon_prim) {
       double q1[4], q2[4];
@@ -612,8 +632,8 @@ __device__ __forceinline__ void face_contrib(O &o, const DevMesh &m, const DevSt
       for (int k = 0; k < 4; k++) UR[k] = us.get(k, N);
     }
     if (ORDER == 2 && DISS != 2) {
-      const int n2 = m.n2[idx];
-      const double d1 = m.d1l[idx], d2 = m.d2l[idx];
+      const int n2 = g.n2;
+      const double d1 = g.d1, d2 = g.d2;
       double q2[4], phi[4];
 #pragma unroll
       for (int k = 0; k < 4; k++) q2[k] = us.get(k, n2);
@@ -700,7 +720,7 @@ __device__ __noinline__ double4 face_contrib_again(const DevMesh &m, const DevSt
   CellState q;
   load_cell<DISS, ORDER>(m, st, us, c, q);
   double X[4], t;
-  face_contrib<DISS, ORDER>(o, m, st, fp, us, q, c, f, X, t);
+  face_contrib<DISS, ORDER>(o, m, st, fp, us, q, load_face<DISS, ORDER>(m, c, f), f, X, t);
   return make_double4(X[0], X[1], X[2], X[3]);
 }
 
@@ -738,7 +758,7 @@ __global__ void __launch_bounds__(kFluxBlock, MINB) k_flux(const __grid_constant
 #pragma unroll 1
     for (int f = 0; f < nf; f++) {
       double X[4], t;
-      face_contrib<DISS, ORDER>(o, m, st, fp, us, q, c, f, X, t);
+      face_contrib<DISS, ORDER>(o, m, st, fp, us, q, load_face<DISS, ORDER>(m, c, f), f, X, t);
       N0 += X[0];
       N1s += X[1];
       N2s += X[2];
@@ -771,29 +791,17 @@ __global__ void __launch_bounds__(kFluxBlock, MINB) k_flux(const __grid_constant
 // The same evaluation with four lanes per cell (one face each): lane 0 of each quad adds the
 // quad's face contributions in face order 0..nF-1 (warp shuffles), so every sum keeps the
 // reference's order and value; fewer live registers per thread give the SM more warps to hide
-// the gather and FP64 latencies.
+// the gather and FP64 latencies.  R and den are lane 0's.
 template <int DISS, int ORDER>
-__global__ void __launch_bounds__(kFlux4Block) k_flux4(const __grid_constant__ DevMesh m,
-                                                       const __grid_constant__ DevState st,
-                                                       const __grid_constant__ FluxParams fp, int src_is_S,
-                                                       int want) {
-  pdl_enter();
-  __shared__ double sh[32];
-  const int NP = m.NP, NT = m.NT;
-  const int gid = blockIdx.x * blockDim.x + threadIdx.x;
-  const int c = gid >> 2, f = gid & 3;
-  const bool done = step_done(st.ctl);
-  if (done) return;
-  const bool cell_ok = c < NP;
-  const int nf = cell_ok ? m.nf[c] : 0;
+__device__ __forceinline__ void quad_residual(const DevMesh &m, const DevState &st, const FluxParams &fp, int use_S, int c,
+                                              int f, int nf, const FaceGeo &g, double R[4], double &den) {
   double X[4] = {0.0, 0.0, 0.0, 0.0}, t = 0.0;
   if (f < nf) {
-    const int use_S = fp.consistent && src_is_S;
-    const USrc us{st.U, st.S, NT, NP, use_S};
+    const USrc us{st.U, st.S, m.NT, m.NP, use_S};
     CellState q;
     load_cell<DISS, ORDER>(m, st, us, c, q);
     Fast64 o;
-    face_contrib<DISS, ORDER>(o, m, st, fp, us, q, c, f, X, t);
+    face_contrib<DISS, ORDER>(o, m, st, fp, us, q, g, f, X, t);
     if (o.bad()) {
       const double4 Y = face_contrib_again<DISS, ORDER>(m, st, fp, use_S, c, f);
       X[0] = Y.x;
@@ -809,21 +817,37 @@ __global__ void __launch_bounds__(kFlux4Block) k_flux4(const __grid_constant__ D
     for (int k = 0; k < 4; k++) Y[d - 1][k] = __shfl_down_sync(kFull, X[k], d, 4);
     T[d - 1] = __shfl_down_sync(kFull, t, d, 4);
   }
-  double dt = 1e308 * 10.0;
-  if (cell_ok && f == 0) {
-    double R[4] = {0.0, 0.0, 0.0, 0.0};
-    double den = 0.0;
+  R[0] = R[1] = R[2] = R[3] = 0.0;
+  den = 0.0;
 #pragma unroll
-    for (int k = 0; k < 4; k++) R[k] += X[k];
-    den += t;
+  for (int k = 0; k < 4; k++) R[k] += X[k];
+  den += t;
 #pragma unroll
-    for (int d = 1; d < 4; d++) {
-      if (d < nf) {
+  for (int d = 1; d < 4; d++) {
+    if (d < nf) {
 #pragma unroll
-        for (int k = 0; k < 4; k++) R[k] += Y[d - 1][k];
-        den += T[d - 1];
-      }
+      for (int k = 0; k < 4; k++) R[k] += Y[d - 1][k];
+      den += T[d - 1];
     }
+  }
+}
+
+template <int DISS, int ORDER>
+__global__ void __launch_bounds__(kFlux4Block) k_flux4(const __grid_constant__ DevMesh m,
+                                                       const __grid_constant__ DevState st,
+                                                       const __grid_constant__ FluxParams fp, int src_is_S,
+                                                       int want) {
+  pdl_enter();
+  __shared__ double sh[32];
+  const int NP = m.NP;
+  const int gid = blockIdx.x * blockDim.x + threadIdx.x;
+  const int c = gid >> 2, f = gid & 3;
+  if (step_done(st.ctl)) return;
+  double R[4], den, dt = 1e308 * 10.0;
+  const int nf = c < NP ? m.nf[c] : 0;
+  const FaceGeo g = load_face<DISS, ORDER>(m, c < NP ? c : 0, f);
+  quad_residual<DISS, ORDER>(m, st, fp, fp.consistent && src_is_S, c, f, nf, g, R, den);
+  if (c < NP && f == 0) {
 #pragma unroll
     for (int k = 0; k < 4; k++) st.R[k * NP + c] = R[k];
     if (want) {
@@ -2355,6 +2379,147 @@ __global__ void __launch_bounds__(kStepsThreads, 1) k_steps(const __grid_constan
       steps_barrier(st, a, count, blk.blocks, arrivals);
     }
     if (a.may_stop && step_done(st.ctl)) break;  // the same flag in every block
+  }
+}
+
+// Pseudo-steps of a small per-cell solve in one cooperative launch: four lanes per cell, every cell resident,
+// the evaluation of k_flux4 and the update of k_stage one after the other with a grid barrier behind each
+// (a stage overwrites the primitives that its neighbours' evaluation reads; Min_dt is complete at the first).
+// Min_dt is an atomic minimum of order-preserving keys in three slots used in turn, so that a slot is reset
+// two barriers before it is used again.  Same operations on the same operands as the separate kernels: same
+// bits.  The residual, del_t and the norms stay out, so a step by the separate kernels follows.  Bound by
+// latency: two barriers, the gathers' L2 rounds (a barrier empties the L1, so what stays the same is kept in
+// registers) and one face's dependent FP64 chain per stage.  Per pseudo-step of three stages (separate
+// kernels against this, LLF / ROE / ROE_2O / HLLC, B200): 29 / 31 / 33 / 29 us against 17 / 20 / 22 / 19 at
+// 1,600 cells, 33 / 38 / 41 / 35 against 24 / 27 / 31 / 27 at 18,944, so every mesh that fits uses it.
+struct BcCell {
+  double nxv, nyv, av;
+  const double *W, *X;  // current state, exit-copy source
+  int e;
+  const double4 *bstate;
+  const double *bexit;
+  __device__ __forceinline__ double nx() const { return nxv; }
+  __device__ __forceinline__ double ny() const { return nyv; }
+  __device__ __forceinline__ double a() const { return av; }
+  __device__ __forceinline__ double cur(int k) const { return W[k]; }
+  __device__ __forceinline__ double src(int k) const { return X[k]; }
+};
+
+struct CellStepsArgs {
+  StepsArgs s;
+  int lts0, lts1;  // lts argument (see k_stage) of the first stage and of the others
+  int src_S;
+  unsigned long long *dt_min;  // [3], all ones before the launch
+};
+
+__device__ __forceinline__ unsigned long long ordered_key(double x) {
+  const unsigned long long b = (unsigned long long)__double_as_longlong(x);
+  return (b >> 63) ? ~b : b | (1ull << 63);
+}
+__device__ __forceinline__ double key_value(unsigned long long k) {
+  return __longlong_as_double((long long)((k >> 63) ? k & ~(1ull << 63) : ~k));
+}
+
+template <int DISS, int ORDER>
+__global__ void __launch_bounds__(kFlux4Block, 4) k_cell_steps(const __grid_constant__ DevMesh m,
+                                                               const __grid_constant__ DevState st,
+                                                               const __grid_constant__ FluxParams fp,
+                                                               const __grid_constant__ BcParams bp,
+                                                               const __grid_constant__ CellStepsArgs a) {
+  __shared__ double sh[32];
+  if (step_done(st.ctl)) return;  // the same for every block: nothing in the launch writes the flag
+  const int gid = blockIdx.x * blockDim.x + threadIdx.x;
+  const int c = gid >> 2, f = gid & 3;
+  const int nf = c < m.NP ? m.nf[c] : 0;
+  const bool owner = c < m.NP && f == 0, first_thread = gid == 0;
+  const int NP = m.NP, NT = m.NT;
+  const FaceGeo g = load_face<DISS, ORDER>(m, c < NP ? c : 0, f);
+  // The cell's boundary entries; two are kept.
+  const int b0 = owner ? m.bptr[c] : 0, ne = owner ? m.bptr[c + 1] - b0 : 0;
+  int ent[2];
+  int4 bnd[2];
+  double2 bn[2];
+#pragma unroll
+  for (int j = 0; j < 2; j++)
+    if (j < ne) {
+      ent[j] = m.bidx[b0 + j];
+      bnd[j] = m.bnd[ent[j]];
+      bn[j] = make_double2(m.nx[bnd[j].z * NP + c], m.ny[bnd[j].z * NP + c]);
+    }
+  unsigned int arrivals = 0;
+  int slot = 0;
+  double dtmin = 0.0, dtstep = 0.0, dtk = 0.0, total = first_thread ? st.ctl[CTL_TOTAL_TIME] : 0.0;
+  for (int i = 0; i < a.s.n_steps; i++) {
+    for (int k = 0; k < a.s.n_stages; k++) {
+      const int kind = a.s.kind0 ? a.s.kind0 + k : 0;
+      const int lts = k ? a.lts1 : a.lts0;
+      const bool last = k == a.s.n_stages - 1;
+      const bool want_min = lts == 0 || (k == 0 && lts != 1);
+      double R[4], den, dt = 1e308 * 10.0;
+      StageIn in;
+      if (owner) load_stage_in(m, st, c, kind, in);
+      quad_residual<DISS, ORDER>(m, st, fp, fp.consistent && k > 0, c, f, nf, g, R, den);
+      if (owner && (want_min || lts == 1)) dt = cell_dt(m, fp, c, den);
+      if (want_min) {
+        const double bm = block_min(dt, sh);
+        if (threadIdx.x == 0) atomicMin(a.dt_min + slot, ordered_key(bm));
+      }
+      steps_barrier(st, a.s, a.s.arrivals, gridDim.x, arrivals);
+      if (want_min) dtmin = key_value(__ldcg(a.dt_min + slot));
+      if (first_kind(kind)) {
+        dtstep = dtmin;
+        dtk = dt;
+      }
+      if (owner) {
+        const double d = lts == 0 ? dtmin : (lts == 1 ? dt : (lts == 2 ? dtk : dtstep));
+        double out[4];
+        const bool fin = stage_values(m, st, c, kind, d, R, in.Un, in, out);
+        if (fin && !direct_kind(kind)) {
+#pragma unroll
+          for (int j = 0; j < 4; j++) out[j] = in.Un[j] + out[j];
+        }
+#pragma unroll
+        for (int j = 0; j < 4; j++) {
+          if (last) st.U[(size_t)j * NT + c] = out[j];
+          else st.S[(size_t)j * NP + c] = out[j];
+        }
+        Prim q;
+        const bool ok = eos_fast(out[0], out[1], out[2], out[3], q);
+        store_prim(st.prim, st.q4, NT, c, q);
+        if (!ok) flag_bad(st.status, c);
+        // The next evaluation's ghosts (after the last stage from U^{n+1}, which `out` is).
+        BcCell src{0.0, 0.0, q.a, out, last || a.src_S ? out : in.Un, 0, m.bstate, m.bexit};
+        double G[4];
+#pragma unroll
+        for (int j = 0; j < 2; j++)
+          if (j < ne) {
+            src.nxv = bn[j].x;
+            src.nyv = bn[j].y;
+            src.e = ent[j];
+            if (bc_values(src, bp, bnd[j].x, q.rho, q.u, q.v, q.p, G)) store_ghost(st, NT, bnd[j].w, G);
+          }
+        for (int j = 2; j < ne; j++) {
+          const int4 b = m.bnd[m.bidx[b0 + j]];
+          src.nxv = m.nx[b.z * NP + c];
+          src.nyv = m.ny[b.z * NP + c];
+          src.e = m.bidx[b0 + j];
+          if (bc_values(src, bp, b.x, q.rho, q.u, q.v, q.p, G)) store_ghost(st, NT, b.w, G);
+        }
+      }
+      const int next = slot == 2 ? 0 : slot + 1;
+      if (first_thread) {
+        if (last) total += lts >= 2 ? dtstep : dtmin;
+        a.dt_min[next == 2 ? 0 : next + 1] = ~0ull;
+      }
+      slot = next;
+      steps_barrier(st, a.s, a.s.arrivals, gridDim.x, arrivals);
+    }
+  }
+  if (first_thread) {
+    st.ctl[CTL_TOTAL_TIME] = total;
+    st.ctl[CTL_ITER] += a.s.n_steps;
+    st.ctl[CTL_DTMIN] = dtmin;
+    st.ctl[CTL_DTSTEP] = dtstep;
   }
 }
 
@@ -3986,6 +4151,55 @@ StepsShape steps_shape(const FluxParams &fp, const int *bptr, const int4 *inst, 
   }
   cudaGetLastError();
   return sh;
+}
+
+const void *cell_steps_kernel(const FluxParams &fp) {
+  const bool two = fp.second_order;
+  switch (fp.dissipation) {
+    case 1: return (const void *)k_cell_steps<1, 1>;
+    case 2: return two ? (const void *)k_cell_steps<2, 2> : (const void *)k_cell_steps<2, 1>;
+    case 3: return two ? (const void *)k_cell_steps<3, 2> : (const void *)k_cell_steps<3, 1>;
+    case 4: return two ? (const void *)k_cell_steps<4, 2> : (const void *)k_cell_steps<4, 1>;
+    case 5: return two ? (const void *)k_cell_steps<5, 2> : (const void *)k_cell_steps<5, 1>;
+    case 6: return (const void *)k_cell_steps<6, 1>;
+    case 7: return (const void *)k_cell_steps<7, 1>;
+  }
+  return nullptr;
+}
+
+bool cell_steps_available(const FluxParams &fp, int cells) {
+  const void *k = cell_steps_kernel(fp);
+  int dev = 0, coop = 0, per_sm = 0;
+  if (!k || cudaGetDevice(&dev) != cudaSuccess ||
+      cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev) != cudaSuccess || !coop ||
+      cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k, kFlux4Block, 0) != cudaSuccess)
+    return false;
+  return nblk(4 * cells, kFlux4Block) <= per_sm * device_sms();
+}
+
+int launch_cell_steps(cudaStream_t s, const DevMesh &m, const DevState &st, const FluxParams &fp, const BcParams &bp,
+                      unsigned int *sync, int n_steps, int n_stages, int kind0, int lts0, int lts1, int src_S,
+                      unsigned int test_arrivals) {
+  DevMesh mm = m;
+  DevState ss = st;
+  FluxParams ff = fp;
+  BcParams bb = bp;
+  CellStepsArgs a{};
+  a.s.n_steps = n_steps;
+  a.s.n_stages = n_stages;
+  a.s.kind0 = kind0;
+  a.s.arrivals = sync;
+  a.s.gave_up = sync + kStepsBarrierStride;
+  a.s.test_arrivals = test_arrivals;
+  a.lts0 = lts0;
+  a.lts1 = lts1;
+  a.src_S = src_S;
+  a.dt_min = reinterpret_cast<unsigned long long *>(sync + 2 * kStepsBarrierStride);
+  void *args[] = {&mm, &ss, &ff, &bb, &a};
+  cudaMemsetAsync(sync, 0, sizeof(unsigned int), s);
+  cudaMemsetAsync(a.dt_min, 0xff, 3 * sizeof(unsigned long long), s);
+  cudaLaunchCooperativeKernel(cell_steps_kernel(fp), dim3(nblk(4 * m.NP, kFlux4Block)), dim3(kFlux4Block), args, 0, s);
+  return 1;
 }
 
 int launch_steps(cudaStream_t s, const DevMesh &m, const DevState &st, const FluxParams &fp, const BcParams &bp,

@@ -245,6 +245,13 @@ StepsShape steps_shape(const FluxParams &fp, const int *bptr, const int4 *inst, 
 int launch_steps(cudaStream_t s, const DevMesh &m, const DevState &st, const FluxParams &fp, const BcParams &bp,
                  const StepsShape &sh, const StepsBlock *blocks, unsigned int *arrivals, unsigned int *gave_up, int n_steps,
                  int n_stages, int kind0, int keep_delu, int reduce, int may_stop, unsigned int test_arrivals);
+// Whole pseudo-steps of a small per-cell solve in one cooperative launch (k_cell_steps), without residual,
+// del_t and norms, the next step's ghosts left behind.  Available when the cells' four lanes fit the chip.
+// sync: 3 * kStepsBarrierStride words, zero at first: the barrier's count, its give-up flag, the minima.
+bool cell_steps_available(const FluxParams &fp, int cells);
+int launch_cell_steps(cudaStream_t s, const DevMesh &m, const DevState &st, const FluxParams &fp, const BcParams &bp,
+                      unsigned int *sync, int n_steps, int n_stages, int kind0, int lts0, int lts1, int src_S,
+                      unsigned int test_arrivals);
 int launch_gather(cudaStream_t s, const DevMesh &m, DevState &st, const FluxParams &fp);
 // Fused gather + stage update of the per-cell-dt forms; del_t comes from the gradient pass
 // (launch_muscl_gradients with with_dt).  flags: bit 1 the owner thread writes its ghosts for the

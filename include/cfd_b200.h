@@ -241,9 +241,10 @@ cfd_status cfd_sync(cfd_ctx *ctx, cfd_step_info *info);
  * one CUDA graph per RK stage; default 0; the batched solves' form, see cfd_batch_set_option),
  * "persist_minb" (the persistent kernel's register budget: built for 4, 6 or 8 resident blocks per
  * SM; default 0: 6 in FP64 and 8 in the FP32-flux form, the faster of each on B200),
- * "one_launch_steps" (multi-step calls of the face-based forms with a per-cell dt frozen per step, of at
- * most 98,304 cells -- a batch's active instances together -- run many pseudo-steps in one cooperative
- * launch; default 1, 0: the separate kernels),
+ * "one_launch_steps" (multi-step calls run many pseudo-steps in one cooperative launch: the face-based
+ * forms with a per-cell dt frozen per step, of at most 98,304 cells -- a batch's active instances
+ * together -- and the per-cell forms without WENO whose four lanes per cell fit the chip; default 1,
+ * 0: the separate kernels),
  * "barrier_timeout_test" (a test of the bounded barriers: every barrier of the persistent form
  * waits for `value` more blocks than it has, so each wait runs out and the step reports
  * CFD_ERR_TIMEOUT; default 0),

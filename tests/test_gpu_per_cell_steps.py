@@ -43,3 +43,24 @@ def test_steps_in_one_call_equal_single_steps(nx, ny, reorder, diss, order, inte
         for k in ("U", "prim", "dt", "net_flux", "delU"):
             assert_bits_equal(a[k], b[k], k)
         assert ia == ib
+
+
+@pytest.mark.parametrize("nx,ny,steps", [(2, 2, 300), (148, 128, 5), (149, 128, 5)])
+@pytest.mark.parametrize("diss,order,lts", [(3, 2, 0), (1, 1, 1)])
+def test_one_launch_limits(nx, ny, steps, diss, order, lts):
+    """More steps than one launch holds; the largest mesh whose four lanes per cell are resident on 148 SMs
+    (18,944 cells) and one beyond it.  Against the separate kernels in the same calls."""
+    m = cb.Mesh.ramp(nx, ny, open_top=True)
+    NP = m.n_physical
+    U = np.zeros((m.n_total, 4))
+    x = m.centers[:NP]
+    U[:NP] = cb.conserved_from_primitive(1 + 0.02 * np.sin(7 * x[:, 0]), 2 + 0.02 * np.cos(5 * x[:, 1]), 0 * x[:, 0],
+                                         (1 + 0.01 * np.sin(9 * x[:, 1])) / 1.4)
+    U[m.boundary[:, 3]] = U[m.boundary[:, 1]]
+    kw = dict(dissipation_type=diss, is_second_order=order - 1, integrator=0, time_accurate=1, local_time_stepping=lts,
+              cfl=0.1, inlet_rho=1.0, inlet_p=1.0 / 1.4, inlet_u=2.0, reorder=4)
+    a, ia = _run(m, kw, U, dict(one_launch_steps=0), [(steps, 0.0), (3, 0.0)])
+    b, ib = _run(m, kw, U, {}, [(steps, 0.0), (3, 0.0)])
+    for k in ("U", "prim", "dt", "net_flux", "delU"):
+        assert_bits_equal(a[k], b[k], k)
+    assert ia == ib
