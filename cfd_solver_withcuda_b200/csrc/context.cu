@@ -1251,6 +1251,13 @@ cfd_status cfd_create(const cfd_mesh_desc *d, const cfd_config *cfg, cfd_ctx **o
     launch_face_weights(ctx->stream, m, gw);
     if (cudaGetLastError() != cudaSuccess) return bail(fail(CFD_ERR_CUDA, "face weights"));
     m.gw = gw;
+    if (cfg->precision == CFD_PREC_FP32_FLUX) {
+      float4 *r = nullptr;
+      if ((s = ctx_alloc(ctx, (void **)&r, 2 * (size_t)m.NF * sizeof(float4))) != CFD_OK) return bail(s);
+      launch_face_records(ctx->stream, m, r);
+      if (cudaGetLastError() != cudaSuccess) return bail(fail(CFD_ERR_CUDA, "face records"));
+      m.frec = r;
+    }
   }
   if (tile_tables && tile_prepare()) {
     TileMesh &tm = ctx->tm;

@@ -101,6 +101,18 @@ __device__ __forceinline__ void ld32f(const float4 *p, double4 &a, double4 &b) {
   a = make_double4(v[0], v[1], v[2], v[3]);
   b = make_double4(v[4], v[5], v[6], v[7]);
 }
+// Geometry and cells of one face of the FP32-flux form (DevMesh::frec).
+struct FaceRecord {
+  float nx, ny, dl, dx, dy;
+  int2 on;
+};
+__device__ __forceinline__ FaceRecord load_face_record(const float4 *rec, size_t i) {
+  float v[8];
+  asm("ld.global.v8.f32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+      : "=f"(v[0]), "=f"(v[1]), "=f"(v[2]), "=f"(v[3]), "=f"(v[4]), "=f"(v[5]), "=f"(v[6]), "=f"(v[7])
+      : "l"(rec + 2 * i));
+  return FaceRecord{v[0], v[1], v[2], v[3], v[4], make_int2(__float_as_int(v[5]), __float_as_int(v[6]))};
+}
 __device__ __forceinline__ void st32f(float4 *p, const double g[8]) {
   asm volatile("st.global.v8.f32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"(p), "f"(float(g[0])), "f"(float(g[1])),
                "f"(float(g[2])), "f"(float(g[3])), "f"(float(g[4])), "f"(float(g[5])), "f"(float(g[6])), "f"(float(g[7]))
@@ -1165,11 +1177,27 @@ __global__ void __launch_bounds__(MINB >= 6 ? 128 : 256, MINB) k_faces(const __g
   const int i = item_index(m.fblk, m.NF);
   if (i >= m.NF || step_done(st.ctl)) return;
   const int NP = m.NP;
-  const int2 on = m.fon[i];
-  const int c = on.x, N = on.y;
   const int glim = fp.limiter == LIM_REF_MINMOD ? LIM_MINMOD : fp.limiter;
-  const double4 gq = ld32(m.fg4 + i);
-  const T nx = T(gq.x), ny = T(gq.y), dl = T(gq.z), dx = T(gq.w), dy = T(m.fdy[i]);
+  int2 on;
+  T nx, ny, dl, dx, dy;
+  if constexpr (sizeof(T) == sizeof(float)) {
+    const FaceRecord r = load_face_record(m.frec, i);
+    on = r.on;
+    nx = r.nx;
+    ny = r.ny;
+    dl = r.dl;
+    dx = r.dx;
+    dy = r.dy;
+  } else {
+    on = m.fon[i];
+    const double4 gq = ld32(m.fg4 + i);
+    nx = gq.x;
+    ny = gq.y;
+    dl = gq.z;
+    dx = gq.w;
+    dy = m.fdy[i];
+  }
+  const int c = on.x, N = on.y;
   const double4 c0 = ld32(st.q4 + c), n0 = ld32(st.q4 + N);
   const int G = N < NP ? N : c;  // a ghost neighbour uses the owner's gradients
   double4 c1, c2, n1, n2;
@@ -1190,7 +1218,18 @@ __global__ void __launch_bounds__(MINB >= 6 ? 128 : 256, MINB) k_faces(const __g
   if constexpr (FaceOps<T>::fast) {
     if (o.bad()) F = face_flux_again<DISS>(m, st, fp, i);
   }
-  st32(st.F + i, F);
+  if constexpr (sizeof(T) == sizeof(float))  // float results: stored as such
+    reinterpret_cast<float4 *>(st.F)[i] = make_float4(float(F.x), float(F.y), float(F.z), float(F.w));
+  else
+    st32(st.F + i, F);
+}
+
+// Flux of face id as k_faces left it (FF: the FP32-flux form's floats).
+template <bool FF>
+__device__ __forceinline__ double4 load_flux(const DevState &st, int id) {
+  if (!FF) return ld32(st.F + id);
+  const float4 v = reinterpret_cast<const float4 *>(st.F)[id];
+  return make_double4(v.x, v.y, v.z, v.w);
 }
 
 // Sum of the face fluxes of cell c in face order (+F on the owner side, -F on the neighbour
@@ -1225,7 +1264,7 @@ __device__ __forceinline__ void sum_faces(int nf, const int4 e4, const double4 F
   }
 }
 
-template <bool DEN = true, bool CG = false>
+template <bool DEN = true, bool CG = false, bool FF = false>
 __device__ __forceinline__ void gather_faces(const DevMesh &m, const DevState &st, int c, double R[4], double &den) {
   const int NP = m.NP, NT = m.NT;
   const double uc = DEN ? st.prim[NT + c] : 0.0, vc = DEN ? st.prim[2 * NT + c] : 0.0,
@@ -1237,7 +1276,7 @@ __device__ __forceinline__ void gather_faces(const DevMesh &m, const DevState &s
 #pragma unroll
   for (int f = 0; f < 4; f++) {
     const int id = e[f] < 0 ? -e[f] - 1 : e[f];
-    F[f] = CG ? ldcg4(st.F + id) : ld32(st.F + id);
+    F[f] = CG ? ldcg4(st.F + id) : load_flux<FF>(st, id);
   }
   R[0] = R[1] = R[2] = R[3] = 0.0;
   den = 0.0;
@@ -1266,6 +1305,7 @@ __device__ __forceinline__ void gather_faces(const DevMesh &m, const DevState &s
 
 // Per cell: Net = sum of its face fluxes in face order, del_t from the cell's own state
 // (src/Time_Step.cpp:293-329), block min.
+template <bool FF>
 __global__ void __launch_bounds__(kFluxBlock) k_gather(DevMesh m, DevState st, FluxParams fp) {
   __shared__ double sh[32];
   const int NP = m.NP;
@@ -1274,7 +1314,7 @@ __global__ void __launch_bounds__(kFluxBlock) k_gather(DevMesh m, DevState st, F
   double dt = 1e308 * 10.0;
   if (c < NP && !done) {
     double R[4], den;
-    gather_faces(m, st, c, R, den);
+    gather_faces<true, false, FF>(m, st, c, R, den);
     dt = cell_dt(m, fp, c, den);
 #pragma unroll
     for (int k = 0; k < 4; k++) st.R[k * NP + c] = R[k];
@@ -1599,7 +1639,7 @@ __device__ __forceinline__ void stage_final_reduce(const DevState &st, const dou
 // block instead of once per 128 cells; each thread sums its cells' terms in cell order and the
 // grid is fixed per device, so the sums are reproducible.  Its accumulators spill 64 bytes at the
 // same 80-register cap, which measured faster than 96 registers at 5 blocks per SM.
-template <bool STRIDED>
+template <bool STRIDED, bool FF>
 __global__ void __launch_bounds__(kFluxBlock, 6) k_gather_stage(DevMesh m, DevState st, FluxParams fp,
                                                                              BcParams bp, int kind, int lts,
                                                                              int fuse_final, int keep_delu, int flags) {
@@ -1614,14 +1654,14 @@ __global__ void __launch_bounds__(kFluxBlock, 6) k_gather_stage(DevMesh m, DevSt
       // The residual gather is issued first; loading the state rows ahead of it (more registers,
       // fewer resident warps) measured slower on B200.
       double R[4], den = 0.0;
-      gather_faces<false>(m, st, c, R, den);
+      gather_faces<false, false, FF>(m, st, c, R, den);
       const double dtc = (lts == 1 || first_kind(kind)) ? st.dtc[c] : 0.0;  // the only stages that use it
       dtu = stage_cell(m, st, bp, c, R, dtc, kind, lts, fuse_final, keep_delu, flags, e);
     }
   } else {
     for (int c = blockIdx.x * blockDim.x + threadIdx.x; c < NP; c += gridDim.x * blockDim.x) {
       double R[4], den = 0.0;
-      gather_faces<false>(m, st, c, R, den);
+      gather_faces<false, false, FF>(m, st, c, R, den);
       const double dtc = (lts == 1 || first_kind(kind)) ? st.dtc[c] : 0.0;
       const double dt = stage_cell(m, st, bp, c, R, dtc, kind, lts, fuse_final, keep_delu, flags, e);
       dtu = dt < dtu ? dt : dtu;
@@ -1653,7 +1693,7 @@ struct BcRegs {
 // memory traffic: 204 - 236 bytes per cell and the fluxes.
 // MODE 0: not the last stage; 1: the last stage (one wave of blocks strides over the cells when there are
 // no work lists).
-template <int MODE>
+template <int MODE, bool FF>
 __global__ void __launch_bounds__(kFluxBlock, 6) k_gather_lean(DevMesh m, DevState st, BcParams bp, int kind, int flags,
                                                               int store_a) {
   pdl_enter();
@@ -1664,7 +1704,8 @@ __global__ void __launch_bounds__(kFluxBlock, 6) k_gather_lean(DevMesh m, DevSta
   for (int c = item_index(m.cblk, NP); c < NP; c += step) {
     const int info = m.nfb[c];
     const int4 e4 = m.cface4[c];
-    const double4 F0 = st.F[face_id(e4.x)], F1 = st.F[face_id(e4.y)], F2 = st.F[face_id(e4.z)], F3 = st.F[face_id(e4.w)];
+    const double4 F0 = load_flux<FF>(st, face_id(e4.x)), F1 = load_flux<FF>(st, face_id(e4.y)),
+                  F2 = load_flux<FF>(st, face_id(e4.z)), F3 = load_flux<FF>(st, face_id(e4.w));
     StageIn in;
     load_stage_in(m, st, c, kind, in);
     const bool first = first_kind(kind);
@@ -1720,6 +1761,16 @@ __global__ void __launch_bounds__(kFluxBlock, 6) k_gather_lean(DevMesh m, DevSta
       }
     }
   }
+}
+
+// The FP32-flux form's face records.
+__global__ void k_face_records(DevMesh m, float4 *r) {
+  const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= (size_t)m.NF) return;
+  const double4 g = m.fg4[i];
+  const int2 on = m.fon[i];
+  r[2 * i] = make_float4(float(g.x), float(g.y), float(g.z), float(g.w));
+  r[2 * i + 1] = make_float4(float(m.fdy[i]), __int_as_float(on.x), __int_as_float(on.y), 0.0f);
 }
 
 // Weights of the gradient passes: (nx dl, ny dl) of every face slot.
@@ -3658,7 +3709,7 @@ int launch_flux(cudaStream_t s, const DevMesh &m, DevState &st, const FluxParams
   if (fp.second_order && fp.muscl && m.NF > 0) {
     if (fp.precision == 1) launch_faces_t<float>(s, m, st, fp);
     else launch_faces_t<double>(s, m, st, fp);
-    k_gather<<<nblk(m.NP, kFluxBlock), kFluxBlock, 0, s>>>(m, st, fp);
+    (st.recf ? k_gather<true> : k_gather<false>)<<<nblk(m.NP, kFluxBlock), kFluxBlock, 0, s>>>(m, st, fp);
     return n + 2;
   }
   if (fp.weno) {
@@ -3704,7 +3755,7 @@ int launch_stage(cudaStream_t s, const DevMesh &m, DevState &st, const BcParams 
 
 int launch_gather(cudaStream_t s, const DevMesh &m, DevState &st, const FluxParams &fp) {
   const int g = m.cblk ? m.n_cblk : nblk(m.NP, kFluxBlock);
-  k_gather<<<g, kFluxBlock, 0, s>>>(m, st, fp);
+  (st.recf ? k_gather<true> : k_gather<false>)<<<g, kFluxBlock, 0, s>>>(m, st, fp);
   return 1;
 }
 
@@ -3753,7 +3804,7 @@ int gather_stage_wave_blocks() {
   int dev = 0, sms = 0, per_sm = 0;
   if (cudaGetDevice(&dev) != cudaSuccess) return 0;
   if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) return 0;
-  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_gather_stage<true>, kFluxBlock, 0) != cudaSuccess)
+  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_gather_stage<true, false>, kFluxBlock, 0) != cudaSuccess)
     return 0;
   return sms * per_sm;
 }
@@ -3762,10 +3813,10 @@ int launch_gather_stage(cudaStream_t s, const DevMesh &m, DevState &st, const Fl
                         int kind, int lts, int fuse_final, int keep_delu, int flags) {
   const int g = m.cblk ? m.n_cblk : nblk(m.NP, kFluxBlock);
   if (!m.cblk && fuse_final && final_kind(kind) && m.wave_blocks > 0 && g > m.wave_blocks)
-    launch_k(m, k_gather_stage<true>, m.wave_blocks, kFluxBlock, s, m, st, fp, bp, kind, lts, fuse_final, keep_delu,
+    launch_k(m, st.recf ? k_gather_stage<true, true> : k_gather_stage<true, false>, m.wave_blocks, kFluxBlock, s, m, st, fp, bp, kind, lts, fuse_final, keep_delu,
              flags);
   else
-    launch_k(m, k_gather_stage<false>, g, kFluxBlock, s, m, st, fp, bp, kind, lts, fuse_final, keep_delu, flags);
+    launch_k(m, st.recf ? k_gather_stage<false, true> : k_gather_stage<false, false>, g, kFluxBlock, s, m, st, fp, bp, kind, lts, fuse_final, keep_delu, flags);
   return 1;
 }
 
@@ -3775,22 +3826,27 @@ int launch_gather_lean(cudaStream_t s, const DevMesh &m, const DevState &st, con
   const int g = m.cblk ? m.n_cblk : nblk(m.NP, kFluxBlock);
   if (g == 0) return 0;
   if (final_kind(kind))
-    launch_k(m, k_gather_lean<1>, !m.cblk && m.lean_blocks > 0 ? std::min(g, m.lean_blocks) : g, kFluxBlock, s, m, st, bp,
+    launch_k(m, st.recf ? k_gather_lean<1, true> : k_gather_lean<1, false>, !m.cblk && m.lean_blocks > 0 ? std::min(g, m.lean_blocks) : g, kFluxBlock, s, m, st, bp,
              kind, flags, store_a);
-  else launch_k(m, k_gather_lean<0>, g, kFluxBlock, s, m, st, bp, kind, flags, store_a);
+  else launch_k(m, st.recf ? k_gather_lean<0, true> : k_gather_lean<0, false>, g, kFluxBlock, s, m, st, bp, kind, flags, store_a);
   return 1;
 }
 
 int gather_lean_wave_blocks() {
   int per_sm = 0;
   const int sms = device_sms();
-  if (sms <= 0 || cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_gather_lean<1>, kFluxBlock, 0) != cudaSuccess)
+  if (sms <= 0 || cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_gather_lean<1, false>, kFluxBlock, 0) != cudaSuccess)
     return 0;
   return sms * per_sm;
 }
 
 int launch_face_weights(cudaStream_t s, const DevMesh &m, double2 *gw) {
   k_face_weights<<<(unsigned)((4 * (size_t)m.NP + kBlock - 1) / kBlock), kBlock, 0, s>>>(m, gw);
+  return 1;
+}
+
+int launch_face_records(cudaStream_t s, const DevMesh &m, float4 *r) {
+  k_face_records<<<nblk(m.NF, kBlock), kBlock, 0, s>>>(m, r);
   return 1;
 }
 

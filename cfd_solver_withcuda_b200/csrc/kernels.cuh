@@ -48,6 +48,7 @@ struct DevMesh {
   const int *cface;  // [4][NP]
   const int2 *fon;     // [NF] owner, neighbour of each face (one load)
   const double4 *fg4;  // [NF] nx, ny, dl, dx of each face (dy stays in fdy)
+  const float4 *frec;  // [NF][2] FP32-flux form: nx, ny, dl, dx, dy as the floats they are used as, owner, neighbour
   const int4 *cface4;  // [NP] the same four slots per cell (one 16-byte load)
   const int4 *nbr4;    // [NP] the four neighbour slots per cell
   // Optional work lists (batched solves): each entry is one thread block's [start, end) range of
@@ -264,6 +265,7 @@ int launch_gather_lean(cudaStream_t s, const DevMesh &m, const DevState &st, con
                        int store_a);
 int gather_lean_wave_blocks();
 int launch_face_weights(cudaStream_t s, const DevMesh &m, double2 *gw);
+int launch_face_records(cudaStream_t s, const DevMesh &m, float4 *r);
 // Patch form of one stage (gradients, face fluxes, gather and stage update in one kernel): reads
 // the primitives `prim_in` and writes the stage's primitives and ghosts to st.prim, which must be a
 // different buffer (blocks read their halo cells' primitives while others write theirs).  Same
