@@ -1410,6 +1410,7 @@ cfd_status cfd_create(const cfd_mesh_desc *d, const cfd_config *cfg, cfd_ctx **o
   fp.muscl = cfg->muscl && cfg->is_second_order;
   fp.lanes = flux_lanes_for(NP);
   ctx->dm.pdl = pdl_for(NP);
+  ctx->dm.grad_ahead = grad_ahead_for(NP);
   fp.faces_shape = 3;
   // WENO (Is_WENO): Explicit_Method falls back to the 1O/2O residual when any cell is not a quad
   // (src/Numerical_Method.cpp:31-55); Runge_Kutta_Method keeps WENO (zero flux on those cells).

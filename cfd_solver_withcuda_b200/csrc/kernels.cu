@@ -81,6 +81,12 @@ __device__ __forceinline__ double4 ld32(const double4 *p) {
   asm("ld.global.v4.f64 {%0, %1, %2, %3}, [%4];" : "=d"(v.x), "=d"(v.y), "=d"(v.z), "=d"(v.w) : "l"(p));
   return v;
 }
+// Starts bringing the 16-byte granules inside [off, off + bytes) of a device array into L2.
+__device__ __forceinline__ void prefetch_l2(const void *p, size_t off, unsigned int bytes) {
+  const size_t a = reinterpret_cast<size_t>(p) + off, lo = (a + 15) & ~(size_t)15;
+  const size_t hi = (a + bytes) & ~(size_t)15;
+  if (hi > lo) asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(lo), "r"((unsigned int)(hi - lo)) : "memory");
+}
 __device__ __forceinline__ double4 ld32_ordered(const double4 *p) {
   double4 v;
   asm volatile("ld.global.v4.f64 {%0, %1, %2, %3}, [%4];"
@@ -1937,6 +1943,11 @@ __device__ __forceinline__ void cell_gradients_w(const DevMesh &m, const double4
 // with_bc: first stage of a step; each thread first applies the boundary conditions of its own
 // cell's boundary entries (Apply_Boundary_Conditions, as k_bc does), which is exact because a
 // ghost row depends only on its owner cell and is read by no other cell's gradient.
+// Bound by the latency of its two dependent loads (neighbour slots, then their rows), most of them from
+// DRAM: each block first starts bringing what a block one per SM later reads (grad_ahead) into L2, which
+// takes a pseudo-step of 524,288 cells from 246.6 to 241 us (FP32-flux 212 to 204.5), 245,000 cells from
+// 134 to 131.8 us; at 125,000 cells, in L2 anyway, 75.8 to 76.7, so meshes below two waves leave it out
+// (B200).  The same in the face and gather kernels gained nothing: their fluxes and rows are mostly in L2.
 template <bool DT>
 __global__ void __launch_bounds__(kBlock, 4) k_muscl_gradients(DevMesh m, DevState st, FluxParams fp, BcParams bp,
                                                                int with_bc) {
@@ -1944,6 +1955,26 @@ __global__ void __launch_bounds__(kBlock, 4) k_muscl_gradients(DevMesh m, DevSta
   const int c = item_index(m.rblk, m.NT);
   const int NP = m.NP;
   if (step_done(st.ctl)) return;
+  if (m.grad_ahead > 0 && threadIdx.x < (DT ? 17 : 7)) {
+    const int w = blockIdx.x + m.grad_ahead, t = threadIdx.x;
+    int c0 = w * kBlock, n = min(kBlock, NP - c0);
+    if (m.rblk) {
+      const int2 r = w < m.n_rblk ? m.rblk[w] : make_int2(0, 0);
+      c0 = r.x;
+      n = min(r.y, NP) - r.x;
+    }
+    if (n > 0) {
+      if (t == 0) prefetch_l2(m.nbr4, (size_t)c0 * 16, n * 16);
+      else if (t == 1) prefetch_l2(st.q4, (size_t)c0 * 32, n * 32);
+      else if (t == 2) prefetch_l2(m.inv_area, (size_t)c0 * 8, n * 8);
+      else if (!DT) prefetch_l2(m.gw, ((size_t)(t - 3) * NP + c0) * 16, n * 16);
+      else if (t < 7) prefetch_l2(m.nx, ((size_t)(t - 3) * NP + c0) * 8, n * 8);
+      else if (t < 11) prefetch_l2(m.ny, ((size_t)(t - 7) * NP + c0) * 8, n * 8);
+      else if (t < 15) prefetch_l2(m.dl, ((size_t)(t - 11) * NP + c0) * 8, n * 8);
+      else if (t == 15) prefetch_l2(m.area, (size_t)c0 * 8, n * 8);
+      else prefetch_l2(st.prim, ((size_t)4 * m.NT + c0) * 8, n * 8);
+    }
+  }
   if (c < NP) {
     if (with_bc && (m.nfb[c] & kHasEntries)) {
       const double4 q = ld32_ordered(st.q4 + c);
@@ -4144,11 +4175,14 @@ int device_sms() {
 // 47 / 52 / 62 / 52 against 37 / 48 / 56 / 44 at 45,451.
 int flux_lanes_for(int cells) { return 4LL * cells <= 640LL * device_sms() ? 4 : 1; }
 
+bool two_waves(int cells) { return cells >= 2LL * 6 * kFluxBlock * device_sms(); }
+
 // Programmatic dependent launch pays from two waves of the six-blocks-per-SM kernels on: per pseudo-step at
 // 524,288 cells 252 -> 249 us (gradient MUSCL), 225 -> 220 (FP32-flux), 358 -> 355 (ROE_2O), 239 -> 235
 // (LLF).  Below, blocks that start while the previous kernel still holds part of the chip are spread unevenly
 // over the SMs: ROE_2O at 45,451 cells 57 -> 64 us, at 11,250 35.4 -> 35.4 (B200).
-int pdl_for(int cells) { return cells >= 2LL * 6 * kFluxBlock * device_sms() ? 1 : 0; }
+int pdl_for(int cells) { return two_waves(cells) ? 1 : 0; }
+int grad_ahead_for(int cells) { return two_waves(cells) ? device_sms() : 0; }
 
 // Threads of a block whose widest phase has n items, in whole warps; at least four (reduce_rows takes
 // three of the nine reduced quantities per warp).

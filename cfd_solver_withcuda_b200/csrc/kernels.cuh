@@ -74,6 +74,7 @@ struct DevMesh {
   // Blocks of k_gather_stage resident on the whole device at once (SMs x blocks per SM): the grid
   // of its reducing stage (0 = one block per 128 cells).
   int wave_blocks;
+  int grad_ahead;       // blocks ahead whose inputs a block of the gradient pass brings into L2 (0: none)
   int lean_blocks;      // the same for k_gather_lean's last stage
   const uint8_t *nfb;   // [NP] face count, kHasEntries when the cell has boundary entries
   const double2 *gw;    // [4][NP] nx dl, ny dl (face-based forms)
@@ -204,6 +205,7 @@ int launch_flux(cudaStream_t s, const DevMesh &m, DevState &st, const FluxParams
                 int want = kWantDt | kWantMin);
 int flux_lanes_for(int cells);
 int pdl_for(int cells);
+int grad_ahead_for(int cells);
 // Lax_Fedrichs over cells grouped by wavefront level (cells[level_start[l] .. level_start[l+1])).
 int launch_lax_friedrichs(cudaStream_t s, const DevMesh &m, DevState &st, const int *cells,
                           const std::vector<int> &level_start);
