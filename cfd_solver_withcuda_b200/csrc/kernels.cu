@@ -1695,8 +1695,12 @@ struct BcRegs {
 // are formed again: every stage but the last, and the last stage of every pseudo-step but the last of a
 // call without t_end.  It leaves out those stores (R 32 bytes, three or four primitive planes of 8, dU)
 // and, in the last stage, all of the reduction but the step's Min_dt; the rows q4, the states, the frozen
-// dt, the sound speed (where the next gradient pass forms del_t) and the ghosts stay.  Bound by its
-// memory traffic: 204 - 236 bytes per cell and the fluxes.
+// dt, the sound speed (where the next gradient pass forms del_t) and the ghosts stay.  204 - 236 bytes per
+// cell and the fluxes; bound by the latency of the face slots and of the fluxes they name (16 - 18
+// long-scoreboard stalls per issue, DRAM 32 % busy): 28 us on 524,288 cells against k_gather_stage's 35.6.
+// Six blocks per SM: 53.1 us on 1,038,240 mixed cells, 28.0 on 524,288; seven 54.7 and 27.7, five and
+// eight slower.  A persistent loop with the next cell's face slots loaded ahead took 32.0 us, loading the
+// stage inputs before the fluxes and the branch-free EOS gained nothing (B200).
 // MODE 0: not the last stage; 1: the last stage (one wave of blocks strides over the cells when there are
 // no work lists).
 template <int MODE, bool FF>
