@@ -109,7 +109,8 @@ class MpnnNet(ctypes.Structure):
     """cfd_mpnn_net."""
     _fields_ = [(n, ctypes.c_int) for n in ("layers", "node_in", "edge_in", "out", "n_nodes", "n_edges")] + \
                [(n, ctypes.c_void_p) for n in ("params", "grads", "xn", "xe", "src", "dst", "dst_ptr", "src_ptr",
-                                                "src_order", "act", "pred", "dpred", "workspace")]
+                                                "src_order", "act", "pred", "dpred", "workspace")] + \
+               [(n, ctypes.c_int) for n in ("ld_xn", "ld_xe", "ld_dpred")]
 
 
 class StepInfo(ctypes.Structure):

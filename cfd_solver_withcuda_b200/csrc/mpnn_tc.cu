@@ -1275,8 +1275,12 @@ struct NetLayout {
   }
 };
 
+// Row stride of a network input or gradient (0: packed rows).
+int net_ld(int ld, int width) { return ld ? ld : width; }
+
 bool net_ok(const cfd_mpnn_net *n) {
-  return n && n->layers >= 0 && n->node_in >= 1 && n->node_in <= KMAX && n->edge_in >= 1 && n->edge_in <= KMAX &&
+  return n && net_ld(n->ld_xn, n->node_in) >= n->node_in && net_ld(n->ld_xe, n->edge_in) >= n->edge_in &&
+         n->layers >= 0 && n->node_in >= 1 && n->node_in <= KMAX && n->edge_in >= 1 && n->edge_in <= KMAX &&
          n->out >= 1 && n->out <= 16 && n->n_nodes >= 0 && n->n_edges >= 0 && n->params && n->act &&
          (n->n_nodes == 0 || (n->xn && n->dst_ptr && n->pred)) && (n->n_edges == 0 || (n->xe && n->src && n->dst)) &&
          aligned(n->params, 16) && aligned(n->act, 16);
@@ -1460,8 +1464,8 @@ cfd_status cfd_mpnn_net_forward(const cfd_mpnn_net *n, void *stream) {
   };
   const SegDev none{nullptr, nullptr, 0, 0, 0};
   const int N = n->n_nodes, E = n->n_edges;
-  run(y.enc_n, N, 1, seg_of(n->xn, n->node_in), none, none, nullptr, A + y.z_enc_n, A + y.h);
-  run(y.enc_e, E, 1, seg_of(n->xe, n->edge_in), none, none, nullptr, A + y.z_enc_e, A + y.e);
+  run(y.enc_n, N, 1, SegDev{n->xn, nullptr, n->node_in, net_ld(n->ld_xn, n->node_in), 0}, none, none, nullptr, A + y.z_enc_n, A + y.h);
+  run(y.enc_e, E, 1, SegDev{n->xe, nullptr, n->edge_in, net_ld(n->ld_xe, n->edge_in), 0}, none, none, nullptr, A + y.z_enc_e, A + y.e);
   for (int l = 0; l < y.L; l++) {
     const float *h = A + y.h + l * y.nh, *e = A + y.e + l * y.ne;
     float *e1 = A + y.e + (l + 1) * y.ne, *agg = A + y.agg + l * y.nh;
@@ -1474,7 +1478,7 @@ cfd_status cfd_mpnn_net_forward(const cfd_mpnn_net *n, void *stream) {
 }
 
 cfd_status cfd_mpnn_net_backward(const cfd_mpnn_net *n, void *stream) {
-  if (!net_ok(n) || !n->grads || !n->workspace || (n->n_nodes > 0 && (!n->dpred || !n->src_ptr)) ||
+  if (!net_ok(n) || !n->grads || !n->workspace || net_ld(n->ld_dpred, n->out) < n->out || (n->n_nodes > 0 && (!n->dpred || !n->src_ptr)) ||
       (n->n_edges > 0 && !n->src_order))
     return bad("cfd_mpnn_net_backward: bad argument");
   const NetLayout y(n->layers, n->node_in, n->edge_in, n->out, n->n_nodes, n->n_edges);
@@ -1483,7 +1487,7 @@ cfd_status cfd_mpnn_net_backward(const cfd_mpnn_net *n, void *stream) {
   float *A = n->act, *G = n->grads;
   const int N = n->n_nodes, E = n->n_edges;
   float *dh = A + y.dh, *de = A + y.de, *dagg = A + y.dagg, *dx = A + y.dx, *dz = A + y.dz;
-  auto wgrad = [&](int rows, int nout, const float *z, int K, int nseg, SegDev s0, SegDev s1, SegDev s2, size_t w,
+  auto wgrad = [&](int rows, int nout, const float *z, int ld_z, int K, int nseg, SegDev s0, SegDev s1, SegDev s2, size_t w,
                    size_t b, const float *ga, int ld_ga, const int *gidx) {
     WgArgs a{};
     a.M = rows;
@@ -1494,7 +1498,7 @@ cfd_status cfd_mpnn_net_backward(const cfd_mpnn_net *n, void *stream) {
     a.seg[1] = s1;
     a.seg[2] = s2;
     a.dz = z;
-    a.ld_dz = nout;
+    a.ld_dz = ld_z;
     a.partial = n->workspace;
     a.ga = ga;
     a.ld_ga = ld_ga;
@@ -1505,17 +1509,17 @@ cfd_status cfd_mpnn_net_backward(const cfd_mpnn_net *n, void *stream) {
   // Gradients of one block from its output gradient dy (+ the rows ga added through gidx): the
   // second layer's weights first (they read dy, which upd may overwrite), then the data path, then
   // the first layer's weights.
-  auto block = [&](const NetBlock &b, int rows, const float *dy, const float *z1, int nseg, SegDev s0, SegDev s1,
+  auto block = [&](const NetBlock &b, int rows, const float *dy, int ld_dy, const float *z1, int nseg, SegDev s0, SegDev s1,
                    SegDev s2, float *dxo, int ld_dx, float *upd, int upd_c0, const float *ga, int ld_ga,
                    const int *gidx) {
-    wgrad(rows, b.N, dy, HID, 1, seg_of(z1, HID, nullptr, 1), none, none, b.w2, b.b2, ga, ld_ga, gidx);
+    wgrad(rows, b.N, dy, ld_dy, HID, 1, seg_of(z1, HID, nullptr, 1), none, none, b.w2, b.b2, ga, ld_ga, gidx);
     if (rows > 0) {
       BwdArgs a{};
       a.M = rows;
       a.K = b.K;
       a.N2 = b.N;
       a.dy = dy;
-      a.ld_dy = b.N;
+      a.ld_dy = ld_dy;
       a.z1 = z1;
       a.w1 = P + b.w1;
       a.w2 = P + b.w2;
@@ -1530,25 +1534,25 @@ cfd_status cfd_mpnn_net_backward(const cfd_mpnn_net *n, void *stream) {
       a.upd_c0 = upd_c0;
       launch_mlp_bwd(a, s);
     }
-    wgrad(rows, HID, dz, b.K, nseg, s0, s1, s2, b.w1, b.b1, nullptr, 0, nullptr);
+    wgrad(rows, HID, dz, HID, b.K, nseg, s0, s1, s2, b.w1, b.b1, nullptr, 0, nullptr);
   };
-  block(y.dec, N, n->dpred, A + y.z_dec, 1, seg_of(A + y.h + y.L * y.nh, HID), none, none, dh, HID, nullptr, 0, nullptr,
+  block(y.dec, N, n->dpred, net_ld(n->ld_dpred, n->out), A + y.z_dec, 1, seg_of(A + y.h + y.L * y.nh, HID), none, none, dh, HID, nullptr, 0, nullptr,
         0, nullptr);
   if (E > 0) cudaMemsetAsync(de, 0, y.ne * sizeof(float), s);
   for (int l = y.L - 1; l >= 0; l--) {
     const float *h = A + y.h + l * y.nh, *e = A + y.e + l * y.ne, *agg = A + y.agg + l * y.nh;
     // Node block: dh += its input gradient's columns [0, 64); columns [64, 128) are the gradient of
     // agg, [N][64] rows of their own (the column offset taken off the pointer).
-    block(y.node(l), N, dh, A + y.z_node + l * y.nh, 2, seg_of(h, HID), seg_of(agg, HID), none, dagg - HID, HID, dh, 0,
+    block(y.node(l), N, dh, HID, A + y.z_node + l * y.nh, 2, seg_of(h, HID), seg_of(agg, HID), none, dagg - HID, HID, dh, 0,
           nullptr, 0, nullptr);
     // Edge block: its output gradient is de + dagg[dst].
-    block(y.edge(l), E, de, A + y.z_edge + l * y.ne, 3, seg_of(h, HID, n->src), seg_of(h, HID, n->dst), seg_of(e, HID),
+    block(y.edge(l), E, de, HID, A + y.z_edge + l * y.ne, 3, seg_of(h, HID, n->src), seg_of(h, HID, n->dst), seg_of(e, HID),
           dx, 3 * HID, de, 2 * HID, dagg, HID, n->dst);
     if (N > 0) k_edge_gather_bwd<<<(N + 7) / 8, 256, 0, s>>>(dx, 3 * HID, n->src_ptr, n->src_order, n->dst_ptr, N, dh);
   }
-  block(y.enc_e, E, de, A + y.z_enc_e, 1, seg_of(n->xe, n->edge_in), none, none, nullptr, 0, nullptr, 0, nullptr, 0,
+  block(y.enc_e, E, de, HID, A + y.z_enc_e, 1, SegDev{n->xe, nullptr, n->edge_in, net_ld(n->ld_xe, n->edge_in), 0}, none, none, nullptr, 0, nullptr, 0, nullptr, 0,
         nullptr);
-  block(y.enc_n, N, dh, A + y.z_enc_n, 1, seg_of(n->xn, n->node_in), none, none, nullptr, 0, nullptr, 0, nullptr, 0,
+  block(y.enc_n, N, dh, HID, A + y.z_enc_n, 1, SegDev{n->xn, nullptr, n->node_in, net_ld(n->ld_xn, n->node_in), 0}, none, none, nullptr, 0, nullptr, 0, nullptr, 0,
         nullptr);
   return status_of("cfd_mpnn_net_backward");
 }

@@ -413,7 +413,10 @@ class Net:
         """The library's description of one whole pass (cfd_mpnn_net)."""
         b = self._bufs
         a = cb.MpnnNet()
-        a.layers, a.node_in, a.edge_in, a.out = self.L, xn.shape[1], xe.shape[1], self.out
+        a.layers, a.node_in, a.edge_in, a.out = self.L, self.dims["enc_n"][0], self.dims["enc_e"][0], self.out
+        # A stride of 0 (expanded rows) is refused, where 0 would mean packed rows.
+        a.ld_xn, a.ld_xe = xn.stride(0) or -1, xe.stride(0) or -1
+        a.ld_dpred = (dpred.stride(0) or -1) if dpred is not None else 0
         a.n_nodes, a.n_edges = xn.shape[0], xe.shape[0]
         a.params, a.grads, a.workspace = self.flat.data_ptr(), self.grad.data_ptr(), self.workspace.data_ptr()
         a.xn, a.xe = xn.data_ptr(), xe.data_ptr()
@@ -429,6 +432,9 @@ class Net:
         N, E = xn.shape[0], xe.shape[0]
         b = self._buffers(N, E)
         if self.whole:
+            if (xn.shape[1], xe.shape[1]) != (self.dims["enc_n"][0], self.dims["enc_e"][0]):
+                raise ValueError("the network takes %d node and %d edge features, got %d and %d" % (
+                    self.dims["enc_n"][0], self.dims["enc_e"][0], xn.shape[1], xe.shape[1]))
             cb._check(cb.lib().cfd_mpnn_net_forward(ctypes.byref(self._net(xn, xe, gb)), _stream(xn)))
             self._graph = gb
             self._x = (xn, xe)

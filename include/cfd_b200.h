@@ -519,6 +519,7 @@ typedef struct {
   float *pred;                 /* out [n_nodes][out] */
   const float *dpred;          /* backward only */
   float *workspace;            /* backward only */
+  int ld_xn, ld_xe, ld_dpred;  /* row strides of xn, xe and dpred in elements, at least the width; 0: packed */
 } cfd_mpnn_net;
 size_t cfd_mpnn_net_floats(int layers, int node_in, int edge_in, int out, int n_nodes, int n_edges);
 cfd_status cfd_mpnn_net_forward(const cfd_mpnn_net *n, void *stream);
