@@ -31,13 +31,17 @@ struct Prim {  // the five primitive slots the fluxes read: Primitive_Cells[c][0
 //
 // Fast64: the same values without branches (every result is the correctly rounded one).
 //   Reciprocal: y0 = rcp.approx.ftz.f64(b) (PTX; relative error e about 2^-20), one third-order step
-//   y = y0 (1 + e + e^2).  Its error before rounding is e^3, so y = RN(1/b) unless 1/b lies next to a
-//   rounding boundary; of those b only 2^k (2 - 2^-52) matters for the quotients, and there RN(1/b),
-//   whose last mantissa bit is 1, is put in directly.
+//   y1 = y0 (1 + e + e^2), then one Newton step y = y1 + y1 (1 - b y1).  y1 is off by x <= 1/2 + e^3 2^53
+//   units u = 2^-53 of a b in [1, 2); the residual 1 - b y1 is exact and the Newton step's value before
+//   rounding is (1 - (b x u)^2) / b, so y = RN(1/b) unless the middle m of two numbers has
+//   0 < 1 - b m <= (b x u)^2 < 2 2^-106.  1 - b m is a multiple of 2^-106, so it would be 2^-106 itself;
+//   of the divisors of 2^106 - 1 only 2^53 - 1 lies in the range of b (2^52 .. 2^53), and for that one
+//   RN(1/b), whose last mantissa bit is 1, is put in directly.  Without the Newton step y1 is the wrong
+//   neighbour for many b just below a power of two, and one numerator of each then missed its quotient.
 //   Quotient: q = a y, then twice q + (a - b q) y.  The first pass leaves q within one unit in the last
-//   place, so the second residual is exact and its correction rounds correctly (P. Markstein,
-//   Computation of elementary functions on the IBM RISC System/6000, IBM J. Res. Dev. 34, 1990).
-//   Quotients by one denominator share its reciprocal.
+//   place, so the second residual is exact and its correction rounds correctly, y being RN(1/b)
+//   (P. Markstein, Computation of elementary functions on the IBM RISC System/6000, IBM J. Res. Dev. 34,
+//   1990).  Quotients by one denominator share its reciprocal.
 //   Square root: y0 = rsqrt.approx.ftz.f64(a); g = a y0 and h = y0 / 2 take the third-order step
 //   (1 + r + 3/2 r^2), r = 1/2 - g h; then g + (a - g^2) h.  sqrt(a) is nearer than that result's
 //   error to a rounding boundary only just below it (a = 1 - 2^-53, say), so the one correction left
@@ -76,6 +80,25 @@ struct Fast64 {
   static constexpr unsigned kNumLo = (1023u - 500u) << 20, kNumHi = (1023u + 500u) << 20;
   static constexpr unsigned kDenLo = (1023u - 400u) << 20, kDenHi = (1023u + 400u) << 20;
   unsigned nlo = ~0u, nhi = 0u, dlo = ~0u, dhi = 0u;
+  // A host program that includes this file brings its own model of the two seeds.
+  static __device__ __forceinline__ double rcp_seed(double b) {
+#ifdef __CUDACC__
+    double y;
+    asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(b));
+    return y;
+#else
+    return fast64_rcp_seed(b);
+#endif
+  }
+  static __device__ __forceinline__ double rsqrt_seed(double a) {
+#ifdef __CUDACC__
+    double y;
+    asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(a));
+    return y;
+#else
+    return fast64_rsqrt_seed(a);
+#endif
+  }
   __device__ __forceinline__ void num(double a) {
     const unsigned h = static_cast<unsigned>(__double2hiint(a)) & 0x7fffffffu;
     nlo = min(nlo, h - 1u);  // zero wraps to the largest value: allowed
@@ -103,10 +126,10 @@ struct Fast64 {
   }
   __device__ __forceinline__ Rcp rcp(double b) {
     den(b);
-    double y;
-    asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(b));
+    double y = rcp_seed(b);
     const double e = fma(-b, y, 1.0);
     y = fma(fma(e, e, e), y, y);
+    y = fma(fma(-b, y, 1.0), y, y);
     const bool ones = ((static_cast<unsigned>(__double2hiint(b)) | 0xfff00000u) &
                        static_cast<unsigned>(__double2loint(b))) == 0xffffffffu;
     return Rcp{b, __hiloint2double(__double2hiint(y), ones ? 1 : __double2loint(y))};
@@ -136,16 +159,12 @@ struct Fast64 {
     const double q = fma(a, yh, a * yl);
     return fma(-fma(kGM1, q, -a), yh, q);
   }
-  __device__ __forceinline__ double inv(double b) {
-    const Rcp r = rcp(b);
-    return fma(-fma(b, r.y, -1.0), r.y, r.y);
-  }
+  __device__ __forceinline__ double inv(double b) { return rcp(b).y; }
   __device__ __forceinline__ double root(double a) {
     const unsigned h = static_cast<unsigned>(__double2hiint(a));  // a set sign bit is above every bound
     nlo = min(nlo, h);
     nhi = max(nhi, h);
-    double y;
-    asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(a));
+    const double y = rsqrt_seed(a);
     const double g0 = a * y, h0 = 0.5 * y;
     const double r = fma(-g0, h0, 0.5);
     const double t = fma(1.5 * r, r, r);

@@ -1,0 +1,119 @@
+"""The branch-free division, reciprocal and square root of the flux functions and the functions built on
+them, operation by operation against the plain operators: on the CPU with seeds of the documented form
+(20 leading bits in and out, three roundings), on the GPU with its own.  The operands are the ones next to
+rounding boundaries, found from the congruences that define them, and the ends of the ranges."""
+import ctypes
+import os
+import random
+import subprocess
+
+import numpy as np
+import pytest
+
+from conftest import ROOT, assert_bits_equal
+
+SRC = os.path.join(ROOT, "tests", "fast64_ops.cu")
+CSRC = os.path.join(ROOT, "cfd_solver_withcuda_b200", "csrc")
+DP, IP = ctypes.POINTER(ctypes.c_double), ctypes.POINTER(ctypes.c_int)
+DIV, DIV_SIGNED, INV, ROOT_OP, DIV_GM1, SLOPE = 0, 1, 2, 3, 4, 10
+
+
+def _dp(a):
+    return a.ctypes.data_as(DP)
+
+
+class Ops:
+    def __init__(self, lib):
+        self.lib = lib
+
+    def __call__(self, k, a, b):
+        """(branch-free, plain, bad) of operation k on every (a, b)."""
+        a, b = (np.ascontiguousarray(x, np.float64) for x in np.broadcast_arrays(a, b))
+        f, p, bad = np.empty_like(a), np.empty_like(a), np.empty(a.shape, np.int32)
+        assert self.lib.ops_items(k, a.size, _dp(a), _dp(b), _dp(f), _dp(p), bad.ctypes.data_as(IP)) == 0
+        return f, p, bad.astype(bool)
+
+
+@pytest.fixture(scope="module")
+def host(tmp_path_factory):
+    out = str(tmp_path_factory.mktemp("ops") / "ops.so")
+    subprocess.check_call(["g++", "-x", "c++", "-std=c++17", "-O2", "-mfma", "-ffp-contract=off", "-fPIC", "-shared",
+                           "-I/usr/local/cuda/include", "-I" + CSRC, SRC, "-o", out])
+    return ctypes.CDLL(out)
+
+
+@pytest.fixture(scope="module")
+def device(tmp_path_factory):
+    from cfd_solver_withcuda_b200 import build
+    out = str(tmp_path_factory.mktemp("ops") / "ops_gpu.so")
+    subprocess.check_call([build.nvcc()] + build.ARCH + ["-std=c++17", "-O3", "--fmad=false", "-Xcompiler", "-fPIC",
+                                                         "-shared", "-I" + CSRC, SRC, "-o", out])
+    return Ops(ctypes.CDLL(out))
+
+
+@pytest.fixture(params=[0, 1, 2, pytest.param("gpu", marks=pytest.mark.gpu)])
+def ops(request):
+    """The operations with seeds rounded to nearest, down and up, and on the GPU."""
+    if request.param == "gpu":
+        return request.getfixturevalue("device")
+    lib = request.getfixturevalue("host")
+    lib.ops_seed_rounding(request.param)
+    return Ops(lib)
+
+
+def quotients_beside_boundaries(n):
+    """(a, b): b = 2^53 - d with the reciprocals next to a rounding boundary (d odd), a from the inverse of b
+    modulo 2^54, so that a / b lies one unit of 2^-105 / b from the middle of two numbers."""
+    rng = random.Random(1)
+    out = []
+    while len(out) < n:
+        b = 2 ** 53 - (rng.getrandbits(rng.randint(1, 45)) | 1)
+        inv = pow(b, -1, 2 ** 54)
+        for s in (1, -1):
+            m = (s * inv) % 2 ** 54
+            for shift in (53, 54):
+                if m >= 2 ** 53 and (b * m - s) % 2 ** shift == 0 and 2 ** 52 <= (b * m - s) >> shift < 2 ** 53:
+                    out.append(((b * m - s) >> shift, b))
+    return (np.array([x[i] for x in out], np.float64) for i in (0, 1))
+
+
+def test_quotients_beside_rounding_boundaries(ops):
+    a, b = quotients_beside_boundaries(100000)
+    for scale in (1.0, -2.0 ** -300):
+        f, p, bad = ops(DIV, a * scale, b * 2.0 ** 20)
+        assert not bad.any()
+        assert_bits_equal(f, p, "quotient")
+
+
+def test_reciprocals_beside_rounding_boundaries(ops):
+    """1 / b for b just below a power of two (1 / b next to the middle of two numbers), all mantissa bits set
+    among them, and for random b."""
+    rng = random.Random(2)
+    d = [1, 3, 5] + [rng.getrandbits(rng.randint(1, 45)) for _ in range(100000)]
+    b = np.array([2 ** 53 - x for x in d] + [rng.getrandbits(52) | 2 ** 52 for _ in range(100000)], np.float64)
+    f, p, bad = ops(INV, 1.0, b * 2.0 ** -60)
+    assert not bad.any()
+    assert_bits_equal(f, p, "reciprocal")
+
+
+def test_roots_beside_rounding_boundaries(ops):
+    """sqrt(a) nearest to the middle m of two numbers, m^2 = a + k 2^-106 for small k, in both binades."""
+    out = []
+    for bits in (54, 55):
+        for k in range(-257, 258):
+            if k % 8 != 1:
+                continue
+            x = 1  # x^2 = k modulo 2^bits, one more bit at a time
+            for j in range(3, bits):
+                if (x * x - k) % 2 ** (j + 1):
+                    x += 2 ** (j - 1)
+            for m in (x, -x, x + 2 ** (bits - 1), -x + 2 ** (bits - 1)):
+                m %= 2 ** bits
+                if 2 ** 53 < m < 2 ** 54 and (m * m - k) % 2 ** bits == 0 and 2 ** 52 <= (m * m - k) >> bits < 2 ** 53:
+                    out.append(float((m * m - k) >> bits) * 2.0 ** (bits - 106))
+    a = np.array(out)
+    assert a.size > 64
+    for e in (0, 40, -300):
+        f, p, bad = ops(ROOT_OP, 0.0, a * 2.0 ** e)
+        assert not bad.any()
+        assert_bits_equal(f, p, "root")
