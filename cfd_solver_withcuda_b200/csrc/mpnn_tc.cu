@@ -1055,11 +1055,13 @@ __global__ void __launch_bounds__(256) k_edge_gather_bwd(const float *__restrict
 
 // Mean-squared error: grad = 2 (pred - target) / n and loss = sum (pred - target)^2 / n.  Block 0 sums
 // the loss (each thread its stride of values, eight loads ahead of the additions, then a fixed-order
-// tree); the other blocks write the gradient.
-__global__ void __launch_bounds__(1024) k_mse(const float *pred, const float *target, int n, float *grad, float *loss) {
+// tree); the other blocks write the gradient.  A gradient written over its inputs (in_place) is block 0's
+// too, each value after its thread has read it.
+__global__ void __launch_bounds__(1024) k_mse(const float *pred, const float *target, int n, float *grad, float *loss,
+                                              bool in_place) {
   const float inv = 1.0f / (float)n;
   if (blockIdx.x > 0) {
-    const int i = (blockIdx.x - 1) * blockDim.x + threadIdx.x;
+    const long long i = (long long)(blockIdx.x - 1) * blockDim.x + threadIdx.x;
     if (i < n) {
       const float d = pred[i] - target[i];
       grad[i] = 2.0f * d * inv;
@@ -1068,8 +1070,8 @@ __global__ void __launch_bounds__(1024) k_mse(const float *pred, const float *ta
   }
   __shared__ float sh[1024];
   float s = 0.0f;
-  int i = threadIdx.x;
-  for (; (long long)i + 7 * 1024 < n; i += 8 * 1024) {
+  long long i = threadIdx.x;
+  for (; !in_place && i + 7 * 1024 < n; i += 8 * 1024) {
     float d[8];
 #pragma unroll
     for (int k = 0; k < 8; k++) d[k] = pred[i + k * 1024] - target[i + k * 1024];
@@ -1078,6 +1080,7 @@ __global__ void __launch_bounds__(1024) k_mse(const float *pred, const float *ta
   }
   for (; i < n; i += 1024) {
     const float d = pred[i] - target[i];
+    if (in_place) grad[i] = 2.0f * d * inv;
     s += d * d;
   }
   sh[threadIdx.x] = s;
@@ -1425,7 +1428,10 @@ cfd_status cfd_mpnn_segment_sum_acc(const float *x, int ldx, const int *ptr, con
 
 cfd_status cfd_mpnn_mse(const float *pred, const float *target, int n, float *grad, float *loss, void *stream) {
   if (n < 1 || !pred || !target || !grad || !loss) return bad("cfd_mpnn_mse: bad argument");
-  k_mse<<<1 + (n - 1) / 1024 + 1, 1024, 0, static_cast<cudaStream_t>(stream)>>>(pred, target, n, grad, loss);
+  auto overlaps = [&](const float *x) { return x < grad + n && grad < x + n; };
+  const bool in_place = overlaps(pred) || overlaps(target);
+  k_mse<<<in_place ? 1 : 1 + (n - 1) / 1024 + 1, 1024, 0, static_cast<cudaStream_t>(stream)>>>(pred, target, n, grad, loss,
+                                                                                           in_place);
   return status_of("cfd_mpnn_mse");
 }
 
