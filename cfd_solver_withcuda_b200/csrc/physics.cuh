@@ -99,9 +99,12 @@ struct Fast64 {
     return fast64_rsqrt_seed(a);
 #endif
   }
+  // The low word's last place tells zero (allowed: its word wraps to the largest value) from the subnormals
+  // below 2^-1042.
   __device__ __forceinline__ void num(double a) {
-    const unsigned h = static_cast<unsigned>(__double2hiint(a)) & 0x7fffffffu;
-    nlo = min(nlo, h - 1u);  // zero wraps to the largest value: allowed
+    const unsigned h = (static_cast<unsigned>(__double2hiint(a)) & 0x7fffffffu) |
+                       min(static_cast<unsigned>(__double2loint(a)), 1u);
+    nlo = min(nlo, h - 1u);
     nhi = max(nhi, h);
   }
   __device__ __forceinline__ void den(double b) {
@@ -109,7 +112,7 @@ struct Fast64 {
     dlo = min(dlo, h);
     dhi = max(dhi, h);
   }
-  // Numerators known to be 0 or positive.
+  // Numerators known to be 0 or positive with a high word that is not zero.
   __device__ __forceinline__ void num_pos(double a) {
     const unsigned h = static_cast<unsigned>(__double2hiint(a));
     nlo = min(nlo, h - 1u);
