@@ -51,8 +51,7 @@ struct Prim {  // the five primitive slots the fluxes read: Primitive_Cells[c][0
 // denominators 2^-400 .. 2^400, radicands 2^-500 .. 2^500 (positive).  Every operand's high word goes
 // into a running minimum and maximum; bad() tells that some operand was outside (infinities, NaN,
 // zero denominators, negative radicands among them), and the caller then evaluates the same item
-// again with Ieee.  Zero numerators keep their sign for positive denominators (div_signed flags them
-// for the others).
+// again with Ieee.  div keeps the sign of a zero numerator for positive denominators, div_signed for all.
 template <typename T>
 struct Ieee {
   static constexpr bool fast = false;
@@ -151,9 +150,13 @@ struct Fast64 {
     return quotient(a, rcp(b));
   }
   __device__ __forceinline__ double div(double a, double b) { return div(a, rcp(b)); }
+  // Denominators of either sign: the corrections lose the sign of a zero, which the operands' signs give.
+  // (Flagged, a face of gas at rest or of a stream along it, whose contact speed is zero, was evaluated
+  // twice: an HLLC solve from a uniform start.)
   __device__ __forceinline__ double div_signed(double a, double b) {
-    if (a == 0.0) flag();
-    return div(a, b);
+    const double q = div(a, b);
+    const int sign = (__double2hiint(a) ^ __double2hiint(b)) & 0x80000000;
+    return __hiloint2double((__double2hiint(q) & 0x7fffffff) | sign, __double2loint(q));
   }
   // a / (1.4 - 1.0): 1 / (1.4 - 1.0) as a sum of two doubles brings q within one unit at once.
   __device__ __forceinline__ double div_gm1(double a) {

@@ -133,3 +133,38 @@ def test_subnormal_numerators(ops):
         f, p, bad = ops(k, np.array([0.0, -0.0]), 3.0)
         assert not bad.any()
         assert_bits_equal(f, p, "zero")
+
+
+def test_signed_zero_quotients(ops):
+    """Zero numerators over denominators of either sign: IEEE's zero, not flagged."""
+    a = np.array([0.0, -0.0, 0.0, -0.0, 1.5, -1.5, 1.5, -1.5])
+    b = np.array([3.0, 3.0, -3.0, -3.0, 0.7, 0.7, -0.7, -0.7])
+    f, p, bad = ops(DIV_SIGNED, a, b)
+    assert not bad.any()
+    assert_bits_equal(f, p, "quotient")
+
+
+@pytest.mark.parametrize("case", ["rest", "aligned", "shear", "jump"])
+def test_hllc_of_uniform_states_is_evaluated_once(host, case):
+    """Faces with zero contact speeds or pressure jumps (gas at rest, uniform streams along the face, a
+    shear layer) and with jumps: the plain operators' flux without a second evaluation."""
+    host.ops_seed_rounding(0)
+    rng = np.random.default_rng(3)
+    n = 2000
+    th = rng.uniform(0, 2 * np.pi, n)
+    nrm = np.stack([np.cos(th), np.sin(th), rng.uniform(0.1, 2, n)], 1)
+    nrm[:8, :2] = [(1, 0), (-1, 0), (0, 1), (0, -1)] * 2
+    q = np.empty((n, 2, 4))
+    q[:, :, 0], q[:, :, 3] = 1.0, 1.0 / 1.4
+    q[:, :, 1:3] = 0.0
+    if case == "aligned":
+        q[:, :, 1:3] = 1.5 * np.stack([-nrm[:, 1], nrm[:, 0]], 1)[:, None]
+    if case == "shear":
+        q[:, 0, 1:3] = np.stack([-nrm[:, 1], nrm[:, 0]], 1)
+        q[:, 1, 0] = 2.0
+    if case == "jump":
+        q[:, 1, 0], q[:, 1, 3] = 0.125, 0.1
+    f, p, bad = np.empty((n, 4)), np.empty((n, 4)), np.empty(n, np.int32)
+    host.ops_hllc(n, _dp(q), _dp(nrm), _dp(f), _dp(p), bad.ctypes.data_as(IP))
+    assert not bad.any()
+    assert_bits_equal(f, p, "flux")
