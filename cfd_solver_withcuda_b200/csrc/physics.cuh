@@ -111,12 +111,6 @@ struct Fast64 {
     dlo = min(dlo, h);
     dhi = max(dhi, h);
   }
-  // Numerators known to be 0 or positive with a high word that is not zero.
-  __device__ __forceinline__ void num_pos(double a) {
-    const unsigned h = static_cast<unsigned>(__double2hiint(a));
-    nlo = min(nlo, h - 1u);
-    nhi = max(nhi, h);
-  }
   __device__ __forceinline__ void flag() { dlo = 0u; }
   // Flags values that are not positive (their sign bit or a zero high word; NaN is flagged where it is
   // used).
@@ -144,10 +138,6 @@ struct Fast64 {
   __device__ __forceinline__ double div(double a, const Rcp &r) {
     num(a);
     return quotient(a, r);
-  }
-  __device__ __forceinline__ double div_pos(double a, double b) {
-    num_pos(a);
-    return quotient(a, rcp(b));
   }
   __device__ __forceinline__ double div(double a, double b) { return div(a, rcp(b)); }
   // Denominators of either sign: the corrections lose the sign of a zero, which the operands' signs give.
@@ -619,13 +609,14 @@ __device__ __forceinline__ T muscl_slope(int kind, T a, T b) {
 
 // Half of muscl_slope of a Fast64 evaluation: the Van Leer and van Albada quotients without branches (where
 // the slope is zero the quotient is 0 / 1), the others as they are.  Halving Van Leer's 2ab / (a + b)
-// cancels its 2: both are exact.  ab > 0 is read off its high word (products below 2^-1042 count as 0).
+// cancels its 2: both are exact.  The tests are muscl_slope's, so that a NaN difference (a gradient next to
+// a non-physical cell) reaches the quotient, which flags it.
 template <int KIND>
 __device__ __forceinline__ double muscl_half_slope(Fast64 &o, double a, double b) {
   if (KIND == LIM_VANLEER || KIND == LIM_VANALBADA) {
     const double ab = a * b;
-    const bool on = !(fabs(b) < 1e-12) && __double2hiint(ab) > 0;
-    if (KIND == LIM_VANLEER) return o.div_pos(on ? ab : 0.0, on ? a + b : 1.0);
+    const bool on = !(fabs(b) < 1e-12) && !(ab <= 0.0);
+    if (KIND == LIM_VANLEER) return o.div(on ? ab : 0.0, on ? a + b : 1.0);
     const double a2 = a * a;
     return 0.5 * o.div(on ? b * (a2 + ab) : 0.0, on ? a2 + b * b : 1.0);
   }

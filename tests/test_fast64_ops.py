@@ -168,3 +168,19 @@ def test_hllc_of_uniform_states_is_evaluated_once(host, case):
     host.ops_hllc(n, _dp(q), _dp(nrm), _dp(f), _dp(p), bad.ctypes.data_as(IP))
     assert not bad.any()
     assert_bits_equal(f, p, "flux")
+
+
+@pytest.mark.parametrize("limiter", [1, 2, 4])  # MinMod, Van Leer, van Albada
+def test_limited_slopes_of_special_values(ops, limiter):
+    """NaN of either sign (a neighbour's gradient after its state has become non-physical), infinities,
+    zeros, products that underflow and ordinary differences: the plain operators' slope, or the flag."""
+    v = np.array([0.0, 1e-13, 1e-12, 2e-12, 1e-5, 0.3, 1.0, 7.0, 1e-150, 1e-160, 1e-304, 5e-324, 1e160, 1e308, np.inf])
+    v = np.concatenate([v, -v, np.array([0x7ff8000000000000, 0x7fffffffffffffff], np.int64).view(np.float64),
+                        np.array([0xfff8000000000000, 0xffffffffffffffff], np.uint64).view(np.float64)])
+    a, b = (x.ravel() for x in np.meshgrid(v, v))
+    f, p, bad = ops(SLOPE + limiter, a, b)
+    f = np.where(bad, p, f)
+    assert np.array_equal(np.isnan(f), np.isnan(p))
+    assert_bits_equal(np.where(np.isnan(p), 0.0, f), np.where(np.isnan(p), 0.0, p), "slope")
+    ordinary = (np.abs(a) < 10) & (np.abs(b) < 10) & (np.abs(a * b) > 1e-140)
+    assert not bad[ordinary].any()
