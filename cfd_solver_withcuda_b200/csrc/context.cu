@@ -365,7 +365,8 @@ struct cfd_ctx {
   int lean_graph_launches = 0;
   // Persistent batched form (option "persistent"): one cooperative launch per RK stage, one
   // CUDA graph per stage; persist_grid = co-resident blocks used; persist_test_arrivals = barrier
-  // arrivals that never come (option "barrier_timeout_test", a test of the timeout path).
+  // arrivals that never come, here and in the one-launch forms (option "barrier_timeout_test", a test
+  // of the timeout path).
   bool persistent = false;
   int persist_grid = 0;
   int partial_blocks = 0;  // blocks the reduction buffers (st.partial) are sized for
@@ -1475,8 +1476,8 @@ cfd_status cfd_set_option(cfd_ctx *ctx, const char *name, double value) {
     return CFD_OK;
   }
   if (n == "barrier_timeout_test") {
-    // Test of the bounded barrier: every barrier of the persistent form waits for `value` more
-    // arrivals than the grid has, so each wait runs out and the run reports CFD_ERR_TIMEOUT.
+    // Test of the bounded barriers: every barrier of the persistent and one-launch forms waits for `value`
+    // more arrivals than it has blocks, so the first wait runs out and the run reports CFD_ERR_TIMEOUT.
     drop_graphs(ctx);
     ctx->persist_test_arrivals = value > 0.0 ? static_cast<unsigned int>(value) : 0u;
     return CFD_OK;
@@ -1655,7 +1656,7 @@ static cfd_status enqueue_steps(cfd_ctx *ctx, int n_steps) {
     }
     if (ctx->steps.blocks > 0) return enqueue_steps_one_launch(ctx, n_steps, false);
   }
-  if (ctx->dm.cblk && ctx->steps.blocks > 0 && ctx->persist_test_arrivals == 0 && one_launch_form(ctx))
+  if (ctx->dm.cblk && ctx->steps.blocks > 0 && one_launch_form(ctx))
     return enqueue_steps_one_launch(ctx, n_steps, true);
   if (ctx->persistent && ctx->persist_grid > 0 && ctx->dm.NF > 0) return enqueue_steps_persistent(ctx, n_steps);
   // Every step but the last leaves out what the next one overwrites, unless a t_end may make any the last.

@@ -245,8 +245,8 @@ cfd_status cfd_sync(cfd_ctx *ctx, cfd_step_info *info);
  * forms with a per-cell dt frozen per step, of at most 98,304 cells -- a batch's active instances
  * together -- and the per-cell forms without WENO whose four lanes per cell fit the chip; default 1,
  * 0: the separate kernels),
- * "barrier_timeout_test" (a test of the bounded barriers: every barrier of the persistent form
- * waits for `value` more blocks than it has, so each wait runs out and the step reports
+ * "barrier_timeout_test" (a test of the bounded barriers: every barrier of the persistent and one-launch
+ * forms waits for `value` more blocks than it has, so the first wait runs out and the call reports
  * CFD_ERR_TIMEOUT; default 0),
  * "tile_stage" (with reorder 4 on a structured block, the gradient-MUSCL forms with a per-cell dt
  * frozen per step and three stages (CFD_INT_SSPRK3, CFD_INT_RK3_GPU_REF with local time stepping)
