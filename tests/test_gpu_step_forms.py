@@ -1,0 +1,100 @@
+"""The forms a call of several pseudo-steps can take, each forced by its options and compared with the others:
+the many-step kernels, the separate kernels with what the next step overwrites left out, single full steps,
+and the persistent stage kernel; every boundary kind through every source of boundary values."""
+import numpy as np
+import pytest
+
+import cfd_solver_withcuda_b200 as cb
+from cases import CASES, initial_state, make_mesh, solver_config
+from conftest import assert_bits_equal
+from test_gpu_batch import config, ramp_case
+from test_gpu_parity import ADDITIVE, OPTION_SETS
+
+pytestmark = pytest.mark.gpu
+
+SEPARATE = dict(one_launch_steps=0)
+FORMS = {"gradient": dict(muscl=1, is_second_order=1, dissipation_type=3, limiter=2, integrator=2,
+                          local_time_stepping=1),
+         "gradient_fp32_hllc": dict(muscl=1, is_second_order=1, dissipation_type=7, limiter=1, integrator=3,
+                                    local_time_stepping=1, precision=cb.PREC_FP32_FLUX),
+         "per_cell": dict(is_second_order=1, dissipation_type=3),
+         "per_cell_lts": dict(is_second_order=0, dissipation_type=1, integrator=2, local_time_stepping=1)}
+
+
+@pytest.mark.parametrize("form", sorted(FORMS))
+@pytest.mark.parametrize("inlet,outlet", [(1, 1), (1, 3), (4, 3), (4, 1), (2, 2), (3, 0)])
+def test_boundary_kinds_in_every_form(form, inlet, outlet):
+    m = cb.Mesh.bump(31, 14, 3.0, 1.0, 0.1, 4, 0.3, 7, True)
+    NP = m.n_physical
+    rng = np.random.default_rng(4)
+    f = lambda: 1.0 + 0.01 * rng.normal(size=NP)
+    U = np.zeros((m.n_total, 4))
+    U[:NP] = cb.conserved_from_primitive(f(), 0.6 * f(), 0.01 * rng.normal(size=NP), f() / 1.4)
+    U[m.boundary[:, 3]] = U[m.boundary[:, 1]]
+    kw = dict(FORMS[form], time_accurate=1, cfl=0.3, reorder=1, inlet_bc=inlet, exit_bc=outlet, inlet_rho=1.0,
+              inlet_u=0.6, inlet_v=0.01, inlet_p=1.0 / 1.4, inlet_p0=0.97, inlet_t0=0.0027, exit_p=0.99 / 1.4, r_gas=287.0)
+    got = []
+    for opts, calls in (({}, (9, 2)), (SEPARATE, (9, 2)), (dict(SEPARATE, use_graph=0), (1,) * 11)):
+        s = cb.Solver(m, cb.default_config(**kw))
+        for k, v in opts.items():
+            s.set_option(k, v)
+        s.upload_state(U)
+        for n in calls:
+            i = s.step(n)
+        got.append((s.download(), (i.iterations, i.min_dt, i.total_time), s.kernel_launches))
+        s.close()
+    assert got[0][2] < got[1][2]  # the many-step kernel ran
+    for d, i, _ in got[1:]:
+        assert i == got[0][1]
+        for k in ("U", "prim", "dt", "net_flux", "delU"):
+            assert_bits_equal(got[0][0][k], d[k], k)
+
+
+@pytest.mark.parametrize("form", ["grad_muscl_minmod_ssp_lts", "grad_muscl_ausm_fp32_ssp_lts", "grad_muscl_hllc_minmod"])
+def test_launch_options_of_the_separate_kernels(form):
+    """Fused gather, face-kernel shapes, graphs, programmatic launch and the L2 window, with the many-step
+    kernel off: the bits of the default options, which take that kernel where the form allows it."""
+    case = CASES["cyl_roe2_lts"]
+    m = make_mesh(case)
+    U0 = initial_state(case, m)
+    want, launches = None, []
+    for opts in [{}, SEPARATE] + [dict(o, **SEPARATE) for o in OPTION_SETS]:
+        s = cb.Solver(m, solver_config(case, **ADDITIVE[form]))
+        for k, v in opts.items():
+            s.set_option(k, v)
+        s.upload_state(U0)
+        n0 = s.kernel_launches
+        s.step(12)
+        launches.append(s.kernel_launches - n0)
+        d = s.download()
+        s.close()
+        want = want or d
+        for k in ("U", "prim", "dt", "net_flux", "delU"):
+            assert_bits_equal(d[k], want[k], "%s %s" % (k, opts))
+    assert min(launches[1:]) >= 12 * 3 * 3  # three kernels per stage at least
+    if "ssp_lts" in form:
+        assert launches[0] < 12
+
+
+@pytest.mark.parametrize("minb", [0, 4, 6, 8])
+@pytest.mark.parametrize("precision", [cb.PREC_FP64, cb.PREC_FP32_FLUX])
+def test_persistent_stage_kernel_of_a_batch(precision, minb):
+    """The persistent stage kernel (many-step kernel off) with every register budget: the bits of the
+    separate kernels, instances freezing in the middle of the run."""
+    specs = [(24, 12, 1.5), (64, 32, 2.2), (16, 8, 3.0), (40, 24, 2.6), (12, 6, 2.0)]
+    cases = [ramp_case(*sp) for sp in specs]
+    out = []
+    for persistent in (0, 1):
+        b = cb.Batch([c[0] for c in cases], config(precision=precision, limiter=cb.LIM_MINMOD),
+                     inflow=[c[2] for c in cases])
+        for k, v in dict(SEPARATE, persistent=persistent, persist_minb=minb).items():
+            b.set_option(k, v)
+        b.upload_state([c[1] for c in cases])
+        res = b.run(max_steps=1500, tol=1e-4, check_every=50)
+        out.append((res, b.download_state()))
+        b.close()
+    (r0, u0), (r1, u1) = out
+    assert np.array_equal(r0["steps_to_tol"], r1["steps_to_tol"]) and (r0["steps_to_tol"] > 0).any()
+    assert np.array_equal(r0["res_ratio"].view(np.int64), r1["res_ratio"].view(np.int64))
+    for a, b_ in zip(u0, u1):
+        assert_bits_equal(b_, a, "instance")
