@@ -359,6 +359,8 @@ def run_ramps(args, rank, world):
                "dtype": "f64", "data": "synthetic (seeded ramp generator, freestream start)",
                "config": {"workload": "batched_ramps_15deg", "instances": args.instances, "seed": args.seed,
                           "persistent": bool(args.persistent),
+                          "form": ("persistent stage kernel" if args.persistent else "three kernels per stage") +
+                          "; whole pseudo-steps in one launch once the active instances fit one",
                           "tol": args.tol, "max_steps": args.max_steps, "vl_steps": args.vl_steps,
                           "check_every": args.check_every,
                           "total_cells": int(sum(nx * ny for nx, ny, _ in specs)),

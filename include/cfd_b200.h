@@ -238,7 +238,8 @@ cfd_status cfd_sync(cfd_ctx *ctx, cfd_step_info *info);
  * the device maximum; it is never lowered and lasts as long as the process's CUDA context),
  * "persistent" (face-based forms with a per-cell dt: each RK stage as one persistent cooperative
  * kernel over the cells, faces and cells again, with bounded grid barriers between the phases and
- * one CUDA graph per RK stage; default 0; the batched solves' form, see cfd_batch_set_option),
+ * one CUDA graph per RK stage; default 0; a single solve then takes it in place of "one_launch_steps";
+ * for batches see cfd_batch_set_option),
  * "persist_minb" (the persistent kernel's register budget: built for 4, 6 or 8 resident blocks per
  * SM; default 0: 6 in FP64 and 8 in the FP32-flux form, the faster of each on B200),
  * "one_launch_steps" (multi-step calls run many pseudo-steps in one cooperative launch: the face-based
@@ -413,10 +414,13 @@ cfd_status cfd_batch_download_state(cfd_batch *b, double *U);
  * actually advanced.  Any output pointer may be NULL. */
 cfd_status cfd_batch_run(cfd_batch *b, int max_steps, double tol, int check_every, int *steps_to_tol,
                          double *time_to_tol, double *res_ratio, long long *cell_updates, int *steps_done);
-/* Run-time options of the batch's solver context (cfd_set_option), e.g. "persistent" = 1: each RK
- * stage of every instance runs as one persistent cooperative kernel over the (instance, block)
- * work lists, bounded grid barriers between its phases, one CUDA graph per RK stage (results
- * bit-identical to the three-kernel form; CFD_ERR_TIMEOUT when a barrier wait runs out).
+/* Run-time options of the batch's solver context (cfd_set_option).  A batch whose active instances fit
+ * one launch runs whole pseudo-steps in it ("one_launch_steps", the fastest form, whatever "persistent"
+ * says; a batch comes into it when enough instances have stopped).  Others, and all with
+ * "one_launch_steps" = 0: "persistent" = 1 runs each RK stage of every instance as one persistent
+ * cooperative kernel over the (instance, block) work lists, bounded grid barriers between its phases,
+ * one CUDA graph per RK stage (results bit-identical to the three-kernel form; CFD_ERR_TIMEOUT when a
+ * barrier wait runs out); 0: the three kernels per stage.
  * "divergence_ratio" = x > 0: in cfd_batch_run an instance whose residual ratio exceeds x at a
  * check stops updating and gets steps_to_tol = -2 (residual growth; 0 = never). */
 cfd_status cfd_batch_set_option(cfd_batch *b, const char *name, double value);
