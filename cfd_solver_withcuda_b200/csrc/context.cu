@@ -2057,7 +2057,9 @@ cfd_status cfd_amr_tags(cfd_ctx *ctx, double threshold, double max_fraction, dou
 // Autotuner: times each combination of the launch options that never change a result bit
 // (face-kernel shape, fused gather + stage, per-cell flux lanes) over `steps` graph-replayed
 // pseudo-steps of this context's own mesh and state, keeps the fastest, and restores the state
-// (every candidate starts from the same state; the solve is not advanced).
+// (every candidate starts from the same state; the solve is not advanced).  The face-based candidates
+// are timed as separate kernels, which their options are about; where the one-launch form applies it is
+// timed beside them, and stays on when it is faster than the best of them.
 cfd_status cfd_autotune(cfd_ctx *ctx, int steps, char *report, size_t report_len) {
   if (!ctx || steps < 1) return fail(CFD_ERR_BAD_ARG, "bad argument");
   DevState &st = ctx->ds;
@@ -2107,15 +2109,15 @@ cfd_status cfd_autotune(cfd_ctx *ctx, int steps, char *report, size_t report_len
     }
     cands.push_back({ctx->fp.faces_shape, ctx->fuse_gather, 4, ctx->dm.pdl, 0, 1, 0, 0.0});
   }
-  const int prof = ctx->profile, graph_on = ctx->use_graph;
+  const int prof = ctx->profile, graph_on = ctx->use_graph, steps_off = ctx->steps_off;
+  if (ctx->dm.NF > 0) ctx->steps_off = 1;
   ctx->profile = 0;
   ctx->use_graph = 1;
   cudaEvent_t e0, e1;
   cudaEventCreate(&e0);
   cudaEventCreate(&e1);
   copy_all(true);
-  cfd_status status = CFD_OK;
-  for (Cand &cd : cands) {
+  auto use = [&](const Cand &cd) {
     ctx->fp.faces_shape = cd.faces_shape;
     ctx->fuse_gather = cd.fuse;
     ctx->fp.lanes = cd.lanes;
@@ -2124,17 +2126,36 @@ cfd_status cfd_autotune(cfd_ctx *ctx, int steps, char *report, size_t report_len
     ctx->fp.flux_minb = cd.minb;
     ctx->tile_stage = cd.tile;
     drop_graphs(ctx);
+  };
+  auto time_steps = [&](double *per_step) -> cfd_status {
+    cfd_status s;
     ctx->launches += launch_set_ctl(ctx->stream, st, CTL_TEND, 0.0);
     ctx->launches += launch_set_ctl(ctx->stream, st, CTL_DONE, 0.0);
-    if ((status = enqueue_steps(ctx, 2)) != CFD_OK) break;
+    if ((s = enqueue_steps(ctx, 2)) != CFD_OK) return s;
     cudaEventRecord(e0, ctx->stream);
-    if ((status = enqueue_steps(ctx, steps)) != CFD_OK) break;
+    if ((s = enqueue_steps(ctx, steps)) != CFD_OK) return s;
     cudaEventRecord(e1, ctx->stream);
-    if ((status = sync_status(ctx, nullptr)) != CFD_OK) break;
+    if ((s = sync_status(ctx, nullptr)) != CFD_OK) return s;
     float ms = 0.f;
     cudaEventElapsedTime(&ms, e0, e1);
-    cd.ms = ms / steps;
+    *per_step = ms / steps;
     copy_all(false);
+    return CFD_OK;
+  };
+  cfd_status status = CFD_OK;
+  for (Cand &cd : cands) {
+    use(cd);
+    if ((status = time_steps(&cd.ms)) != CFD_OK) break;
+  }
+  double one_launch_ms = -1.0;
+  ctx->steps_off = steps_off;
+  if (status == CFD_OK && ctx->dm.NF > 0 && steps > 1 && graph_on && !prof && !ctx->persistent) {
+    use(cands[2]);  // any fused candidate of the three kernels: the form ignores the rest
+    if (one_launch_form(ctx)) {
+      double ms = -1.0;
+      status = time_steps(&ms);
+      if (ctx->steps.blocks > 0) one_launch_ms = ms;
+    }
   }
   copy_all(false);
   cudaStreamSynchronize(ctx->stream);
@@ -2148,13 +2169,15 @@ cfd_status cfd_autotune(cfd_ctx *ctx, int steps, char *report, size_t report_len
   const Cand *best = &cands[0];
   for (const Cand &cd : cands)
     if (cd.ms < best->ms) best = &cd;
-  ctx->fp.faces_shape = best->faces_shape;
-  ctx->fuse_gather = best->fuse;
-  ctx->fp.lanes = best->lanes;
-  ctx->dm.pdl = best->pdl;
-  ctx->patch_stage = best->patch;
-  ctx->fp.flux_minb = best->minb;
-  ctx->tile_stage = best->tile;
+  const bool one_launch = one_launch_ms >= 0.0 && one_launch_ms < best->ms;
+  if (one_launch) {  // the options of single steps, among those that leave the form available
+    best = nullptr;
+    for (const Cand &cd : cands)
+      if (cd.fuse && !cd.patch && !cd.tile && (!best || cd.ms < best->ms)) best = &cd;
+  } else if (one_launch_ms >= 0.0) {
+    ctx->steps_off = 1;
+  }
+  use(*best);
   if (report && report_len > 0) {
     std::string r;
     char line[160];
@@ -2163,6 +2186,11 @@ cfd_status cfd_autotune(cfd_ctx *ctx, int steps, char *report, size_t report_len
                "faces_shape=%d fuse_gather=%d flux_lanes=%d pdl=%d patch_stage=%d flux_minb=%d tile_stage=%d: %.4f "
                "ms/step%s\n",
                cd.faces_shape, cd.fuse, cd.lanes, cd.pdl, cd.patch, cd.minb, cd.tile, cd.ms, &cd == best ? " (chosen)" : "");
+      r += line;
+    }
+    if (one_launch_ms >= 0.0) {
+      snprintf(line, sizeof(line), "one_launch_steps=1: %.4f ms a step%s\n", one_launch_ms,
+               one_launch ? " (kept for calls of several steps)" : " (turned off)");
       r += line;
     }
     snprintf(report, report_len, "%s", r.c_str());

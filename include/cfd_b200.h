@@ -266,7 +266,9 @@ cfd_status cfd_sync(cfd_ctx *ctx, cfd_step_info *info);
 cfd_status cfd_set_option(cfd_ctx *ctx, const char *name, double value);
 /* Times every combination of the options above that applies to this configuration over `steps`
  * pseudo-steps of the context's own mesh and state, keeps the fastest and restores the state
- * (the solve is not advanced).  report (may be NULL) receives one line per candidate. */
+ * (the solve is not advanced).  The face-based forms are tuned as separate kernels; where
+ * "one_launch_steps" applies it is timed beside them and stays on if it is faster than all of them.
+ * report (may be NULL) receives one line per candidate. */
 cfd_status cfd_autotune(cfd_ctx *ctx, int steps, char *report, size_t report_len);
 
 /* Entry points of the reference path, one call each, same semantics and post-conditions. */

@@ -98,3 +98,21 @@ def test_persistent_stage_kernel_of_a_batch(precision, minb):
     assert np.array_equal(r0["res_ratio"].view(np.int64), r1["res_ratio"].view(np.int64))
     for a, b_ in zip(u0, u1):
         assert_bits_equal(b_, a, "instance")
+
+
+def test_autotune_times_the_separate_kernels_and_the_many_step_kernel():
+    """The candidates of a small frozen-dt solve differ in options the many-step kernel ignores: each runs as
+    separate kernels, and the many-step kernel has its own line."""
+    case = CASES["cyl_roe2_lts"]
+    m = make_mesh(case)
+    s = cb.Solver(m, solver_config(case, **ADDITIVE["grad_muscl_minmod_ssp_lts"]))
+    s.upload_state(initial_state(case, m))
+    steps, n0 = 10, s.kernel_launches
+    report = s.autotune(steps=steps)
+    assert report.count("ms/step") == 20 and report.count("(chosen)") == 1
+    assert s.kernel_launches - n0 >= 20 * (2 + steps) * 9
+    kept = "kept for calls of several steps" in report
+    assert kept or "one_launch_steps=1" in report and "turned off" in report
+    n0 = s.kernel_launches
+    s.step(steps)
+    assert (s.kernel_launches - n0 < steps) == kept
