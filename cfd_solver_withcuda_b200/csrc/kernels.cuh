@@ -230,7 +230,7 @@ int launch_persistent_stage(cudaStream_t s, const DevMesh &m, DevState &st, cons
                             int with_dt, int with_bc, int grid, unsigned int test_arrivals);
 // Whole pseudo-steps of the face-based forms with a dt frozen per step in one cooperative launch (k_steps).
 // steps_shape: the launch for `instances` solves over the cell and face ranges inst[i] (x, y; z, w), and
-// its blocks' shares; blocks = 0 when the separate kernels are the faster ones or the launch is not
+// its blocks' shares; blocks = 0 when a share does not fit a block's shared memory or the launch is not
 // available.  bptr: the cells' boundary-entry offsets (host copy).  cells, faces, entries: shared-memory
 // capacity per block.
 struct StepsBlock {
@@ -240,7 +240,6 @@ struct StepsBlock {
 struct StepsShape {
   int blocks, threads, groups, cells, faces, entries;
 };
-constexpr int kStepsCells = 98304;       // most cells of one launch, all instances together
 constexpr int kStepsPerLaunch = 128;     // bounds a launch's run time to a few milliseconds
 constexpr int kStepsBarrierStride = 32;  // a group's arrival count has its own 128 bytes
 StepsShape steps_shape(const FluxParams &fp, const int *bptr, const int4 *inst, int instances,

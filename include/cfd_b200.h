@@ -243,8 +243,8 @@ cfd_status cfd_sync(cfd_ctx *ctx, cfd_step_info *info);
  * "persist_minb" (the persistent kernel's register budget: built for 4, 6 or 8 resident blocks per
  * SM; default 0: 6 in FP64 and 8 in the FP32-flux form, the faster of each on B200),
  * "one_launch_steps" (multi-step calls run many pseudo-steps in one cooperative launch: the face-based
- * forms with a per-cell dt frozen per step, of at most 98,304 cells -- a batch's active instances
- * together -- and the per-cell forms without WENO whose four lanes per cell fit the chip; default 1,
+ * forms with a per-cell dt frozen per step whose cells and faces fit the shared memory of one block per
+ * SM -- about 101,000 cells, a batch's active instances together -- and the per-cell forms without WENO whose four lanes per cell fit the chip; default 1,
  * 0: the separate kernels),
  * "barrier_timeout_test" (a test of the bounded barriers: every barrier of the persistent and one-launch
  * forms waits for `value` more blocks than it has, so the first wait runs out and the call reports

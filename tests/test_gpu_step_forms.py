@@ -116,3 +116,46 @@ def test_autotune_times_the_separate_kernels_and_the_many_step_kernel():
     n0 = s.kernel_launches
     s.step(steps)
     assert (s.kernel_launches - n0 < steps) == kept
+
+
+@pytest.mark.parametrize("nx,fits", [(395, True), (400, False)])
+def test_capacity_of_the_many_step_kernel(nx, fits):
+    """The largest shares that fit 148 blocks' shared memory (101,120 cells) and the first that do not."""
+    m = cb.Mesh.box(nx, 256, 0.0, 2.0, 0.0, 1.0)
+    NP = m.n_physical
+    x = m.centers[:NP]
+    U = np.zeros((m.n_total, 4))
+    U[:NP] = cb.conserved_from_primitive(1 + 0.02 * np.sin(7 * x[:, 0]), 2 + 0.02 * np.cos(5 * x[:, 1]), 0 * x[:, 0],
+                                         (1 + 0.01 * np.sin(9 * x[:, 1])) / 1.4)
+    U[m.boundary[:, 3]] = U[m.boundary[:, 1]]
+    kw = dict(FORMS["gradient"], time_accurate=1, cfl=0.4, inlet_bc=3, inlet_rho=1.0, inlet_u=2.0, inlet_p=1.0 / 1.4,
+              reorder=4)
+    got = []
+    for on in (1, 0):
+        s = cb.Solver(m, cb.default_config(**kw))
+        s.set_option("one_launch_steps", on)
+        s.upload_state(U)
+        n0 = s.kernel_launches
+        s.step(6)
+        got.append((s.download(), s.kernel_launches - n0))
+        s.close()
+    assert (got[0][1] < 6) == fits and got[1][1] >= 6 * 9
+    for k in ("U", "prim", "dt", "net_flux", "delU"):
+        assert_bits_equal(got[0][0][k], got[1][0][k], k)
+
+
+def test_batch_up_to_the_capacity():
+    """49 channels of 64 x 32 cells (100,352) run in one launch, 50 (two blocks each, too large a share) do
+    not; every instance has the separate kernels' bits."""
+    m, U0, q = ramp_case(64, 32, 2.2)
+    for n in (49, 50):
+        out = []
+        for on in (1, 0):
+            b = cb.Batch([m] * n, config(limiter=cb.LIM_MINMOD), inflow=[q] * n)
+            b.set_option("one_launch_steps", on)
+            b.upload_state([U0 * (1.0 + 0.001 * i) for i in range(n)])
+            b.run(max_steps=9, tol=0.0, check_every=8)
+            out.append(b.download_state())
+            b.close()
+        for x, y in zip(*out):
+            assert_bits_equal(x, y, "instance")
