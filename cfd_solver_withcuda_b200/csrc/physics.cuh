@@ -30,7 +30,7 @@ struct Prim {  // the five primitive slots the fluxes read: Primitive_Cells[c][0
 // 43.7 instead of 52.8, the HLLC faces of 1,038,240 mixed cells 62.9 instead of 73.3 (B200).
 //
 // Fast64: the same values without branches (every result is the correctly rounded one).
-//   Reciprocal: y0 = rcp.approx.ftz.f64(b) (PTX; relative error e about 2^-20), one third-order step
+//   Reciprocal: y0 = rcp.approx.ftz.f64(b) (PTX; relative error e below 2^-19, tested), one third-order step
 //   y1 = y0 (1 + e + e^2), then one Newton step y = y1 + y1 (1 - b y1).  y1 is off by x <= 1/2 + e^3 2^53
 //   units u = 2^-53 of a b in [1, 2); the residual 1 - b y1 is exact and the Newton step's value before
 //   rounding is (1 - (b x u)^2) / b, so y = RN(1/b) unless the middle m of two numbers has
@@ -43,9 +43,10 @@ struct Prim {  // the five primitive slots the fluxes read: Primitive_Cells[c][0
 //   (P. Markstein, Computation of elementary functions on the IBM RISC System/6000, IBM J. Res. Dev. 34,
 //   1990).  Quotients by one denominator share its reciprocal.
 //   Square root: y0 = rsqrt.approx.ftz.f64(a); g = a y0 and h = y0 / 2 take the third-order step
-//   (1 + r + 3/2 r^2), r = 1/2 - g h; then g + (a - g^2) h.  sqrt(a) is nearer than that result's
-//   error to a rounding boundary only just below it (a = 1 - 2^-53, say), so the one correction left
-//   is to the next smaller number p, when a <= p g (B. Tuckerman's test).
+//   (1 + r + 3/2 r^2), r = 1/2 - g h; then g + (a - g^2) h.  That is off by less than 2^-104 before
+//   rounding, and the middle m of two numbers has m^2 - a = k 2^-106 with k = 1 modulo 8: the test goes
+//   through the a with |k| <= 257.  sqrt(a) just below m (k = 1; a = 1 - 2^-53, say) can round up, so the
+//   one correction left is to the next smaller number p, when a <= p g (B. Tuckerman's test).
 //
 // The steps hold for operands well inside the exponent range: numerators 0 or 2^-500 .. 2^500,
 // denominators 2^-400 .. 2^400, radicands 2^-500 .. 2^500 (positive).  Every operand's high word goes
@@ -98,14 +99,16 @@ struct Fast64 {
     return fast64_rsqrt_seed(a);
 #endif
   }
-  // The low word's last place tells zero (allowed: its word wraps to the largest value) from the subnormals
+  // The high word, its last bit set where the low word is not zero: 0 for zero alone, not for the subnormals
   // below 2^-1042.
-  __device__ __forceinline__ void num(double a) {
-    const unsigned h = (static_cast<unsigned>(__double2hiint(a)) & 0x7fffffffu) |
-                       min(static_cast<unsigned>(__double2loint(a)), 1u);
-    nlo = min(nlo, h - 1u);
+  static __device__ __forceinline__ unsigned word(double a) {
+    return static_cast<unsigned>(__double2hiint(a)) | min(static_cast<unsigned>(__double2loint(a)), 1u);
+  }
+  __device__ __forceinline__ void num_word(unsigned h) {
+    nlo = min(nlo, h - 1u);  // zero wraps to the largest value: allowed
     nhi = max(nhi, h);
   }
+  __device__ __forceinline__ void num(double a) { num_word(word(a) & 0x7fffffffu); }
   __device__ __forceinline__ void den(double b) {
     const unsigned h = static_cast<unsigned>(__double2hiint(b)) & 0x7fffffffu;
     dlo = min(dlo, h);
@@ -615,8 +618,14 @@ template <int KIND>
 __device__ __forceinline__ double muscl_half_slope(Fast64 &o, double a, double b) {
   if (KIND == LIM_VANLEER || KIND == LIM_VANALBADA) {
     const double ab = a * b;
-    const bool on = !(fabs(b) < 1e-12) && !(ab <= 0.0);
-    if (KIND == LIM_VANLEER) return o.div(on ? ab : 0.0, on ? a + b : 1.0);
+    // !(ab <= 0) as an integer test (the FP64 pipe is the busy one): positive (subnormals and NaN among
+    // them), or NaN with its sign set.
+    const unsigned w = Fast64::word(ab);
+    const bool on = !(fabs(b) < 1e-12) && (static_cast<int>(w) > 0 || w > 0xfff00000u);
+    if (KIND == LIM_VANLEER) {
+      o.num_word(on ? w : 0u);
+      return o.quotient(on ? ab : 0.0, o.rcp(on ? a + b : 1.0));
+    }
     const double a2 = a * a;
     return 0.5 * o.div(on ? b * (a2 + ab) : 0.0, on ? a2 + b * b : 1.0);
   }

@@ -42,6 +42,8 @@ RUN double op(O &o, int k, double a, double b) {
     case 2: return o.inv(b);
     case 3: return o.root(b);
     case 4: return o.div_gm1(a);
+    case 5: return O::fast ? Fast64::rcp_seed(b) : 1.0 / b;
+    case 6: return O::fast ? Fast64::rsqrt_seed(b) : 1.0 / sqrt(b);
     default: return 0.0;
   }
 }

@@ -3,6 +3,7 @@ them, operation by operation against the plain operators: on the CPU with seeds 
 (20 leading bits in and out, three roundings), on the GPU with its own.  The operands are the ones next to
 rounding boundaries, found from the congruences that define them, and the ends of the ranges."""
 import ctypes
+import math
 import os
 import random
 import subprocess
@@ -15,7 +16,7 @@ from conftest import ROOT, assert_bits_equal
 SRC = os.path.join(ROOT, "tests", "fast64_ops.cu")
 CSRC = os.path.join(ROOT, "cfd_solver_withcuda_b200", "csrc")
 DP, IP = ctypes.POINTER(ctypes.c_double), ctypes.POINTER(ctypes.c_int)
-DIV, DIV_SIGNED, INV, ROOT_OP, DIV_GM1, SLOPE = 0, 1, 2, 3, 4, 10
+DIV, DIV_SIGNED, INV, ROOT_OP, DIV_GM1, RCP_SEED, RSQRT_SEED, SLOPE = 0, 1, 2, 3, 4, 5, 6, 10
 
 
 def _dp(a):
@@ -63,12 +64,15 @@ def ops(request):
 
 
 def quotients_beside_boundaries(n):
-    """(a, b): b = 2^53 - d with the reciprocals next to a rounding boundary (d odd), a from the inverse of b
-    modulo 2^54, so that a / b lies one unit of 2^-105 / b from the middle of two numbers."""
+    """(a, b): b = 2^53 - d with the reciprocals next to a rounding boundary, a from the inverse of b modulo
+    2^54, so that a / b lies one unit of 2^-105 / b from the middle of two numbers.  All d below 2^16, those
+    next to the square roots of j 2^53 below 2^30, and n others."""
     rng = random.Random(1)
+    d = list(range(1, 2 ** 16, 2))
+    d += [x for j in range(1, 130) for x in range(math.isqrt(j * 2 ** 53) - 150, math.isqrt(j * 2 ** 53) + 150) if x % 2]
+    d += [rng.getrandbits(rng.randint(1, 45)) | 1 for _ in range(n)]
     out = []
-    while len(out) < n:
-        b = 2 ** 53 - (rng.getrandbits(rng.randint(1, 45)) | 1)
+    for b in (2 ** 53 - x for x in d):
         inv = pow(b, -1, 2 ** 54)
         for s in (1, -1):
             m = (s * inv) % 2 ** 54
@@ -76,6 +80,16 @@ def quotients_beside_boundaries(n):
                 if m >= 2 ** 53 and (b * m - s) % 2 ** shift == 0 and 2 ** 52 <= (b * m - s) >> shift < 2 ** 53:
                     out.append(((b * m - s) >> shift, b))
     return (np.array([x[i] for x in out], np.float64) for i in (0, 1))
+
+
+def test_seeds(ops):
+    """Relative error of the two seeds over every leading mantissa word, in both binades."""
+    rng = np.random.default_rng(7)
+    hi = np.arange(2 ** 21, dtype=np.int64) + (1023 << 20)
+    for lo in (0, 2 ** 32 - 1, rng.integers(0, 2 ** 32, hi.size)):
+        b = ((hi << 32) | lo).view(np.float64)
+        assert np.abs(ops(RCP_SEED, 0.0, b)[0] * b - 1.0).max() < 2.0 ** -19
+        assert np.abs(ops(RSQRT_SEED, 0.0, b)[0] * np.sqrt(b) - 1.0).max() < 2.0 ** -19
 
 
 def test_quotients_beside_rounding_boundaries(ops):
