@@ -159,3 +159,50 @@ def test_batch_up_to_the_capacity():
             b.close()
         for x, y in zip(*out):
             assert_bits_equal(x, y, "instance")
+
+
+@pytest.mark.parametrize("forms", [("gradient", "gradient", "gradient_fp32_hllc"), ("per_cell", "gradient", "per_cell_lts")])
+def test_many_step_kernels_of_several_contexts_at_once(forms):
+    """Three contexts on their own streams, their many-step launches queued side by side: no wait runs out
+    and every context has the bits it has alone."""
+    import torch
+    sizes = ((160, 100), (150, 110), (170, 90))  # each takes most or all of the SMs
+    runs = []
+    for form, (nx, ny) in zip(forms, sizes):
+        m = cb.Mesh.box(nx, ny, 0.0, 2.0, 0.0, 1.0)
+        NP = m.n_physical
+        x = m.centers[:NP]
+        U = np.zeros((m.n_total, 4))
+        U[:NP] = cb.conserved_from_primitive(1 + 0.02 * np.sin(7 * x[:, 0]), 2 + 0.02 * np.cos(5 * x[:, 1]), 0 * x[:, 0],
+                                             (1 + 0.01 * np.sin(9 * x[:, 1])) / 1.4)
+        U[m.boundary[:, 3]] = U[m.boundary[:, 1]]
+        kw = dict(FORMS[form], time_accurate=1, cfl=0.3, inlet_bc=3, inlet_rho=1.0, inlet_u=2.0, inlet_p=1.0 / 1.4,
+                  reorder=4)
+        runs.append((m, kw, U))
+
+    def make(run):
+        m, kw, U = run
+        stream = torch.cuda.Stream()
+        s = cb.Solver(m, cb.default_config(stream=stream.cuda_stream, **kw))
+        s.upload_state(U)
+        return s, stream
+    alone = []
+    for run in runs:
+        s, _ = make(run)
+        n0 = s.kernel_launches
+        s.step_async(400)
+        s.step_async(150)
+        s.sync()
+        assert s.kernel_launches - n0 < 100  # the many-step kernels ran
+        alone.append(s.download())
+        s.close()
+    together = [make(run) for run in runs]
+    for n in (400, 150):
+        for s, _ in together:
+            s.step_async(n)
+    for (s, _), want in zip(together, alone):
+        s.sync()
+        got = s.download()
+        s.close()
+        for k in ("U", "prim", "dt", "net_flux", "delU"):
+            assert_bits_equal(got[k], want[k], k)
