@@ -165,25 +165,27 @@ def face_bytes_per_cell():
     return 32 + 64
 
 
-def gather_stage_bytes_per_cell():
-    """Algorithmic DRAM bytes per cell of the fused gather + stage kernel k_gather_stage, averaged
-    over the three TVD-RK3 stages with frozen local dt (face fluxes counted per face in
-    gather_stage_bytes_per_face).  Every stage reads nf 4, face ids 16, 1/area 8, U^n 32 and writes
-    R 32, the primitive planes 40 and the (rho, u, v, p) row 32; stage 1 also reads del_t 8 and the
-    boundary-entry offsets 4 and writes the frozen dt 8 and the stage state 32; stage 2 reads the
-    offsets 4, the stage state 32 and the frozen dt 8 and writes the stage state 32; stage 3 reads
-    the stage state 32 and the frozen dt 8 and writes U 32.  Per stage 216, 240 and 236 B (the
-    ghost rows the owner threads write are < 0.1 % and left out)."""
-    return (216 + 240 + 236) / 3.0
+def gather_bytes_per_cell(steps):
+    """Algorithmic DRAM bytes per cell of a gather + stage launch (TVD-RK3, frozen local dt; the face
+    fluxes are counted in gather_bytes_per_face), the mean over the launches of a call of `steps`
+    pseudo-steps: k_gather_lean in every launch but the last, k_gather_stage in that one.  Lean: face
+    count 1, face ids 16, 1/area 8, U^n read 32 and the (rho, u, v, p) row written 32; stage 1 also
+    del_t read 8, the frozen dt and the stage state written 8 + 32; stage 2 the stage state and the
+    frozen dt read 32 + 8, the stage state written 32; stage 3 the two read, U and the sound speed
+    written 32 + 8: 137, 161 and 169 B.  The call's last launch also writes R 32 and the other
+    primitive planes 32 (and reads a 4-byte face count): 236 B.  The ghost rows the owner threads write
+    are < 0.1 % and left out."""
+    return (steps * (137 + 161 + 169) + 236 - 169) / (3.0 * steps)
 
 
-def gradient_bytes_per_cell():
-    """Algorithmic DRAM bytes per cell of k_muscl_gradients, averaged over the three stages: the
-    cell's (rho, u, v, p) row 32, nf 4, neighbour ids 16, face normals and lengths 96, 1/area 8,
-    the gradient records written 64 (220 B), plus at the stages that form del_t (first and last)
-    the sound speed 8, the area 8 and del_t written 8 (244 B).  Neighbour rows are re-reads, and
-    the first stage's ghost rows (< 0.1 %) are left out."""
-    return (244 + 220 + 244) / 3.0
+def gradient_bytes_per_cell(steps):
+    """Algorithmic DRAM bytes per cell of k_muscl_gradients, the mean over the launches of a call of
+    `steps` pseudo-steps: the cell's (rho, u, v, p) row 32, face count 1, neighbour ids 16, the faces'
+    weights 64, 1/area 8 and the gradient records written 64 (185 B); at the stages that form del_t (the
+    first of every step, the last of the call's last) the face normals and lengths 96 instead of the
+    weights, the face count as 4, and the sound speed 8, the area 8 and del_t written 8 (245 B).
+    Neighbour rows are re-reads, and the first stage's ghost rows (< 0.1 %) are left out."""
+    return (steps * (245 + 185 + 185) + 245 - 185) / (3.0 * steps)
 
 
 def tile_bytes_per_cell():
@@ -217,7 +219,7 @@ def patch_bytes_per_face():
     return 56
 
 
-def gather_stage_bytes_per_face():
+def gather_bytes_per_face():
     """Each face flux (double4, 32 B) is read by both of its cells; algorithmically once."""
     return 32
 
@@ -811,9 +813,9 @@ def main():
             "k_patch_stage_traffic.json",
             fp64_pipe_active_pct=profile_figure("k_patch_stage_traffic.json", "fp64_pipe_active_pct")))
     if gs_n:
-        rl["k_gather_stage"] = (gs_ms, roofline(
-            "k_gather_stage (face-flux gather + RK stage update)", gs_ms, gs_n,
-            gather_stage_bytes_per_cell() * NP + gather_stage_bytes_per_face() * NF, "k_gather_stage_traffic.json"))
+        rl["k_gather_lean"] = (gs_ms, roofline(
+            "k_gather_lean (face-flux gather + RK stage update; k_gather_stage in the call's last launch)", gs_ms,
+            gs_n, gather_bytes_per_cell(nprof) * NP + gather_bytes_per_face() * NF, "k_gather_lean_traffic.json"))
     if face_n:
         rl["k_faces"] = (face_ms, roofline(
             "k_faces<double> (face fluxes, gradient MUSCL + Roe)", face_ms, face_n,
@@ -823,7 +825,7 @@ def main():
     if grad_n:
         rl["k_muscl_gradients"] = (grad_ms, roofline(
             "k_muscl_gradients (Green-Gauss gradient records, del_t, first-stage BCs)", grad_ms, grad_n,
-            gradient_bytes_per_cell() * NP, "k_muscl_gradients_traffic.json"))
+            gradient_bytes_per_cell(nprof) * NP, "k_muscl_gradients_traffic.json"))
     dominant = max(rl, key=lambda k: rl[k][0]) if rl else None
     rl_main = rl[dominant][1] if dominant else None
     total_kernel_ms = max(sum(v[0] for v in rl.values()) + bc_ms, 1e-30)
