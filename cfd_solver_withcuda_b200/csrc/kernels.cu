@@ -750,7 +750,8 @@ __device__ __noinline__ double4 face_contrib_again(const DevMesh &m, const DevSt
 // state is read), which saves the per-load choice between U and the stage state.  The divisions and
 // square roots are the branch-free ones (Fast64), whose chains interleave within a face, so the face
 // loop is not unrolled: unrolled, the kernels took 124 - 136 registers (12 - 16 warps per SM) and ROE
-// 101 us, ROE_2O 117 us on 524,288 cells, against 73 and 106 us in a loop at 80 (B200).  A cell with an
+// 101 us, ROE_2O 117 us on 524,288 cells, against 68 and 103 us in a loop at 80 (B200), although ROE and
+// HLLC then spill 144 - 244 bytes per thread and the limited forms 304 - 544, held in L1.  A cell with an
 // operand outside their range is evaluated again.
 // want (FluxWant bits): del_t is stored, and Min_dt formed, only for evaluations whose value is used.
 template <int DISS, int ORDER, int MINB = 6, bool SRC_S = true>
@@ -1695,8 +1696,8 @@ struct BcRegs {
 // are formed again: every stage but the last, and the last stage of every pseudo-step but the last of a
 // call without t_end.  It leaves out those stores (R 32 bytes, three or four primitive planes of 8, dU)
 // and, in the last stage, all of the reduction but the step's Min_dt; the rows q4, the states, the frozen
-// dt, the sound speed (where the next gradient pass forms del_t) and the ghosts stay.  204 - 236 bytes per
-// cell and the fluxes; bound by the latency of the face slots and of the fluxes they name (16 - 18
+// dt, the sound speed (where the next gradient pass forms del_t) and the ghosts stay.  201 - 233 bytes per
+// cell, the 64 of its fluxes among them; bound by the latency of the face slots and of the fluxes they name (16 - 18
 // long-scoreboard stalls per issue, DRAM 32 % busy): 28 us on 524,288 cells against k_gather_stage's 35.6.
 // Six blocks per SM: 53.1 us on 1,038,240 mixed cells, 28.0 on 524,288; seven 54.7 and 27.7, five and
 // eight slower.  A persistent loop with the next cell's face slots loaded ahead took 32.0 us, loading the
@@ -2473,7 +2474,8 @@ __global__ void __launch_bounds__(kStepsThreads, 1) k_steps(const __grid_constan
 // (a stage overwrites the primitives that its neighbours' evaluation reads; Min_dt is complete at the first).
 // Min_dt is an atomic minimum of order-preserving keys in three slots used in turn, so that a slot is reset
 // two barriers before it is used again.  Same operations on the same operands as the separate kernels: same
-// bits.  The residual, del_t and the norms stay out, so a step by the separate kernels follows.  Bound by
+// bits.  The residual, del_t and the norms stay out, so a step by the separate kernels follows; a call with a
+// t_end, where any step may be the last, runs them throughout.  Bound by
 // latency: two barriers, the gathers' L2 rounds (a barrier empties the L1, so what stays the same is kept in
 // registers) and one face's dependent FP64 chain per stage.  Per pseudo-step of three stages (separate
 // kernels against this, LLF / ROE / ROE_2O / HLLC, B200): 29 / 31 / 33 / 29 us against 17 / 20 / 22 / 19 at
@@ -3808,11 +3810,11 @@ void launch_faces_b(cudaStream_t s, int g, int b, const DevMesh &m, DevState &st
   else launch_k(m, k_faces<T, 3, MINB>, g, b, s, m, st, fp);
 }
 
-// Launch shapes of the face kernel (identical results).  The double Roe kernel needs 86
-// registers: 256-thread blocks then fit 2 per SM (16 warps, shape 0), 256-thread blocks capped
-// at 80 registers fit 3 (24 warps, a few bytes of spill; shape 1), 128-thread blocks fit 5 (20
+// Launch shapes of the face kernel (identical results).  The double kernels take 114 registers
+// unbounded: 256-thread blocks then fit 2 per SM (16 warps, shape 0), 256-thread blocks capped
+// at 80 registers fit 3 (24 warps, 28 bytes of spill stores; shape 1), 128-thread blocks fit 4 (16
 // warps; shape 2), 128-thread blocks capped at 72 or 64 registers fit 7 or 8 (28 or 32 warps,
-// 44 or 88 bytes of spill held in L1; shapes 3 and 4).  Work lists hold kWorkFaceBlock (128)
+// 36 or 8 bytes of spill stores held in L1; shapes 3 and 4).  Work lists hold kWorkFaceBlock (128)
 // faces per block, so with them every shape runs 128-thread blocks.
 template <typename T>
 void launch_faces_t(cudaStream_t s, const DevMesh &m, DevState &st, const FluxParams &fp) {

@@ -3,9 +3,10 @@
 // Every dense block of the network is a two-layer perceptron y = W2 silu(W1 x + b1) + b2 (+ r),
 // hidden width 64, whose input row x is up to three row segments side by side, each read from
 // its own array, directly or through a row index (the per-edge gathers of the message-passing
-// layers are fused into the operand staging).  Operands are rounded to BF16 when they are staged
-// into shared memory; the products accumulate in FP32 (mma.sync m16n8k16, BF16 inputs, FP32
-// accumulators); bias, SiLU, residual and the SiLU derivative are FP32 epilogues.
+// layers are fused into the operand loads).  Operands are rounded to BF16 when they are loaded, the input
+// rows into the MMA fragments' registers, weights (and the weight gradients' tiles) into shared memory;
+// the products accumulate in FP32 (mma.sync m16n8k16, BF16 inputs, FP32 accumulators); bias, SiLU,
+// residual and the SiLU derivative are FP32 epilogues.
 //
 //   k_mlp_fwd    y and the hidden pre-activation z1 (kept for the backward pass): one warp per 16
 //                rows, input rows straight from global memory into the MMA fragments, weights

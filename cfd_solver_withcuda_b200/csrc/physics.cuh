@@ -26,8 +26,9 @@ struct Prim {  // the five primitive slots the fluxes read: Primitive_Cells[c][0
 // Ieee<T>: the operators themselves.  CUDA's double division and square root test for special
 // operands in a branch each, so a flux with 15 - 25 of them is that many short serial pieces the
 // compiler cannot interleave: the flux kernels were bound by that latency (FP64 pipe 32 - 51 % active).
-// With Fast64 the ROE_2O flux of 524,288 cells takes 117 us instead of 158, the Van Leer + Roe faces
-// 43.7 instead of 52.8, the HLLC faces of 1,038,240 mixed cells 62.9 instead of 73.3 (B200).
+// With Fast64 the ROE_2O flux of 524,288 cells takes 103 us instead of 158 and the Van Leer + Roe faces
+// 45.3 instead of 52.8 (B200; 2.4 us each of them for the Newton step and the tests of the numerators'
+// low words, without which single results were one unit off or subnormals were taken for zeros).
 //
 // Fast64: the same values without branches (every result is the correctly rounded one).
 //   Reciprocal: y0 = rcp.approx.ftz.f64(b) (PTX; relative error e below 2^-19, tested), one third-order step

@@ -440,7 +440,7 @@ cfd_status cfd_mpnn_adam(float *param, const float *grad, float *m, float *v, in
                          float beta2, float eps, int step, void *stream);
 
 /* Dense blocks on the tensor cores: y = W2 silu(W1 x + b1) + b2 (+ r), hidden width 64, BF16
- * operands (rounded when staged), FP32 accumulation and epilogues.  The input row x is up to three
+ * operands (rounded when loaded), FP32 accumulation and epilogues.  The input row x is up to three
  * segments side by side (total width <= 192); segment s supplies columns of row
  * (idx ? idx[row] : row) of src (leading dimension ld), through silu() when silu = 1. */
 typedef struct {
@@ -462,7 +462,7 @@ typedef struct {
   float *z1;               /* out (optional): hidden pre-activation [rows][64] */
   float *y;                /* out [rows][ld_y] */
   int ld_y;
-  int engine;              /* 0: mma.sync m16n8k16 (64-row tiles); 1: tcgen05.mma with the accumulators in
+  int engine;              /* 0: mma.sync m16n8k16 (a warp per 16 rows); 1: tcgen05.mma with the accumulators in
                               tensor memory (128-row tiles, operands in shared memory by matrix
                               descriptors); the two agree up to the FP32 summation order */
 } cfd_mlp_fwd;
