@@ -288,7 +288,8 @@ class Net:
         self.engine = engine
         self.bwd_engine = engine if bwd_engine is None else bwd_engine
         self.L, self.out, self.device = layers, out, torch.device(device)
-        # The mma.sync passes of a network with at most 16 outputs are issued by one library call each.
+        # The mma.sync passes of a network with at most 16 outputs are issued by one library call each
+        # (_whole_pass: the engines are looked at when a forward pass is made; its backward pass follows).
         self.whole = self.engine == 0 and self.bwd_engine == 0 and out <= 16
         self.dims = {"enc_n": (node_in, W), "enc_e": (edge_in, W), "dec": (W, out)}
         for l in range(layers):
@@ -340,20 +341,24 @@ class Net:
     def get_grads(self):
         return {n: tuple(t.detach().cpu().numpy().astype(np.float64) for t in self.g[n]) for n in self.names}
 
-    # -- buffers per (nodes, edges)
+    def _whole_pass(self):
+        return self.whole and self.engine == 0 and self.bwd_engine == 0
+
+    # -- buffers per (nodes, edges, form)
     def _buffers(self, N, E):
-        if self._bufs is not None and self._bufs["key"] == (N, E):
+        whole = self._whole_pass()
+        if self._bufs is not None and self._bufs["key"] == (N, E, whole):
             return self._bufs
         torch = _torch()
         W, L = self.HIDDEN, self.L
         f = lambda r, c: torch.empty((r, c), dtype=torch.float32, device=self.device)
-        if self.whole:
+        if whole:
             n = cb.lib().cfd_mpnn_net_floats(L, self.dims["enc_n"][0], self.dims["enc_e"][0], self.out, N, E)
-            self._bufs = {"key": (N, E), "act": torch.empty(n, dtype=torch.float32, device=self.device),
+            self._bufs = {"key": (N, E, whole), "act": torch.empty(n, dtype=torch.float32, device=self.device),
                           "pred": f(N, self.out), "dpred": f(N, self.out),
                           "loss": torch.zeros(1, dtype=torch.float32, device=self.device)}
             return self._bufs
-        b = {"key": (N, E), "h": [f(N, W) for _ in range(L + 1)], "e": [f(E, W) for _ in range(L + 1)],
+        b = {"key": (N, E, whole), "h": [f(N, W) for _ in range(L + 1)], "e": [f(E, W) for _ in range(L + 1)],
              "agg": [f(N, W) for _ in range(L)], "z_enc_n": f(N, W), "z_enc_e": f(E, W),
              "z_edge": [f(E, W) for _ in range(L)], "z_node": [f(N, W) for _ in range(L)], "z_dec": f(N, W),
              "pred": f(N, self.out), "dpred": f(N, self.out), "dh": f(N, W), "de": f(E, W),
@@ -431,7 +436,7 @@ class Net:
         tensors) on the stacked graph gb; keeps the activations for backward()."""
         N, E = xn.shape[0], xe.shape[0]
         b = self._buffers(N, E)
-        if self.whole:
+        if "act" in b:
             if (xn.shape[1], xe.shape[1]) != (self.dims["enc_n"][0], self.dims["enc_e"][0]):
                 raise ValueError("the network takes %d node and %d edge features, got %d and %d" % (
                     self.dims["enc_n"][0], self.dims["enc_e"][0], xn.shape[1], xe.shape[1]))
@@ -458,7 +463,7 @@ class Net:
         """Gradients of every parameter (into self.grad) from the prediction gradient dpred."""
         b, gb, W, L = self._bufs, self._graph, self.HIDDEN, self.L
         xn, xe = self._x
-        if self.whole:
+        if "act" in b:
             cb._check(cb.lib().cfd_mpnn_net_backward(ctypes.byref(self._net(xn, xe, gb, dpred)), _stream(dpred)))
             return
         N, E = xn.shape[0], xe.shape[0]

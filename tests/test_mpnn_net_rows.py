@@ -12,12 +12,15 @@ torch = pytest.importorskip("torch")
 
 
 class Recorder:
-    """The library with its two whole passes replaced by copies of the structures they are given."""
+    """The library with its two whole passes replaced by copies of the structures they are given, and the
+    single blocks by the engines they are given."""
 
     def __init__(self, real):
-        self.real, self.seen = real, []
+        self.real, self.seen, self.blocks = real, [], []
 
     def __getattr__(self, name):
+        if name in ("cfd_mpnn_mlp_forward", "cfd_mpnn_segment_sum_acc"):
+            return lambda *a: self.blocks.append(a[0]._obj.engine if "mlp" in name else None) or 0
         if name not in ("cfd_mpnn_net_forward", "cfd_mpnn_net_backward"):
             return getattr(self.real, name)
 
@@ -67,6 +70,22 @@ def test_overlapping_rows_are_refused(recorded):
     status = [lib.cfd_mpnn_net_forward(ctypes.byref(seen[0]), None), lib.cfd_mpnn_net_forward(ctypes.byref(seen[1]), None),
               lib.cfd_mpnn_net_backward(ctypes.byref(seen[2]), None)]
     assert status == [cb.CFD_ERR_BAD_ARG] * 3
+
+
+def test_engines_changed_afterwards_are_used(recorded):
+    """A network set to the tcgen05 blocks after it was made runs block by block, and whole passes again when
+    it is set back."""
+    seen, net, g = recorded
+    xn, xe = torch.zeros(g.N, 9), torch.zeros(g.E, 5)
+    net.forward(xn, xe, g)
+    assert len(seen) == 1 and not cb.lib().blocks
+    net.engine = net.bwd_engine = 1
+    net.forward(xn, xe, g)
+    assert len(seen) == 1 and cb.lib().blocks.count(1) == 5
+    net.engine = net.bwd_engine = 0
+    net.forward(xn, xe, g)
+    net.backward(torch.zeros(g.N, 4))
+    assert len(seen) == 3
 
 
 @pytest.mark.gpu
