@@ -354,6 +354,7 @@ struct cfd_ctx {
   int use_graph = 1;
   int fuse_gather = 1;  // face-based forms with per-cell dt: fused gather + stage update
   int patch_stage = 0;  // ... or, with patch tables (reorder 3), the one-kernel patch stage
+  bool stage_ghosts = true;    // k_stage writes the next evaluation's ghosts (stage_ghosts_for)
   bool ghost_private = false;  // every ghost row has one boundary entry and neighbours only its owner
   size_t l2_window = 0;        // bytes of the face-flux L2 window (option "l2_persist" turns it on/off)
   std::vector<int> patch_starts;  // first device cell of each patch (reorder 3)
@@ -532,8 +533,8 @@ int enqueue_stage(cfd_ctx *ctx, int k, bool fuse_final, bool full, bool &ghosts_
     n += launch_bc(s, m, st, ctx->bp, k > 0 && p.src_S, k > 0);
   }
   ghosts_written = false;
-  // The stage kernels' owner threads write the next stage's ghosts.
-  const int ghosts = k < p.n - 1 ? kStageGhosts | (p.src_S ? kStageExitS : 0) : 0;
+  // The stage kernels' owner threads write the next stage's ghosts where that pays.
+  const int ghosts = k < p.n - 1 && ctx->stage_ghosts ? kStageGhosts | (p.src_S ? kStageExitS : 0) : 0;
   if (tile) {
     TimedScope ts(ctx, TK_TILE);
     const bool bc_next = k < p.n - 1;
@@ -601,7 +602,7 @@ int enqueue_stage(cfd_ctx *ctx, int k, bool fuse_final, bool full, bool &ghosts_
     } else {
       { TimedScope ts(ctx, TK_FLUX); n += launch_gather(s, m, st, ctx->fp); }
       { TimedScope ts(ctx, TK_STAGE); n += launch_stage(s, m, st, ctx->bp, kind, lts, fin, ctx->keep_delu, ghosts); }
-      ghosts_written = k < p.n - 1;
+      ghosts_written = ghosts != 0;
     }
     return n;
   }
@@ -612,12 +613,13 @@ int enqueue_stage(cfd_ctx *ctx, int k, bool fuse_final, bool full, bool &ghosts_
   if (lts == 1 && !(last && full)) want = kWantDt;
   { TimedScope ts(ctx, TK_FLUX); n += launch_flux(s, m, st, ctx->fp, k > 0, want); }
   // The last stage of a step that another one follows also writes that step's first ghosts.
-  const int flags = last ? (full || !fuse_final ? 0 : kStageNextStep | kStageNoNorms) : ghosts;
+  const int next = ctx->stage_ghosts ? kStageNextStep : 0;
+  const int flags = last ? (full || !fuse_final ? 0 : next | kStageNoNorms) : ghosts;
   {
     TimedScope ts(ctx, TK_STAGE);
     n += launch_stage(s, m, st, ctx->bp, kind, lts, fin, last && !full ? 0 : ctx->keep_delu, flags);
   }
-  ghosts_written = flags != 0;
+  ghosts_written = (flags & (kStageGhosts | kStageNextStep)) != 0;
   return n;
 }
 
@@ -1411,6 +1413,7 @@ cfd_status cfd_create(const cfd_mesh_desc *d, const cfd_config *cfg, cfd_ctx **o
   fp.muscl = cfg->muscl && cfg->is_second_order;
   fp.lanes = flux_lanes_for(NP);
   ctx->dm.pdl = pdl_for(NP);
+  ctx->stage_ghosts = stage_ghosts_for(NP);
   ctx->dm.grad_ahead = grad_ahead_for(NP);
   fp.faces_shape = 3;
   // WENO (Is_WENO): Explicit_Method falls back to the 1O/2O residual when any cell is not a quad
@@ -1661,8 +1664,9 @@ static cfd_status enqueue_steps(cfd_ctx *ctx, int n_steps) {
   if (ctx->persistent && ctx->persist_grid > 0 && ctx->dm.NF > 0) return enqueue_steps_persistent(ctx, n_steps);
   // Every step but the last leaves out what the next one overwrites, unless a t_end may make any the last.
   int lean = ctx->t_end_set ? 0 : n_steps - 1;
-  // Per-cell forms: such a step also leaves the next one's ghosts, so only the first needs them formed here.
-  const bool ghosts = ctx->dm.NF == 0;
+  // Per-cell forms whose stages write ghosts: such a step also leaves the next one's, so only the first needs
+  // them formed here.
+  const bool ghosts = ctx->dm.NF == 0 && ctx->stage_ghosts;
   if (lean > 0 && ghosts) {
     TimedScope ts(ctx, TK_BC);
     ctx->launches += launch_bc(ctx->stream, ctx->dm, ctx->ds, ctx->bp, 0, 0);
@@ -1822,9 +1826,10 @@ cfd_status cfd_runge_kutta_method(cfd_ctx *ctx) {
   StagePlan p = stage_plan(c, ctx->fp.consistent);
   if (p.kind0 == 0) p = {3, 1, ctx->fp.consistent, 0};  // the reference's RK3 on an explicit config
   for (int k = 0; k < p.n; k++) {
+    if (k > 0 && !ctx->stage_ghosts) ctx->launches += launch_bc(ctx->stream, ctx->dm, ctx->ds, ctx->bp, p.src_S, 1);
     ctx->launches += launch_flux(ctx->stream, ctx->dm, ctx->ds, ctx->fp, k > 0);
     ctx->launches += launch_stage(ctx->stream, ctx->dm, ctx->ds, ctx->bp, p.kind0 + k, stage_lts(p, c, k), 0, 1,
-                                  k < p.n - 1 ? kStageGhosts | (p.src_S ? kStageExitS : 0) : 0);
+                                  k < p.n - 1 && ctx->stage_ghosts ? kStageGhosts | (p.src_S ? kStageExitS : 0) : 0);
   }
   CUDA_TRY(cudaGetLastError());
   ctx->prim_from_S = true;

@@ -751,8 +751,10 @@ __device__ __noinline__ double4 face_contrib_again(const DevMesh &m, const DevSt
 // square roots are the branch-free ones (Fast64), whose chains interleave within a face, so the face
 // loop is not unrolled: unrolled, the kernels took 124 - 136 registers (12 - 16 warps per SM) and ROE
 // 101 us, ROE_2O 117 us on 524,288 cells, against 68 and 103 us in a loop at 80 (B200), although ROE and
-// HLLC then spill 144 - 244 bytes per thread and the limited forms 304 - 544, held in L1.  A cell with an
-// operand outside their range is evaluated again.
+// HLLC then spill 144 - 244 bytes per thread and the limited forms 304 - 544, held in L1.  LLF, which
+// divides nothing, is unrolled at 80 registers without a spill: 41.8 / 117 / 195 us per pseudo-step at 45,000 /
+// 320,000 / 524,288 cells against 43.7 / 123 / 209 in a loop and 45.7 / 137 / 215 unrolled without the bound
+// (B200).  A cell with an operand outside their range is evaluated again.
 // want (FluxWant bits): del_t is stored, and Min_dt formed, only for evaluations whose value is used.
 template <int DISS, int ORDER, int MINB = 6, bool SRC_S = true>
 __global__ void __launch_bounds__(kFluxBlock, MINB) k_flux(const __grid_constant__ DevMesh m,
@@ -774,8 +776,7 @@ __global__ void __launch_bounds__(kFluxBlock, MINB) k_flux(const __grid_constant
     double N0 = 0.0, N1s = 0.0, N2s = 0.0, N3s = 0.0;
     double den = 0.0;
     Fast64 o;
-#pragma unroll 1
-    for (int f = 0; f < nf; f++) {
+    auto add_face = [&](int f) {
       double X[4], t;
       face_contrib<DISS, ORDER>(o, m, st, fp, us, q, load_face<DISS, ORDER>(m, c, f), f, X, t);
       N0 += X[0];
@@ -783,6 +784,14 @@ __global__ void __launch_bounds__(kFluxBlock, MINB) k_flux(const __grid_constant
       N2s += X[2];
       N3s += X[3];
       den += t;
+    };
+    if constexpr (DISS == 1) {  // no divisions
+#pragma unroll
+      for (int f = 0; f < 4; f++)
+        if (f < nf) add_face(f);
+    } else {
+#pragma unroll 1
+      for (int f = 0; f < nf; f++) add_face(f);
     }
     if (o.bad()) {
       N0 = N1s = N2s = N3s = 0.0;
@@ -1523,11 +1532,15 @@ __device__ __forceinline__ void cell_update(const DevMesh &m, const DevState &st
 
 // lts: 0 Min_dt, 1 Cell::del_t (reference stage 1 only), 2 dt frozen per cell at the first stage,
 // 3 Min_dt frozen at the first stage.
-// flags (StageFlags): the owner thread writes its ghosts for the next evaluation, with kStageNextStep those
-// of the next pseudo-step's first one; kStageNoNorms leaves the norms out.  Bound by its traffic (168 - 232
-// bytes per cell) and, on small meshes, by the launch: the ghost writes save a k_bc launch per stage (5.5 us
-// on 524,288 cells), the missing norms 10 us of the last stage's 22 there.
-__global__ void __launch_bounds__(kBlock) k_stage(DevMesh m, DevState st, BcParams bp, int kind, int lts,
+// flags (StageFlags): the owner thread writes its ghosts for the next evaluation (GHOSTS), with
+// kStageNextStep those of the next pseudo-step's first one; kStageNoNorms leaves the norms out (10 us of the
+// last stage's 22 on 524,288 cells).  Bound by its traffic (168 - 232 bytes per cell): 64 registers, 14 us per
+// launch on 524,288 cells.  With the boundary kinds (GHOSTS) it takes 94, half the warps per SM and 24 us
+// there, but saves the k_bc launches, which pays on small meshes: see stage_ghosts_for.  (As a function that is
+// not inlined they leave the kernel at 64 registers; 1.01 - 1.04 x faster on 180,000 cells, 0.95 on 24,000.)
+template <bool GHOSTS>
+__global__ void __launch_bounds__(kBlock, GHOSTS ? 1 : 4) k_stage(const __grid_constant__ DevMesh m, const __grid_constant__ DevState st,
+                                                  const __grid_constant__ BcParams bp, int kind, int lts,
                                                   int fuse_final, int keep_delu, int flags) {
   pdl_enter();
   const int NP = m.NP;
@@ -1550,17 +1563,12 @@ __global__ void __launch_bounds__(kBlock) k_stage(DevMesh m, DevState st, BcPara
 #pragma unroll
     for (int k = 0; k < 4; k++) Rk[k] = st.R[k * NP + c];
     cell_update(m, st, c, kind, dt, Rk, fuse_final, keep_delu, e);
-    if (flags & (kStageGhosts | kStageNextStep)) {
-      const int b0 = m.bptr[c], b1 = m.bptr[c + 1];
-      const int cur_S = (flags & kStageGhosts) ? 1 : 0;
-      for (int i = b0; i < b1; i++) bc_entry(m, st, bp, m.bidx[i], (cur_S && (flags & kStageExitS)) ? 1 : 0, cur_S);
-    }
   }
   if (first_kind(kind) && blockIdx.x == 0 && threadIdx.x == 0 && !done) st.ctl[CTL_DTSTEP] = dtmin;
   if (fuse_final && final_kind(kind)) {
     if (done) return;
     const double dt_time = (lts >= 2) ? st.ctl[CTL_DTSTEP] : dtmin;
-    if (flags & kStageNoNorms) {  // only without t_end
+    if (GHOSTS || (flags & kStageNoNorms)) {  // only without t_end
       if (blockIdx.x == 0 && threadIdx.x == 0) {
         st.ctl[CTL_TOTAL_TIME] += dt_time;
         st.ctl[CTL_ITER] += 1.0;
@@ -1568,6 +1576,11 @@ __global__ void __launch_bounds__(kBlock) k_stage(DevMesh m, DevState st, BcPara
     } else {
       reduce_err_and_epilogue(st, e, true, dt_time);
     }
+  }
+  if (GHOSTS && active) {
+    const int b0 = m.bptr[c], b1 = m.bptr[c + 1];
+    const int cur_S = (flags & kStageGhosts) ? 1 : 0;
+    for (int i = b0; i < b1; i++) bc_entry(m, st, bp, m.bidx[i], (cur_S && (flags & kStageExitS)) ? 1 : 0, cur_S);
   }
 }
 
@@ -3785,8 +3798,9 @@ int launch_flux(cudaStream_t s, const DevMesh &m, DevState &st, const FluxParams
 
 int launch_stage(cudaStream_t s, const DevMesh &m, DevState &st, const BcParams &bp, int kind, int lts, int fuse_final,
                  int keep_delu, int flags) {
-  if (m.cblk) launch_k(m, k_stage, m.n_cblk, kWorkCellBlock, s, m, st, bp, kind, lts, fuse_final, keep_delu, flags);
-  else launch_k(m, k_stage, nblk(m.NP, kBlock), kBlock, s, m, st, bp, kind, lts, fuse_final, keep_delu, flags);
+  const auto k = (flags & (kStageGhosts | kStageNextStep)) ? k_stage<true> : k_stage<false>;
+  if (m.cblk) launch_k(m, k, m.n_cblk, kWorkCellBlock, s, m, st, bp, kind, lts, fuse_final, keep_delu, flags);
+  else launch_k(m, k, nblk(m.NP, kBlock), kBlock, s, m, st, bp, kind, lts, fuse_final, keep_delu, flags);
   return 1;
 }
 
@@ -4182,6 +4196,12 @@ int device_sms() {
 int flux_lanes_for(int cells) { return 4LL * cells <= 640LL * device_sms() ? 4 : 1; }
 
 bool two_waves(int cells) { return cells >= 2LL * 6 * kFluxBlock * device_sms(); }
+
+// Whether k_stage writes the next evaluation's ghosts or k_bc forms them in its own launch.  Per pseudo-step
+// (k_stage / k_bc, B200): ROE_2O 54 / 58 us at 24,200 cells, 89 / 92 at 109,200, 136 / 136.5 at 180,000,
+// 241 / 227 at 320,000, 381 / 354 at 524,288, ROE 270 / 244 there: with more than two waves the kernel's
+// lower occupancy costs more than the launch.
+bool stage_ghosts_for(int cells) { return !two_waves(cells); }
 
 // Programmatic dependent launch pays from two waves of the six-blocks-per-SM kernels on: per pseudo-step at
 // 524,288 cells 252 -> 249 us (gradient MUSCL), 225 -> 220 (FP32-flux), 358 -> 355 (ROE_2O), 239 -> 235

@@ -205,6 +205,7 @@ int launch_flux(cudaStream_t s, const DevMesh &m, DevState &st, const FluxParams
                 int want = kWantDt | kWantMin);
 int flux_lanes_for(int cells);
 int pdl_for(int cells);
+bool stage_ghosts_for(int cells);
 int grad_ahead_for(int cells);
 // Lax_Fedrichs over cells grouped by wavefront level (cells[level_start[l] .. level_start[l+1])).
 int launch_lax_friedrichs(cudaStream_t s, const DevMesh &m, DevState &st, const int *cells,

@@ -206,3 +206,38 @@ def test_many_step_kernels_of_several_contexts_at_once(forms):
         s.close()
         for k in ("U", "prim", "dt", "net_flux", "delU"):
             assert_bits_equal(got[k], want[k], k)
+
+
+@pytest.mark.parametrize("nx,ny", [(512, 443), (512, 445)])  # 226,816 and 227,840 cells: two waves on 148 SMs
+@pytest.mark.parametrize("kw", [dict(is_second_order=0, dissipation_type=1),
+                                dict(is_second_order=1, dissipation_type=3, integrator=2, local_time_stepping=1)])
+def test_per_cell_forms_around_two_waves(nx, ny, kw, oracle_lib):
+    """Below two waves the stage kernel writes the ghosts, from there on the boundary kernel: steps in one call,
+    single steps and the reference's entry points against the C restatement."""
+    m = cb.Mesh.box(nx, ny, 0.0, 2.0, 0.0, 1.0)
+    NP = m.n_physical
+    x = m.centers[:NP]
+    U = np.zeros((m.n_total, 4))
+    U[:NP] = cb.conserved_from_primitive(1 + 0.02 * np.sin(7 * x[:, 0]), 2 + 0.02 * np.cos(5 * x[:, 1]), 0 * x[:, 0],
+                                         (1 + 0.01 * np.sin(9 * x[:, 1])) / 1.4)
+    U[m.boundary[:, 3]] = U[m.boundary[:, 1]]
+    kw = dict(kw, time_accurate=1, cfl=0.3, inlet_rho=1.0, inlet_u=2.0, inlet_p=1.0 / 1.4)
+    o = oracle_lib.OracleRun(m, **kw)
+    o.set_state(U)
+    o.iterate(2)
+    want = o.state()
+    for calls in ((2,), (1, 1), None):
+        s = cb.Solver(m, cb.default_config(reorder=4, **kw))
+        s.upload_state(U)
+        for n in calls or ():
+            s.step(n)
+        if calls is None:
+            for _ in range(2):
+                s.Apply_Boundary_Conditions()
+                s.Runge_Kutta_Method()
+                s.Estimate_Error()
+                s.Update()
+        got = s.download()
+        s.close()
+        for k in ("U", "net_flux", "delU"):
+            assert_bits_equal(got[k], want[k], "%s %s" % (k, calls))
